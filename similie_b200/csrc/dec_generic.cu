@@ -6,13 +6,17 @@
 // Each kernel is instantiated for the field rank ND (lattice + spectator
 // dims, 1..6) so the index arithmetic unrolls; the sampling rules (faces of
 // the basis simplices, Hodge-star factors) come from tables built on the
-// host (host.cu).
+// host (host.cu).  Fields without spectator dims go to the compile-time-rank
+// kernels of dec_dense.cu where those take them.
 #include <algorithm>
 #include <type_traits>
 
 #include "sil_internal.cuh"
 
 namespace sil {
+
+bool dense_ok(uint32_t mask, sil_field const& in, sil_field const& out);
+bool launch_dense(cudaStream_t stream, int op, Geometry const* geo, int k, sil_field const& in, sil_field const& out);
 
 namespace {
 
@@ -566,11 +570,15 @@ void launch_fused_t(cudaStream_t stream, Geometry const& geo, uint32_t mask, int
 sil_status launch_coboundary(cudaStream_t stream, uint32_t mask, int k, sil_field const& in, sil_field const& out,
                              bool transposed)
 {
+    int64_t const total = node_count(out);
+    if (total == 0) return SIL_OK;
+    if (dense_ok(mask, in, out) && launch_dense(stream, transposed ? 1 : 0, nullptr, k, in, out)) {
+        SIL_CUDA_CHECK(cudaGetLastError());
+        return SIL_OK;
+    }
     DimMap dm {};
     dm.n = form_dims(mask, in.ndims, dm.dims);
     CoboundaryRules const rules = make_rules(dm.n, k, transposed);
-    int64_t const total = node_count(out);
-    if (total == 0) return SIL_OK;
     if (in.dtype == SIL_F64) launch_coboundary_t<double>(stream, rules, dm, in, out, transposed, total);
     else launch_coboundary_t<float>(stream, rules, dm, in, out, transposed, total);
     SIL_CUDA_CHECK(cudaGetLastError());
@@ -663,6 +671,10 @@ sil_status launch_fused_laplacian(cudaStream_t stream, Geometry const& geo, uint
 {
     int64_t const total = node_count(out);
     if (total == 0) return SIL_OK;
+    if (dense_ok(mask, in, out) && launch_dense(stream, 3, &geo, k, in, out)) {
+        SIL_CUDA_CHECK(cudaGetLastError());
+        return SIL_OK;
+    }
     if (in.dtype == SIL_F64) launch_fused_t<double>(stream, geo, mask, k, in, out, total);
     else launch_fused_t<float>(stream, geo, mask, k, in, out, total);
     SIL_CUDA_CHECK(cudaGetLastError());
@@ -674,6 +686,10 @@ sil_status launch_codifferential(cudaStream_t stream, Geometry const& geo, uint3
 {
     int64_t const total = node_count(out);
     if (total == 0) return SIL_OK;
+    if (dense_ok(mask, in, out) && launch_dense(stream, 2, &geo, k, in, out)) {
+        SIL_CUDA_CHECK(cudaGetLastError());
+        return SIL_OK;
+    }
     with_nd(out.ndims, [&](auto ndc) {
         constexpr int ND = decltype(ndc)::value;
         if (in.dtype == SIL_F64)
