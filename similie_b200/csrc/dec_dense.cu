@@ -14,8 +14,8 @@
 //
 // Measured on a B200, table-driven -> here: 1-form Laplacian 161x144x130 FP64
 // 2,366 -> 145 us, 1999x2741 FP32 1,016 -> 46 us; d + star + codifferential of
-// a 150x171x128 1-form FP64 651 -> 122 us (the star, 38 us, is the same
-// kernel on both sides).
+// a 150x171x128 1-form FP64 651 -> 122 us (the star is one kernel on both
+// sides).
 #include <algorithm>
 #include <cstdint>
 #include <cstdlib>

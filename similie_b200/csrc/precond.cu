@@ -731,14 +731,29 @@ __global__ void __launch_bounds__(128) wgrad_kernel(const __grid_constant__ Tabl
     if (warp == 0) tmem_dealloc(tmem, 128);
 }
 
-// grad[i] += sum over parts p of part[p][i] (fixed order).
-__global__ void reduce_parts_kernel(float const* part, int nparts, int n, float* grad)
+// grad[i] += sum over parts p of part[p][i], 32 entries per block: each of
+// the eight warps sums a contiguous eighth of the parts in order, warp 0 adds
+// the eight sums in order (a fixed order for a given number of parts).  One
+// thread per entry summing all parts in series took 10.7 us a call at eight
+// 256^2 samples, this 6.1.
+__global__ void __launch_bounds__(256) reduce_parts_kernel(float const* part, int nparts, int n, float* grad)
 {
-    int const i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    __shared__ float red[8][32];
+    int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int const i = blockIdx.x * 32 + lane;
+    int const per = (nparts + 7) / 8, p1 = min(nparts, (warp + 1) * per);
     float sacc = 0.0f;
-    for (int p = 0; p < nparts; ++p) sacc = sacc + part[static_cast<int64_t>(p) * n + i];
-    grad[i] = grad[i] + sacc;
+    if (i < n) {
+#pragma unroll 8
+        for (int p = warp * per; p < p1; ++p) sacc = sacc + part[static_cast<int64_t>(p) * n + i];
+    }
+    red[warp][lane] = sacc;
+    __syncthreads();
+    if (warp != 0 || i >= n) return;
+    float total = 0.0f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) total = total + red[w][lane];
+    grad[i] = grad[i] + total;
 }
 
 // BF16 weights of the 32->32 convolutions: forward [co][tap][ci] and, for
@@ -902,95 +917,161 @@ __global__ void out_backward_data_kernel(const __grid_constant__ Table t, float 
     for (int q = 0; q < 8; ++q) dst[q] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
 }
 
+// Weight gradients of the thin convolutions (2 -> 32 input, 32 -> 1 output).
+//
+// Each is a sum over pixels of a 32-channel vector times a small window of
+// the other tensor, so a warp holds the 32 channels in its lanes and every
+// (tap, thin channel) weight of its lane in registers; it walks 16 consecutive
+// pixels of a 128-pixel tile with the window sliding through registers, one
+// coalesced channel load and nine (18) FMAs per pixel.  The tile's three
+// window rows are staged in shared memory; a tile is a flat run of padded
+// pixels, whose border pixels carry zero channels, so no pixel needs its
+// coordinates.  Blocks keep their sums over all their tiles, add the eight
+// warps' in order and write one partial each; reduce_parts_kernel adds those
+// in order (deterministic).  Bound by the latency of the one pass over the
+// channels: with a thread per weight walking 1,024 pixels in series the input
+// and output gradients took 1,117 and 595 us of a 2,685 us gradient of eight
+// 256^2 samples; here 14.8 and 10.7 us of 1,134.
 constexpr int kThinBlock = 256;
-constexpr int kThinPx = 1024;  // pixels per block of the thin weight-gradient kernels
+constexpr int kThinWarps = kThinBlock / 32;
+constexpr int kThinRun = kTilePx / kThinWarps;  // pixels per warp and tile
 
-// Image of a flat pixel of the concatenated padded images of a table.
-__device__ __forceinline__ int image_of_pixel(Table const& t, int64_t p)
+// Adds the block's per-lane sums over its warps; dst[v * 32 + lane].
+template <int NV>
+__device__ __forceinline__ void thin_block_sum(float const (&acc)[NV], float* smem, float (&sum)[(NV + 7) / 8])
 {
-    int lo = 0, hi = t.nimg - 1;
-    while (lo < hi) {
-        int const mid = (lo + hi + 1) / 2;
-        if (t.img[mid].offset <= p) lo = mid;
-        else hi = mid - 1;
+    int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __syncthreads();
+#pragma unroll
+    for (int v = 0; v < NV; ++v) smem[(warp * NV + v) * 32 + lane] = acc[v];
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < (NV + 7) / 8; ++r) {
+        int const v = warp + r * kThinWarps;
+        float t = 0.0f;
+        if (v < NV)
+            for (int w = 0; w < kThinWarps; ++w) t = t + smem[(w * NV + v) * 32 + lane];
+        sum[r] = t;
     }
-    return lo;
 }
 
-constexpr int kThinPerThread = 3;  // parameters per thread (608 <= 3 * 256)
-
-// Weight gradient of the output convolution, per-block partials:
-// part[b][tap*32 + ci] = sum_p du[p] in[p + tap][ci], part[b][288] = sum_p du[p],
-// block b covering the flat pixels [b*kThinPx, (b+1)*kThinPx) of the table's images.
+// part[b][tap*32 + ci] = sum_q in[q][ci] du[q - tap], part[b][288] = sum_q du[q], over the block's tiles.
 __global__ void __launch_bounds__(kThinBlock) out_wgrad_kernel(const __grid_constant__ Table t, float const* du,
-                                                               bf16 const* in, float* part, int64_t total_px)
+                                                               bf16 const* in, float* part)
 {
-    int const n = kOutW + 1;
-    float acc[kThinPerThread] = {0.0f, 0.0f, 0.0f};
-    int64_t const p0 = static_cast<int64_t>(blockIdx.x) * kThinPx;
-    for (int64_t p = p0; p < p0 + kThinPx && p < total_px; ++p) {
-        Img const o = t.img[image_of_pixel(t, p)];
-        int64_t const g = p - o.offset;
-        int64_t const P = o.w + 2;
-        int64_t const y = g / P, x = g - y * P;
-        if (y == 0 || x == 0 || y > o.h || x > o.w) continue;
-        float const d = du[p];
+    constexpr int NV = kTaps + 1;
+    __shared__ float win[3][kHalo + 2];
+    __shared__ float red[kThinWarps * NV * 32];
+    int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float acc[NV] = {};
+    for (int tile = blockIdx.x; tile < t.tile_base[t.nimg]; tile += gridDim.x) {
+        int const im = find_image(t, tile);
+        Img const o = t.img[im];
+        int const P = o.w + 2, npx = P * (o.h + 2), end = P * (o.h + 1);
+        int const start = P + (tile - t.tile_base[im]) * kTilePx;
+        __syncthreads();
+        for (int i = threadIdx.x; i < 3 * kHalo; i += kThinBlock) {
+            int const r = i / kHalo, j = i - r * kHalo, g = start + (r - 1) * P - 1 + j;
+            win[r][j] = g >= 0 && g < npx ? du[o.offset + g] : 0.0f;
+        }
+        __syncthreads();
+        int const m0 = warp * kThinRun;
+        bf16 const* src = in + (o.offset + start + m0) * kCh + lane;
+        float d[3][3];
 #pragma unroll
-        for (int r = 0; r < kThinPerThread; ++r) {
-            int const k = threadIdx.x + r * kThinBlock;
-            if (k > kOutW) continue;
-            if (k == kOutW) {
-                acc[r] = acc[r] + d;
-            } else {
-                int const tap = k / kCh, ci = k % kCh;
-                int64_t const q = p + (tap / 3 - 1) * P + (tap % 3 - 1);
-                acc[r] = acc[r] + d * __bfloat162float(in[q * kCh + ci]);
+        for (int r = 0; r < 3; ++r) {
+            d[r][1] = win[r][m0];
+            d[r][2] = win[r][m0 + 1];
+        }
+#pragma unroll
+        for (int m = 0; m < kThinRun; ++m) {
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                d[r][0] = d[r][1];
+                d[r][1] = d[r][2];
+                d[r][2] = win[r][m0 + m + 2];
             }
+            float const v = start + m0 + m < end ? __bfloat162float(src[m * kCh]) : 0.0f;
+            // du at q - tap: the window read backwards
+#pragma unroll
+            for (int tap = 0; tap < kTaps; ++tap) acc[tap] = __fmaf_rn(v, d[2 - tap / 3][2 - tap % 3], acc[tap]);
+            if (start + m0 + m < end) acc[kTaps] = acc[kTaps] + d[1][1];
         }
     }
-    float* dst = part + static_cast<int64_t>(blockIdx.x) * n;
-    for (int r = 0; r < kThinPerThread; ++r) {
-        int const k = threadIdx.x + r * kThinBlock;
-        if (k < n) dst[k] = acc[r];
+    float sum[(NV + 7) / 8];
+    thin_block_sum<NV>(acc, red, sum);
+    float* dst = part + static_cast<int64_t>(blockIdx.x) * (kOutW + 1);
+#pragma unroll
+    for (int r = 0; r < (NV + 7) / 8; ++r) {
+        int const v = warp + r * kThinWarps;
+        if (v < kTaps) dst[v * kCh + lane] = sum[r];
+        else if (v == kTaps && lane == 0) dst[kOutW] = sum[r];
     }
 }
 
-// Weight gradient of the input convolution, per-block partials over
-// dz = dh * (h > 0): part[b][(co*9 + tap)*2 + ci], then 32 bias entries.
+// part[b][(co*9 + tap)*2 + ci] = sum_p dz[p][co] feat[p + tap][ci], then the 32 bias sums, with
+// dz = dh * (h > 0), over the block's tiles.
 __global__ void __launch_bounds__(kThinBlock) inc_wgrad_kernel(const __grid_constant__ Table t, float const* dh,
-                                                               bf16 const* h, float const* feat, float* part,
-                                                               int64_t total_px)
+                                                               bf16 const* h, float const* feat, float* part)
 {
-    int const n = kInW + kCh;
-    float acc[kThinPerThread] = {0.0f, 0.0f, 0.0f};
-    int64_t const p0 = static_cast<int64_t>(blockIdx.x) * kThinPx;
-    for (int64_t p = p0; p < p0 + kThinPx && p < total_px; ++p) {
-        Img const o = t.img[image_of_pixel(t, p)];
-        int64_t const g = p - o.offset;
-        int64_t const P = o.w + 2;
-        int64_t const y = g / P, x = g - y * P;
-        if (y == 0 || x == 0 || y > o.h || x > o.w) continue;
+    constexpr int NV = 2 * kTaps + 1;
+    __shared__ float2 win[3][kHalo + 2];
+    __shared__ float red[kThinWarps * NV * 32];
+    int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float acc[NV] = {};
+    for (int tile = blockIdx.x; tile < t.tile_base[t.nimg]; tile += gridDim.x) {
+        int const im = find_image(t, tile);
+        Img const o = t.img[im];
+        int const P = o.w + 2, npx = P * (o.h + 2), end = P * (o.h + 1);
+        int const start = P + (tile - t.tile_base[im]) * kTilePx;
+        __syncthreads();
+        for (int i = threadIdx.x; i < 3 * kHalo; i += kThinBlock) {
+            int const r = i / kHalo, j = i - r * kHalo, g = start + (r - 1) * P - 1 + j;
+            win[r][j] = g >= 0 && g < npx ? reinterpret_cast<float2 const*>(feat)[o.offset + g] : make_float2(0.0f, 0.0f);
+        }
+        __syncthreads();
+        int const m0 = warp * kThinRun;
+        int64_t const px = (o.offset + start + m0) * kCh + lane;
+        // every load of the run in flight before the first use
+        float dz[kThinRun];
+        bf16 hv[kThinRun];
 #pragma unroll
-        for (int r = 0; r < kThinPerThread; ++r) {
-            int const k = threadIdx.x + r * kThinBlock;
-            if (k >= n) continue;
-            int const co = k < kInW ? k / (kTaps * 2) : k - kInW;
-            float const hv = __bfloat162float(h[p * kCh + co]);
-            if (!(hv > 0.0f)) continue;
-            float const d = dh[p * kCh + co];
-            if (k >= kInW) {
-                acc[r] = acc[r] + d;
-            } else {
-                int const tap = (k / 2) % kTaps, ci = k % 2;
-                int64_t const q = p + (tap / 3 - 1) * P + (tap % 3 - 1);
-                acc[r] = acc[r] + d * feat[2 * q + ci];
+        for (int m = 0; m < kThinRun; ++m) {
+            bool const in = start + m0 + m < end;
+            dz[m] = in ? __ldg(dh + px + m * kCh) : 0.0f;
+            hv[m] = in ? h[px + m * kCh] : __float2bfloat16_rn(0.0f);
+        }
+        float2 f[3][3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            f[r][1] = win[r][m0];
+            f[r][2] = win[r][m0 + 1];
+        }
+#pragma unroll
+        for (int m = 0; m < kThinRun; ++m) {
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                f[r][0] = f[r][1];
+                f[r][1] = f[r][2];
+                f[r][2] = win[r][m0 + m + 2];
             }
+            float const d = __bfloat162float(hv[m]) > 0.0f ? dz[m] : 0.0f;
+#pragma unroll
+            for (int tap = 0; tap < kTaps; ++tap) {
+                acc[2 * tap] = __fmaf_rn(d, f[tap / 3][tap % 3].x, acc[2 * tap]);
+                acc[2 * tap + 1] = __fmaf_rn(d, f[tap / 3][tap % 3].y, acc[2 * tap + 1]);
+            }
+            acc[2 * kTaps] = acc[2 * kTaps] + d;
         }
     }
-    float* dst = part + static_cast<int64_t>(blockIdx.x) * n;
-    for (int r = 0; r < kThinPerThread; ++r) {
-        int const k = threadIdx.x + r * kThinBlock;
-        if (k < n) dst[k] = acc[r];
+    float sum[(NV + 7) / 8];
+    thin_block_sum<NV>(acc, red, sum);
+    float* dst = part + static_cast<int64_t>(blockIdx.x) * (kInW + kCh);
+#pragma unroll
+    for (int r = 0; r < (NV + 7) / 8; ++r) {
+        int const v = warp + r * kThinWarps;
+        if (v < 2 * kTaps) dst[lane * 2 * kTaps + v] = sum[r];
+        else if (v == 2 * kTaps) dst[kInW + lane] = sum[r];
     }
 }
 
@@ -1606,6 +1687,7 @@ public:
     int nwitems = 0;
     DevBuf wparts;                 // weight-gradient partials
     int wgrad_grid = 0;
+    int thin_grid = 0;
     int64_t max_node_per_sample = 0;
     int const* active = nullptr;   // per-sample switch of the current forward (NULL: all)
 
@@ -1714,9 +1796,9 @@ sil_status Workspace::build(std::vector<Sample> const& s)
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     wgrad_grid = 2 * sms;
-    int64_t const thin_blocks = (top + kThinPx - 1) / kThinPx;
+    thin_grid = 4 * sms;
     size_t const wp = std::max<size_t>(static_cast<size_t>(wgrad_grid) * kWgradParts,
-                                       static_cast<size_t>(thin_blocks) * (kInW + kCh));
+                                       static_cast<size_t>(thin_grid) * (kInW + kCh));
     if (sil_status st = wparts.alloc(wp * sizeof(float)); st != SIL_OK) return st;
     return SIL_OK;
 }
@@ -2097,7 +2179,7 @@ sil_status wgrad(Net& net, Workspace& w, cudaStream_t st, Table const& t, int mo
     if (t.nimg == 0 || t.tile_base[t.nimg] == 0) return SIL_OK;
     int const grid = std::min(w.wgrad_grid, t.tile_base[t.nimg]);
     wgrad_kernel<<<grid, 128, wgrad_smem(), st>>>(t, mode, in, in2, dy, y, w.wparts.as<float>(), net.error_flag);
-    reduce_parts_kernel<<<(kWgradParts + 255) / 256, 256, 0, st>>>(w.wparts.as<float>(), grid, kWgradParts, grad_out);
+    reduce_parts_kernel<<<(kWgradParts + 31) / 32, 256, 0, st>>>(w.wparts.as<float>(), grid, kWgradParts, grad_out);
     SIL_CUDA_CHECK(cudaGetLastError());
     return SIL_OK;
 }
@@ -2113,12 +2195,11 @@ sil_status net_backward(Net& net, Workspace& w, cudaStream_t st)
         SIL_CUDA_CHECK(cudaMemsetAsync(w.dg[l].p, 0, a, st));
     }
     Table const t0 = w.table(0, -1, false);
-    int64_t const top = w.levels[0].npx;
-    int const thin_blocks = static_cast<int>((top + kThinPx - 1) / kThinPx);
+    int const thin_blocks = std::min(w.thin_grid, t0.tile_base[t0.nimg]);
     // output convolution
     out_backward_data_kernel<<<image_grid(t0, 1, 0), 256, 0, st>>>(t0, w.gnet.as<float>(), net.params, w.dg[0].as<float>());
-    out_wgrad_kernel<<<thin_blocks, kThinBlock, 0, st>>>(t0, w.gnet.as<float>(), w.g[0].as<bf16>(), w.wparts.as<float>(), top);
-    reduce_parts_kernel<<<(kOutW + 1 + 255) / 256, 256, 0, st>>>(w.wparts.as<float>(), thin_blocks, kOutW + 1,
+    out_wgrad_kernel<<<thin_blocks, kThinBlock, 0, st>>>(t0, w.gnet.as<float>(), w.g[0].as<bf16>(), w.wparts.as<float>());
+    reduce_parts_kernel<<<(kOutW + 1 + 31) / 32, 256, 0, st>>>(w.wparts.as<float>(), thin_blocks, kOutW + 1,
                                                                  net.grad + kOffOut);
     SIL_CUDA_CHECK(cudaGetLastError());
     // decoder, top-down
@@ -2179,8 +2260,8 @@ sil_status net_backward(Net& net, Workspace& w, cudaStream_t st)
     }
     // input convolution
     inc_wgrad_kernel<<<thin_blocks, kThinBlock, 0, st>>>(t0, w.dh[0].as<float>(), w.h[0].as<bf16>(), w.feat.as<float>(),
-                                                         w.wparts.as<float>(), top);
-    reduce_parts_kernel<<<(kInW + kCh + 255) / 256, 256, 0, st>>>(w.wparts.as<float>(), thin_blocks, kInW + kCh,
+                                                         w.wparts.as<float>());
+    reduce_parts_kernel<<<(kInW + kCh + 31) / 32, 256, 0, st>>>(w.wparts.as<float>(), thin_blocks, kInW + kCh,
                                                                   net.grad + kOffIn);
     SIL_CUDA_CHECK(cudaGetLastError());
     return SIL_OK;
