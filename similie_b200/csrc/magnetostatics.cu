@@ -518,6 +518,7 @@ struct Scalars
     double inner_tol2;  // squared relative reduction the inner solve stops at
     double bb;        // b . b (outer right-hand side)
     double alpha, beta;
+    double last_beta; // beta formed after the latest iteration
     double scale;     // outer residual norm used to scale the inner right-hand side
     int done;         // inner / plain solve finished
     int outer_done;   // refinement finished
@@ -532,8 +533,13 @@ struct Scalars
     int learned_iters;
     double pq_hist[kMaxDirs];  // p_j . q_j of the stored directions
     double coef[kMaxDirs];     // (z . q_j) / (p_j . q_j) of the current z
-    // persistent CG
+    // Jacobi-CG iterations (cg_begin): fields a kernel reads are never written
+    // in the same kernel
     int pbuf;                  // buffer (0: p, 1: p2) holding the latest direction
+    int pbuf0;                 // and at the start of the chunk
+    int base_iters;            // total_iters at the start of the chunk
+    int stopped[2];            // by parity of the iteration: it did not run
+    double rz_it[2];           // by parity of the iteration: r . z it starts from
     double scale_prev;         // outer residual norm of the previous refinement pass
     int pending;               // 1: x still lacks alpha times the latest direction
 };
@@ -712,168 +718,457 @@ struct Tile
 // One Jacobi-CG iteration is two kernels over the items of the problems that
 // still iterate (`act`, one CTA per item, so converged problems launch
 // nothing):
-//   cg_dir_apply  p = z + beta p_old (formed on the fly at the row and at its
-//                 stencil neighbours; p double-buffered), q = A p, partial
-//                 p.q; the problem's last CTA forms alpha
-//   cg_update     x += alpha p, r -= alpha q, z = D^-1 r, partials r.z and
-//                 r.r; the last CTA forms beta, counts the iteration, flips
-//                 the direction buffer and decides convergence
+//   direction  p = z + beta p_old (formed on the fly at the row and at its
+//              stencil neighbours; p double-buffered), x += alpha p_old of the
+//              previous iteration, q = A p, partial p.q
+//   update     r -= alpha q, z = D^-1 r, partials r.z and r.r
 // Chunks of iterations are captured as a CUDA graph, captured again when the
 // set of iterating problems changes.
+//
+// No CTA waits for another one's partial: each kernel starts by summing the
+// previous kernel's partials itself (every CTA of a problem the same values in
+// the same order) and forms beta, the stop test or alpha from them; the
+// problem's first CTA records them.  Small problems are bound by the latency of
+// this chain (5.3 + 4.1 us a pair of kernels at 128^2), large ones by memory:
+// at the 21 M nodes of 60 problems in FP64 the direction takes 220 us for its
+// seven vectors (5.3 TB/s), the update 127 for its five (6.6 TB/s).  B200, per
+// iteration of a whole solve, against partials counted in by an atomic and
+// summed by the last CTA, four dependent loads of descriptors, and a thread per
+// row loading its own stencil: four problems of 96^2 .. 161^2 23.1 -> 11.2 us,
+// 512^2 23.3 -> 12.7, 1024^2 26.9 -> 19.8, those 60 problems 549 -> 373 (FP64)
+// and 382 -> 267 (FP32).
 
-template <class T, bool G = false>
-__global__ void __launch_bounds__(kThreads) cg_dir_apply_kernel(Item const* items, int const* act, ProbInfo const* info,
-                                                                Vecs<T> const* vecs, Scalars* sc, double* part)
+// Everything a CTA needs to know of its item, in one 128-byte record.
+template <class T>
+struct alignas(16) Work
 {
-    __shared__ double red[kThreads / 32];
-    Item const it = items[act[blockIdx.x]];
-    Scalars* s = sc + it.prob;
-    if (s->done || s->outer_done) return;
-    ProbInfo const pi = info[it.prob];
-    Vecs<T> const v = vecs[it.prob];
-    int const pb = s->pbuf;
-    T const* pold = pb == 0 ? v.p : v.p2;
-    T* pnew = pb == 0 ? v.p2 : v.p;
-    T const beta = static_cast<T>(s->beta);
-    T const* z = v.z;
-    auto dir = [&](int idx) -> T { return z[idx] + beta * pold[idx]; };
-    double pq = 0.0;
-    if (pi.dim == 3) {
-        // 3D: the direction was formed by cg_direction3_kernel (the curl-curl
-        // stencil reads each operand many times, so forming it on the fly
-        // would double those loads)
-        for (int64_t node = it.begin / 3 + threadIdx.x; node < it.end / 3; node += kThreads) {
-            T q[3];
-            mag3d_apply_node<T, G>(pnew, v.nu, pi, static_cast<int>(node), q);
-            for (int cc = 0; cc < 3; ++cc) {
-                int const row = static_cast<int>(3 * node + cc);
-                v.q[row] = q[cc];
-                pq += static_cast<double>(pnew[row]) * static_cast<double>(q[cc]);
-            }
-        }
-    } else {
-        // (i, j) of the thread's rows advance by adding: no division per row
-        int const nx = static_cast<int>(pi.nx);
-        int row = static_cast<int>(it.begin) + threadIdx.x;
-        int j = row / nx, i = row - j * nx;
-        for (; row < it.end; row += kThreads) {
-            T const q = mag_apply_node_ij<T>(dir, v.nu, nx, static_cast<int>(pi.ny), row, i, j);
-            T const pr = dir(row);
-            pnew[row] = pr;
-            v.q[row] = q;
-            pq += static_cast<double>(pr) * static_cast<double>(q);
-            i += kThreads;
-            while (i >= nx) {
-                i -= nx;
-                ++j;
-            }
-        }
+    T* x;
+    T* r;
+    T* z;
+    T* p;
+    T* p2;
+    T* q;
+    T const* dinv;
+    T const* nu;
+    Scalars* s;
+    double* part_pq;
+    double* part_rz;
+    double* part_rr;
+    int begin, end;     // rows of the item
+    int index;          // item (partial) number within the problem
+    int npart, npq;     // partials of r.z and r.r, and of p.q
+    int max_iters;
+};
+
+// Sums of two strided lists of n partials, the same in every thread of every
+// CTA: thread t adds entries t, t + kThreads, ... in order, then a butterfly
+// per warp, then the warps in order.
+__device__ __forceinline__ void sum_partials(double const* a, double const* b, int n, double* smem, double& ta,
+                                             double& tb)
+{
+    double va = 0.0, vb = 0.0;
+    for (int j = threadIdx.x; j < n; j += kThreads) {
+        va += __ldcg(a + j);
+        if (b != nullptr) vb += __ldcg(b + j);
     }
-    double const pq_b = block_sum(pq, red);
-    double tot = 0.0;
-    if (finish_reduction(pq_b, part, it.index, pi.first_item, pi.nitems, &s->counter_a, &tot)) {
-        s->alpha = s->rz / tot;
-        if (!isfinite(s->alpha)) s->nonfinite = 1;
+    for (int o = 16; o > 0; o >>= 1) {
+        va += __shfl_xor_sync(0xffffffffu, va, o);
+        vb += __shfl_xor_sync(0xffffffffu, vb, o);
+    }
+    int const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    if (lane == 0) {
+        smem[warp] = va;
+        smem[kThreads / 32 + warp] = vb;
+    }
+    __syncthreads();
+    ta = tb = 0.0;
+    for (int w = 0; w < kThreads / 32; ++w) {
+        ta += smem[w];
+        tb += smem[kThreads / 32 + w];
     }
 }
 
-// The first half of an iteration for batches of 3D penalty-gauge problems, in
-// marching tiles: p = z + beta p_old, q = A p, the partials of p.q, and the
-// previous iteration's x += alpha p_old, which rides on the read of p_old
-// (`pending`: a chunk's last one is added by refine_kernel).  Against a
-// direction pass, a node-per-thread apply and x in the update, an iteration
-// moves 11.3 vectors instead of 13.3 and launches two kernels instead of three.
-// B200, per iteration of one 160^3 problem: FP64 392 -> 293 us, FP32 270 -> 217
-// (this kernel 155 and 106 us of it).
+struct Begin
+{
+    bool run;        // the iteration runs
+    bool pending;    // x still lacks alpha p_old
+    double alpha;    // of the previous iteration
+    double beta;
+    int pbuf;        // buffer of p_old
+};
+
+// Start of iteration c of a chunk (c > 0: completes iteration c - 1 from its
+// partials).  lead: this CTA records the problem's state.  Every thread of the
+// block calls it; smem holds 2 * kThreads / 32 doubles.
+__device__ __forceinline__ Begin cg_begin(Scalars* s, int c, double const* part_rz, double const* part_rr, int npart,
+                                          int max_iters, bool lead, double* smem)
+{
+    Begin b {};
+    int const now = c & 1, before = now ^ 1;
+    if (s->outer_done || (c == 0 ? s->done : s->stopped[before])) {
+        if (lead && threadIdx.x == 0) s->stopped[now] = 1;
+        return b;
+    }
+    b.pbuf = s->pbuf0 ^ now;
+    if (c == 0) {
+        b.run = true;
+        b.beta = s->beta;
+        if (lead && threadIdx.x == 0) {
+            s->rz_it[0] = s->rz;
+            s->stopped[0] = 0;
+        }
+        return b;
+    }
+    double const rz_old = s->rz_it[before];
+    double rz = 0.0, rr = 0.0;
+    sum_partials(part_rz, part_rr, npart, smem, rz, rr);
+    b.pending = true;
+    b.alpha = s->alpha;
+    b.beta = rz / rz_old;
+    bool const bad = !isfinite(rr) || !isfinite(rz);
+    b.run = !(rr <= s->inner_tol2 * s->rr0 || bad || s->base_iters + c >= max_iters);
+    if (lead && threadIdx.x == 0) {
+        s->rz_it[now] = rz;
+        s->stopped[now] = b.run ? 0 : 1;
+        s->rz = rz;
+        s->rr = rr;
+        s->last_beta = b.beta;
+        s->iters = c;
+        s->total_iters = s->base_iters + c;
+        s->pbuf = b.pbuf;
+        s->pending = 1;
+        if (bad) s->nonfinite = 1;
+    }
+    return b;
+}
+
+// ---- 2D strips: the 2D operator marched down a strip of columns, a warp per
+// strip.  Lane l holds column c0 - 1 + l; lanes 1..30 own theirs.  Walking down
+// the rows a column's operand and reluctivity at rows j - 1 and j stay in
+// registers and its neighbours' come from the next lanes, so a node costs one
+// load per input array where a thread per node made fourteen; four rows' loads
+// are in flight before the first is used.  The values are those of
+// mag_apply_node_ij (an excluded term adds a zero).
+constexpr int kStripCols = 30;
+constexpr int kStripBatch = 4;   // rows whose loads are issued together
+
+// Strips of a problem: strip w % strips of row block w / strips, `rows` rows each.
+struct Strips
+{
+    int strips;    // per row block
+    int rows;      // per strip, a multiple of kStripBatch
+    int count;     // in all
+    int ctas;      // of kThreads / 32 strips
+};
+
+__host__ __device__ inline Strips strips_of(int64_t nx, int64_t ny, int rows)
+{
+    Strips s {};
+    s.strips = static_cast<int>((nx + kStripCols - 1) / kStripCols);
+    s.rows = rows;
+    s.count = s.strips * static_cast<int>((ny + rows - 1) / rows);
+    s.ctas = (s.count + kThreads / 32 - 1) / (kThreads / 32);
+    return s;
+}
+
+// Rows per strip: the fewest, in steps of four, at which the batch fits one
+// wave of two CTAs per multiprocessor; 32 at most (a strip of R rows reads
+// R + 2, and one wave of longer ones leaves too few loads in flight).
+int strip_rows(std::vector<ProbInfo> const& grids)
+{
+    int rows = kStripBatch;
+    for (; rows < 32; rows += kStripBatch) {
+        int64_t ctas = 0;
+        for (ProbInfo const& g : grids) ctas += strips_of(g.nx, g.ny, rows).ctas;
+        if (ctas <= 2 * static_cast<int64_t>(sm_count())) break;
+    }
+    return rows;
+}
+
+// Src: Raw load(row), T value(Raw), and out(row, q, raw): the result of an
+// owned row and its operand.
+template <class T, class Src, class Out>
+__device__ __forceinline__ void mag2d_strip(Src const& src, T const* __restrict__ nu, int nx, int ny, int c0, int j0,
+                                            int j1, Out const& out)
+{
+    constexpr int U = kStripBatch;
+    int const lane = threadIdx.x & 31, i = c0 - 1 + lane, ic = min(max(i, 0), nx - 1);
+    bool const own = lane > 0 && lane <= kStripCols && i < nx, col_in = i > 0 && i + 1 < nx, left_in = i >= 2;
+    auto row_of = [&](int j) { return ic + nx * min(max(j, 0), ny - 1); };
+    typename Src::Raw const raw_m = src.load(row_of(j0 - 1));
+    typename Src::Raw raw_c = src.load(row_of(j0));
+    T n_m = nu[row_of(j0 - 1)], n_c = nu[row_of(j0)];
+    T below = T(0), centre = T(0);
+    bool first = true;
+    for (int j = j0; j < j1; j += U) {
+        typename Src::Raw raw[U];
+        typename Src::Own mine[U];
+        T n[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            int const at = row_of(j + 1 + u);
+            raw[u] = src.load(at);
+            n[u] = nu[at];
+            mine[u] = src.own(row_of(j + u));
+        }
+        if (first) {
+            below = src.value(raw_m);
+            centre = src.value(raw_c);
+            first = false;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            T const above = src.value(raw[u]);
+            T const left = __shfl_up_sync(0xffffffffu, centre, 1), right = __shfl_down_sync(0xffffffffu, centre, 1);
+            T const n_l = __shfl_up_sync(0xffffffffu, n_c, 1);
+            int const jj = j + u;
+            T res = T(0);
+            if (jj >= 2) res = res + (centre - below) * n_m;
+            res = res - (above - centre) * n_c;
+            if (left_in) res = res - (left - centre) * n_l;
+            res = res + (centre - right) * n_c;
+            bool const in = col_in && jj > 0 && jj + 1 < ny;
+            if (own && jj < j1) out(ic + nx * jj, in ? res : centre, centre, raw_c, mine[u]);
+            below = centre;
+            centre = above;
+            raw_c = raw[u];
+            n_m = n_c;
+            n_c = n[u];
+        }
+    }
+}
+
+// Operand z + beta p_old of the search direction, x on the side.
+template <class T>
+struct StripDirection
+{
+    struct Raw
+    {
+        T z, p;
+    };
+    using Own = T;
+    T const* __restrict__ z;
+    T const* __restrict__ pold;
+    T const* x;
+    T beta;
+    bool pending;
+    __device__ __forceinline__ Raw load(int row) const { return {z[row], pold[row]}; }
+    __device__ __forceinline__ Own own(int row) const { return pending ? x[row] : T(0); }
+    __device__ __forceinline__ T value(Raw const& r) const { return r.z + beta * r.p; }
+};
+
+// A stored operand, b on the side.
+struct StripResidual
+{
+    using Raw = double;
+    using Own = double;
+    double const* __restrict__ a;
+    double const* __restrict__ b;
+    __device__ __forceinline__ Raw load(int row) const { return a[row]; }
+    __device__ __forceinline__ Own own(int row) const { return b[row]; }
+    __device__ __forceinline__ double value(Raw r) const { return r; }
+};
+
+// A CTA of strips.
+template <class T>
+struct alignas(16) StripWork
+{
+    T* x;
+    T const* z;
+    T* p;
+    T* p2;
+    T* q;
+    T const* nu;
+    Scalars* s;
+    double* part_pq;
+    double const* part_rz;
+    double const* part_rr;
+    int nx, ny;
+    int strips, rows, count;   // Strips of the problem
+    int first;                 // the CTA's first strip
+    int index;                 // CTA (partial) number within the problem
+    int prob;
+    int npart, max_iters;
+};
+
+template <class T>
+__global__ void __launch_bounds__(kThreads, 2) cg_direction2_kernel(StripWork<T> const* work, int c)
+{
+    __shared__ double red[2 * kThreads / 32];
+    StripWork<T> const w = work[blockIdx.x];
+    Begin const b = cg_begin(w.s, c, w.part_rz, w.part_rr, w.npart, w.max_iters, w.index == 0, red);
+    if (!b.run) return;
+    T* __restrict__ pnew = b.pbuf == 0 ? w.p2 : w.p;
+    T* __restrict__ x = w.x;
+    T* __restrict__ q = w.q;
+    StripDirection<T> const src {w.z, b.pbuf == 0 ? w.p : w.p2, w.x, static_cast<T>(b.beta), b.pending};
+    T const alpha = static_cast<T>(b.alpha);
+    double pq = 0.0;
+    int const strip = w.first + static_cast<int>(threadIdx.x) / 32;
+    if (strip < w.count) {
+        int const block = strip / w.strips, j0 = block * w.rows;
+        mag2d_strip<T>(src, w.nu, w.nx, w.ny, (strip - block * w.strips) * kStripCols, j0, min(w.ny, j0 + w.rows),
+                       [&](int row, T qr, T pr, typename StripDirection<T>::Raw const& raw, T xr) {
+                           if (b.pending) x[row] = xr + alpha * raw.p;
+                           pnew[row] = pr;
+                           q[row] = qr;
+                           pq += static_cast<double>(pr) * static_cast<double>(qr);
+                       });
+    }
+    __syncthreads();
+    double const t = block_sum(pq, red);
+    if (threadIdx.x == 0) w.part_pq[w.index] = t;
+}
+
+template <class T>
+__global__ void __launch_bounds__(kThreads) cg_update_kernel(Work<T> const* work, int c)
+{
+    __shared__ double red[2 * kThreads / 32];
+    Work<T> const w = work[blockIdx.x];
+    Scalars* s = w.s;
+    if (s->stopped[c & 1]) return;
+    T* __restrict__ r = w.r;
+    T* __restrict__ z = w.z;
+    T const* __restrict__ q = w.q;
+    T const* __restrict__ dinv = w.dinv;
+    // the first rows' loads are issued before the partials are summed
+    constexpr int U = 4;
+    T rv[U], qv[U], dv[U];
+    int row = w.begin + static_cast<int>(threadIdx.x);
+    auto fetch = [&](int from) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            int const at = min(from + u * kThreads, w.end - 1);
+            rv[u] = r[at];
+            qv[u] = q[at];
+            dv[u] = dinv[at];
+        }
+    };
+    fetch(row);
+    double pq, none;
+    sum_partials(w.part_pq, nullptr, w.npq, red, pq, none);
+    double const a = s->rz_it[c & 1] / pq;
+    if (w.index == 0 && threadIdx.x == 0) {
+        s->alpha = a;
+        if (!isfinite(a)) s->nonfinite = 1;
+    }
+    T const alpha = static_cast<T>(a);
+    double rz = 0.0, rr = 0.0;
+    for (; row < w.end; row += U * kThreads) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (row + u * kThreads >= w.end) continue;
+            T const rn = rv[u] - alpha * qv[u], zn = dv[u] * rn;
+            r[row + u * kThreads] = rn;
+            z[row + u * kThreads] = zn;
+            rz += static_cast<double>(rn) * static_cast<double>(zn);
+            rr += static_cast<double>(rn) * static_cast<double>(rn);
+        }
+        fetch(row + U * kThreads);
+    }
+    __syncthreads();
+    double const rz_b = block_sum(rz, red), rr_b = block_sum(rr, red);
+    if (threadIdx.x == 0) {
+        w.part_rz[w.index] = rz_b;
+        w.part_rr[w.index] = rr_b;
+    }
+}
+
+// End of a chunk of `c` iterations: completes the last one (one CTA per item;
+// only each problem's first works).
+template <class T>
+__global__ void __launch_bounds__(kThreads) cg_close_kernel(Work<T> const* work, int c)
+{
+    __shared__ double red[2 * kThreads / 32];
+    Work<T> const w = work[blockIdx.x];
+    if (w.index != 0) return;
+    Begin const b = cg_begin(w.s, c, w.part_rz, w.part_rr, w.npart, w.max_iters, true, red);
+    __syncthreads();
+    if (threadIdx.x == 0 && !w.s->outer_done) {
+        w.s->done = b.run ? 0 : 1;
+        w.s->beta = w.s->last_beta;
+    }
+}
+
+// The direction kernel for batches of 3D penalty-gauge problems, in marching
+// tiles (mag3d_march.cuh): p = z + beta p_old, x += alpha p_old on the read of
+// p_old, q = A p, the partials of p.q.  B200, per iteration of one 160^3 problem
+// against a direction pass, a node-per-thread apply and x in the update: FP64
+// 392 -> 293 us, FP32 270 -> 217 (this kernel 155 and 106 us of it).
 template <class T>
 __global__ void __launch_bounds__(kMarchThreads, sizeof(T) == 8 ? 3 : 4)
         cg_march_kernel(Tile const* tiles, int const* act, ProbInfo const* info, Vecs<T> const* vecs, Scalars* sc,
-                        double* part)
+                        double* part_pq, double const* part_rz, double const* part_rr, int c)
 {
     extern __shared__ __align__(16) unsigned char march_smem[];
     auto& sm = *reinterpret_cast<MarchSmem<T, MarchDirection<T>>*>(march_smem);
-    __shared__ double red[kThreads / 32];
+    __shared__ double red[2 * kThreads / 32];
     static_assert(kMarchThreads == kThreads, "block_sum covers the block");
     Tile const t = tiles[act[blockIdx.x]];
-    Scalars* s = sc + t.prob;
-    if (s->done || s->outer_done) return;
     ProbInfo const& pi = info[t.prob];
+    Begin const b = cg_begin(sc + t.prob, c, part_rz + pi.first_item, part_rr + pi.first_item, pi.nitems, pi.max_iters,
+                             t.index == 0, red);
+    if (!b.run) return;
     Vecs<T> const v = vecs[t.prob];
-    bool const first = s->pbuf == 0;
-    MarchDirection<T> const src {v.z, first ? v.p : v.p2, first ? v.p2 : v.p, v.x, static_cast<T>(s->alpha),
-                                 static_cast<T>(s->beta), s->pending != 0};
+    bool const first = b.pbuf == 0;
+    MarchDirection<T> const src {v.z, first ? v.p : v.p2, first ? v.p2 : v.p, v.x, static_cast<T>(b.alpha),
+                                 static_cast<T>(b.beta), b.pending};
     double pq = 0.0;
     mag3d_march(sm, march_grid<T>(pi), static_cast<T const*>(v.nu), src, t.i0, t.j0, t.k0, t.k1, [&](int row, T q, T p) {
         v.q[row] = q;
         pq += static_cast<double>(p) * static_cast<double>(q);
     });
+    __syncthreads();
     double const pq_b = block_sum(pq, red);
-    double tot = 0.0;
-    if (finish_reduction(pq_b, part, t.index, pi.first_tile, pi.ntiles, &s->counter_a, &tot)) {
-        s->alpha = s->rz / tot;
-        if (!isfinite(s->alpha)) s->nonfinite = 1;
+    if (threadIdx.x == 0) part_pq[pi.first_tile + t.index] = pq_b;
+}
+
+// Batches with the divergence gauge, whose stencil reaches two nodes: the
+// direction as a pass of its own, then the apply, a thread per node.
+template <class T>
+__global__ void __launch_bounds__(kThreads) cg_direction3_kernel(Work<T> const* work, int c)
+{
+    __shared__ double red[2 * kThreads / 32];
+    Work<T> const w = work[blockIdx.x];
+    Begin const b = cg_begin(w.s, c, w.part_rz, w.part_rr, w.npart, w.max_iters, w.index == 0, red);
+    if (!b.run) return;
+    T const* __restrict__ z = w.z;
+    T const* __restrict__ pold = b.pbuf == 0 ? w.p : w.p2;
+    T* __restrict__ pnew = b.pbuf == 0 ? w.p2 : w.p;
+    T* __restrict__ x = w.x;
+    T const beta = static_cast<T>(b.beta), alpha = static_cast<T>(b.alpha);
+#pragma unroll 4
+    for (int row = w.begin + static_cast<int>(threadIdx.x); row < w.end; row += kThreads) {
+        T const po = pold[row];
+        pnew[row] = z[row] + beta * po;
+        if (b.pending) x[row] = x[row] + alpha * po;
     }
 }
 
-// p = z + beta p_old into the other direction buffer, for the 3D problems of
-// the batch (2D problems form it inside cg_dir_apply_kernel).
 template <class T>
-__global__ void __launch_bounds__(kThreads) cg_direction3_kernel(Item const* items, int const* act, ProbInfo const* info,
-                                                                 Vecs<T> const* vecs, Scalars const* sc)
-{
-    Item const it = items[act[blockIdx.x]];
-    Scalars const* s = sc + it.prob;
-    if (s->done || s->outer_done || info[it.prob].dim != 3) return;
-    Vecs<T> const v = vecs[it.prob];
-    T const* pold = s->pbuf == 0 ? v.p : v.p2;
-    T* pnew = s->pbuf == 0 ? v.p2 : v.p;
-    T const beta = static_cast<T>(s->beta);
-    for (int64_t row = it.begin + threadIdx.x; row < it.end; row += kThreads) pnew[row] = v.z[row] + beta * pold[row];
-}
-
-// DEFER: x is left to the next iteration's cg_march_kernel.
-template <class T, bool DEFER>
-__global__ void __launch_bounds__(kThreads) cg_update_kernel(Item const* items, int const* act, ProbInfo const* info,
-                                                             Vecs<T> const* vecs, Scalars* sc, double* part_a,
-                                                             double* part_b)
+__global__ void __launch_bounds__(kThreads) cg_apply3_kernel(Item const* items, int const* act, ProbInfo const* info,
+                                                             Vecs<T> const* vecs, Scalars const* sc, double* part_pq,
+                                                             int c)
 {
     __shared__ double red[kThreads / 32];
     Item const it = items[act[blockIdx.x]];
-    Scalars* s = sc + it.prob;
-    if (s->done || s->outer_done) return;
+    Scalars const* s = sc + it.prob;
+    if (s->stopped[c & 1]) return;
     ProbInfo const pi = info[it.prob];
     Vecs<T> const v = vecs[it.prob];
-    T const* pcur = s->pbuf == 0 ? v.p2 : v.p;
-    T const alpha = static_cast<T>(s->alpha);
-    double rz = 0.0, rr = 0.0;
-    for (int64_t row = it.begin + threadIdx.x; row < it.end; row += kThreads) {
-        T x = T(0);
-        if constexpr (!DEFER) x = v.x[row] + alpha * pcur[row];
-        T const r = v.r[row] - alpha * v.q[row];
-        T const z = v.dinv[row] * r;
-        if constexpr (!DEFER) v.x[row] = x;
-        v.r[row] = r;
-        v.z[row] = z;
-        rz += static_cast<double>(r) * static_cast<double>(z);
-        rr += static_cast<double>(r) * static_cast<double>(r);
+    T const* p = (s->pbuf0 ^ (c & 1)) == 0 ? v.p2 : v.p;
+    double pq = 0.0;
+    for (int64_t node = it.begin / 3 + threadIdx.x; node < it.end / 3; node += kThreads) {
+        T q[3];
+        mag3d_apply_node<T, true>(p, v.nu, pi, static_cast<int>(node), q);
+        for (int cc = 0; cc < 3; ++cc) {
+            int const row = static_cast<int>(3 * node + cc);
+            v.q[row] = q[cc];
+            pq += static_cast<double>(p[row]) * static_cast<double>(q[cc]);
+        }
     }
-    double const rz_b = block_sum(rz, red);
-    double const rr_b = block_sum(rr, red);
-    double const vals[2] = {rz_b, rr_b};
-    double* parts[2] = {part_a, part_b};
-    double tot[2];
-    if (finish_reduction_k<2>(vals, parts, it.index, pi.first_item, pi.nitems, &s->counter_b, tot)) {
-        double const trz = tot[0], tot_rr = tot[1];
-        s->beta = trz / s->rz;
-        s->rz = trz;
-        s->rr = tot_rr;
-        s->iters += 1;
-        s->total_iters += 1;
-        s->pbuf ^= 1;
-        if (DEFER) s->pending = 1;
-        if (!isfinite(tot_rr) || !isfinite(trz)) s->nonfinite = 1;
-        if (tot_rr <= s->inner_tol2 * s->rr0 || s->nonfinite || s->total_iters >= pi.max_iters) s->done = 1;
-    }
+    double const pq_b = block_sum(pq, red);
+    if (threadIdx.x == 0) part_pq[pi.first_item + it.index] = pq_b;
 }
 
 // Start or continue the CG of a refinement pass on the new outer residual:
@@ -899,14 +1194,20 @@ __global__ void __launch_bounds__(kThreads) cg_replace_kernel(Item const* items,
     ProbInfo const pi = info[it.prob];
     Vecs<T> const v = vecs[it.prob];
     double const scale = s->scale;
-    T* pold = s->pbuf == 0 ? v.p : v.p2;
+    double const* __restrict__ src = r64[it.prob];
+    T const* __restrict__ dinv = v.dinv;
+    T* __restrict__ x = v.x;
+    T* __restrict__ rv = v.r;
+    T* __restrict__ zv = v.z;
+    T* __restrict__ pold = s->pbuf == 0 ? v.p : v.p2;
     double rz = 0.0, rr = 0.0;
-    for (int64_t row = it.begin + threadIdx.x; row < it.end; row += kThreads) {
-        T const r = static_cast<T>(r64[it.prob][row] / scale);
-        T const z = v.dinv[row] * r;
-        v.x[row] = T(0);
-        v.r[row] = r;
-        v.z[row] = z;
+#pragma unroll 4
+    for (int row = static_cast<int>(it.begin) + threadIdx.x; row < static_cast<int>(it.end); row += kThreads) {
+        T const r = static_cast<T>(src[row] / scale);
+        T const z = dinv[row] * r;
+        x[row] = T(0);
+        rv[row] = r;
+        zv[row] = z;
         if (fresh) pold[row] = z;
         rz += static_cast<double>(r) * static_cast<double>(z);
         rr += static_cast<double>(r) * static_cast<double>(r);
@@ -923,6 +1224,8 @@ __global__ void __launch_bounds__(kThreads) cg_replace_kernel(Item const* items,
         bool const keep = !fresh && s->iters > 0 && s->rz > 0.0 && s->scale_prev > 0.0;
         s->beta = keep ? s->beta * trz / ((s->scale_prev / scale) * s->rz) : 0.0;
         if (fresh) s->pbuf = 0;
+        s->pbuf0 = s->pbuf;
+        s->base_iters = s->total_iters;
         s->pending = 0;
         s->rz = trz;
         s->rr = tot_rr;
@@ -1203,6 +1506,36 @@ __global__ void __launch_bounds__(kThreads) residual64_kernel(Item const* items,
         residual_done(s, tot, tol2, floor2, mark);
 }
 
+// The same for 2D batches, in strips.
+template <class T>
+__global__ void __launch_bounds__(kThreads, 2)
+        residual64_strip_kernel(StripWork<T> const* work, double const* const* nu64, double const* const* rhs,
+                                double* const* x64, double* const* r64, double tol2, double floor2, int mark)
+{
+    __shared__ double red[kThreads / 32];
+    StripWork<T> const w = work[blockIdx.x];
+    Scalars* s = w.s;
+    if (s->outer_done) return;
+    double* r64p = r64[w.prob];
+    double rr = 0.0;
+    int const strip = w.first + static_cast<int>(threadIdx.x) / 32;
+    if (strip < w.count) {
+        int const block = strip / w.strips, j0 = block * w.rows;
+        mag2d_strip<double>(StripResidual {x64[w.prob], rhs[w.prob]}, nu64[w.prob], w.nx, w.ny,
+                            (strip - block * w.strips) * kStripCols, j0, min(w.ny, j0 + w.rows),
+                            [&](int row, double ax, double, double, double b) {
+                                double const r = b - ax;
+                                r64p[row] = r;
+                                rr += r * r;
+                            });
+    }
+    double const rr_b = block_sum(rr, red);
+    double tot = 0.0;
+    int const ctas = (w.count + kThreads / 32 - 1) / (kThreads / 32);
+    if (finish_reduction(rr_b, w.part_pq, w.index, 0, ctas, &s->counter_a, &tot))
+        residual_done(s, tot, tol2, floor2, mark);
+}
+
 // The same for batches of 3D penalty-gauge problems, in marching tiles.
 __global__ void __launch_bounds__(kMarchThreads, 4)
         residual64_march_kernel(Tile const* tiles, int const* act, ProbInfo const* info, double const* const* nu64,
@@ -1238,18 +1571,22 @@ __global__ void __launch_bounds__(kThreads) refine_kernel(Item const* items, int
     Item const it = items[act != nullptr ? act[blockIdx.x] : blockIdx.x];
     Scalars const* s = sc + it.prob;
     if (s->outer_done) return;
-    T const* e = vecs[it.prob].x;
+    T const* __restrict__ e = vecs[it.prob].x;
+    double* __restrict__ x = x64[it.prob];
     double const scale = s->scale;
+    int const end = static_cast<int>(it.end);
     if (s->pending) {
         // the last iteration's step is still to be added to x
-        T const* p = s->pbuf == 0 ? vecs[it.prob].p : vecs[it.prob].p2;
+        T const* __restrict__ p = s->pbuf == 0 ? vecs[it.prob].p : vecs[it.prob].p2;
         T const alpha = static_cast<T>(s->alpha);
-        for (int64_t row = it.begin + threadIdx.x; row < it.end; row += kThreads)
-            x64[it.prob][row] += scale * static_cast<double>(e[row] + alpha * p[row]);
+#pragma unroll 4
+        for (int row = static_cast<int>(it.begin) + threadIdx.x; row < end; row += kThreads)
+            x[row] += scale * static_cast<double>(e[row] + alpha * p[row]);
         return;
     }
-    for (int64_t row = it.begin + threadIdx.x; row < it.end; row += kThreads)
-        x64[it.prob][row] += scale * static_cast<double>(e[row]);
+#pragma unroll 4
+    for (int row = static_cast<int>(it.begin) + threadIdx.x; row < end; row += kThreads)
+        x[row] += scale * static_cast<double>(e[row]);
 }
 
 // nu = 1/mu per node (FP64 and, for the inner solve, the precision T) and
@@ -1478,7 +1815,17 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
                                             static_cast<int>(sizeof(MarchSmem<T, MarchDirection<T>>))));
     }
     int const ntiles = static_cast<int>(tiles.size());
-    int const nparts = std::max(nitems, ntiles);
+    // Strips of a 2D batch.
+    bool const flat = std::all_of(probs.begin(), probs.end(), [](ProblemDesc const& q) { return q.dim == 2; });
+    int nstrip_ctas = 0;
+    int const srows = flat ? strip_rows(info) : 0;
+    std::vector<int> strip_part(np, 0);   // first strip CTA of each problem
+    if (flat)
+        for (int p = 0; p < np; ++p) {
+            strip_part[p] = nstrip_ctas;
+            nstrip_ctas += strips_of(info[p].nx, info[p].ny, srows).ctas;
+        }
+    int const nparts = std::max(std::max(nitems, ntiles), nstrip_ctas);
     int const nvec = 8;  // x r z p q dinv nu p2 in precision T
     size_t const vec_bytes = ((total_rows * sizeof(T) + 255) / 256) * 256;
     size_t const d_bytes = ((total_rows * sizeof(double) + 255) / 256) * 256;
@@ -1505,7 +1852,8 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
     bytes += sizeof(Item) * nitems + sizeof(ProbInfo) * np + sizeof(Vecs<T>) * np + sizeof(Scalars) * np
              + 3 * sizeof(double) * nparts + kMaxDirs * sizeof(double) * nitems + 7 * sizeof(void*) * np
              + sp64.size() * (sizeof(double) + sizeof(float)) + sizeof(int) * np + sizeof(int) * nitems
-             + (sizeof(Tile) + sizeof(int)) * ntiles + 25 * 256;
+             + (sizeof(Tile) + sizeof(int)) * ntiles + sizeof(Work<T>) * nitems
+             + sizeof(StripWork<T>) * nstrip_ctas + 27 * 256;
     DeviceBuffer buf;
     SIL_CUDA_CHECK(cudaMalloc(&buf.ptr, bytes));
     char* base = static_cast<char*>(buf.ptr);
@@ -1531,6 +1879,8 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
     double* part_h = reinterpret_cast<double*>(take(sizeof(double) * kMaxDirs * nitems));
     int* d_active = reinterpret_cast<int*>(take(sizeof(int) * np));
     int* d_act = reinterpret_cast<int*>(take(sizeof(int) * nitems));
+    Work<T>* d_work = reinterpret_cast<Work<T>*>(take(sizeof(Work<T>) * nitems));
+    StripWork<T>* d_strips = reinterpret_cast<StripWork<T>*>(take(sizeof(StripWork<T>) * nstrip_ctas));
     Tile* d_tiles = reinterpret_cast<Tile*>(take(sizeof(Tile) * ntiles));
     int* d_tact = reinterpret_cast<int*>(take(sizeof(int) * ntiles));
     char* gauge_base = gauge_bytes > 0 ? take(gauge_bytes) : nullptr;
@@ -1632,9 +1982,10 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
     std::vector<int> open_host;
     open_host.reserve(nitems);
     int captured_n = -1;
-    bool const any3d = std::any_of(probs.begin(), probs.end(), [](ProblemDesc const& q) { return q.dim == 3; });
     std::vector<int> open_tiles;
-    int captured_tiles = 0;
+    std::vector<Work<T>> work;
+    std::vector<StripWork<T>> swork;
+    int captured_tiles = 0, captured_strips = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     auto build_open = [&]() {
@@ -1652,6 +2003,33 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
         graph = nullptr;
         int const n = static_cast<int>(open_host.size()), nt = static_cast<int>(open_tiles.size());
         SIL_CUDA_CHECK(cudaMemcpyAsync(d_act, open_host.data(), sizeof(int) * n, cudaMemcpyHostToDevice, stream));
+        work.clear();
+        for (int i : open_host) {
+            Item const& it = items[i];
+            ProbInfo const& pi = info[it.prob];
+            Vecs<T> const& v = vecs[it.prob];
+            work.push_back({v.x, v.r, v.z, v.p, v.p2, v.q, v.dinv, v.nu, d_sc + it.prob,
+                            part_a + (march ? pi.first_tile : (flat ? strip_part[it.prob] : pi.first_item)),
+                            part_b + pi.first_item, part_c + pi.first_item, static_cast<int>(it.begin),
+                            static_cast<int>(it.end), it.index, pi.nitems,
+                            march ? pi.ntiles : (flat ? strips_of(pi.nx, pi.ny, srows).ctas : pi.nitems), pi.max_iters});
+        }
+        swork.clear();
+        for (int p = 0; flat && p < np; ++p) {
+            if (hs[p].outer_done) continue;
+            ProbInfo const& pi = info[p];
+            Vecs<T> const& v = vecs[p];
+            Strips const st = strips_of(pi.nx, pi.ny, srows);
+            for (int k = 0; k < st.ctas; ++k)
+                swork.push_back({v.x, v.z, v.p, v.p2, v.q, v.nu, d_sc + p, part_a + strip_part[p], part_b + pi.first_item,
+                                 part_c + pi.first_item, static_cast<int>(pi.nx), static_cast<int>(pi.ny), st.strips,
+                                 st.rows, st.count, k * (kThreads / 32), k, p, pi.nitems, pi.max_iters});
+        }
+        int const ns = static_cast<int>(swork.size());
+        if (ns > 0)
+            SIL_CUDA_CHECK(cudaMemcpyAsync(d_strips, swork.data(), sizeof(StripWork<T>) * ns, cudaMemcpyHostToDevice,
+                                           stream));
+        SIL_CUDA_CHECK(cudaMemcpyAsync(d_work, work.data(), sizeof(Work<T>) * n, cudaMemcpyHostToDevice, stream));
         if (nt > 0)
             SIL_CUDA_CHECK(cudaMemcpyAsync(d_tact, open_tiles.data(), sizeof(int) * nt, cudaMemcpyHostToDevice, stream));
         cudaStream_t cs;
@@ -1660,15 +2038,16 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
         for (int c = 0; c < chunk && err == cudaSuccess; ++c) {
             if (march) {
                 cg_march_kernel<T><<<nt, kMarchThreads, sizeof(MarchSmem<T, MarchDirection<T>>), cs>>>(
-                        d_tiles, d_tact, d_info, d_vecs, d_sc, part_a);
-                cg_update_kernel<T, true><<<n, kThreads, 0, cs>>>(d_items, d_act, d_info, d_vecs, d_sc, part_b, part_c);
-                continue;
+                        d_tiles, d_tact, d_info, d_vecs, d_sc, part_a, part_b, part_c, c);
+            } else if (any_gauge) {
+                cg_direction3_kernel<T><<<n, kThreads, 0, cs>>>(d_work, c);
+                cg_apply3_kernel<T><<<n, kThreads, 0, cs>>>(d_items, d_act, d_info, d_vecs, d_sc, part_a, c);
+            } else {
+                cg_direction2_kernel<T><<<ns, kThreads, 0, cs>>>(d_strips, c);
             }
-            if (any3d) cg_direction3_kernel<T><<<n, kThreads, 0, cs>>>(d_items, d_act, d_info, d_vecs, d_sc);
-            if (any_gauge) cg_dir_apply_kernel<T, true><<<n, kThreads, 0, cs>>>(d_items, d_act, d_info, d_vecs, d_sc, part_a);
-            else cg_dir_apply_kernel<T, false><<<n, kThreads, 0, cs>>>(d_items, d_act, d_info, d_vecs, d_sc, part_a);
-            cg_update_kernel<T, false><<<n, kThreads, 0, cs>>>(d_items, d_act, d_info, d_vecs, d_sc, part_b, part_c);
+            cg_update_kernel<T><<<n, kThreads, 0, cs>>>(d_work, c);
         }
+        cg_close_kernel<T><<<n, kThreads, 0, cs>>>(d_work, chunk);
         cudaError_t const err2 = cudaStreamEndCapture(cs, &graph);
         if (err == cudaSuccess) err = err2;
         if (err == cudaSuccess) err = cudaGraphInstantiate(&exec, graph, 0);
@@ -1676,6 +2055,7 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
         if (err != cudaSuccess) return cuda_fail(err, "solver graph capture");
         captured_n = n;
         captured_tiles = nt;
+        captured_strips = ns;
         return SIL_OK;
     };
     auto read_scalars = [&]() -> sil_status {
@@ -1865,6 +2245,9 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
         if (march)
             residual64_march_kernel<<<captured_tiles, kMarchThreads, 0, stream>>>(
                     d_tiles, d_tact, d_info, d_nu64, d_rhs, d_x64, d_r64, d_sc, part_a, tol * tol, 0.0, 1);
+        else if (flat)
+            residual64_strip_kernel<T><<<captured_strips, kThreads, 0, stream>>>(d_strips, d_nu64, d_rhs, d_x64, d_r64,
+                                                                                 tol * tol, 0.0, 1);
         else
             residual_open<<<n, kThreads, 0, stream>>>(d_items, d_act, d_info, d_nu64, d_rhs, d_x64, d_r64, d_sc, part_a,
                                                       tol * tol, 0.0, 1);
@@ -1925,9 +2308,9 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
 // Work-item size of the batched CG kernels, picked by timing.  The first
 // batch of at least 4 M rows solved in a precision (2D and 3D batches apart)
 // runs a 96-iteration solve with items of 2,048, 4,096 and 8,192 rows and
-// keeps the fastest for the rest of the process (the tuning solves write the
+// keeps the fastest for such batches of the process (the tuning solves write the
 // caller's solution buffers, which the real solve overwrites).  Smaller
-// batches use 4,096 rows until a large one has been tuned.
+// batches take the rows that make one wave, at most 4,096.
 // SIMILIE_B200_ITEM_ROWS=<rows> forces a size; SIMILIE_B200_AUTOTUNE=0 keeps
 // the default.
 constexpr int kItemCandidates[3] = {2048, 4096, 8192};
@@ -1938,7 +2321,13 @@ template <class T>
 sil_status choose_item_rows(std::vector<ProblemDesc> const& probs, sil_solve_settings const& set, cudaStream_t stream,
                             int* rows)
 {
-    *rows = kItemNodes;
+    int64_t total = 0;
+    for (ProblemDesc const& q : probs) total += (q.dim == 3 ? 3 : 1) * q.nx * q.ny * (q.dim == 3 ? q.nz : 1);
+    // small batches: one wave of four CTAs per multiprocessor (fewer than two
+    // rows a thread cost more in partials than they gain)
+    int64_t const wave = 4 * static_cast<int64_t>(sm_count());
+    int64_t const spread = ((total + wave - 1) / wave + kThreads - 1) / kThreads * kThreads;
+    *rows = static_cast<int>(std::max<int64_t>(2 * kThreads, std::min<int64_t>(kItemNodes, spread)));
     if (char const* e = std::getenv("SIMILIE_B200_ITEM_ROWS")) {
         int const v = std::atoi(e);
         if (v >= kThreads && v % kThreads == 0 && v <= 64 * kThreads) {
@@ -1946,6 +2335,7 @@ sil_status choose_item_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
             return SIL_OK;
         }
     }
+    if (total < (int64_t(1) << 22)) return SIL_OK;
     int const key = (sizeof(T) == 8 ? 0 : 2) + (probs.front().dim == 3 ? 1 : 0);
     {
         std::lock_guard<std::mutex> lock(g_item_mutex);
@@ -1956,9 +2346,6 @@ sil_status choose_item_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
     }
     char const* at = std::getenv("SIMILIE_B200_AUTOTUNE");
     if (at != nullptr && at[0] == '0') return SIL_OK;
-    int64_t total = 0;
-    for (ProblemDesc const& q : probs) total += (q.dim == 3 ? 3 : 1) * q.nx * q.ny * (q.dim == 3 ? q.nz : 1);
-    if (total < (int64_t(1) << 22)) return SIL_OK;
     sil_solve_settings probe = set;
     probe.max_iterations = 96;
     std::vector<sil_solve_diagnostics> scratch(probs.size());
