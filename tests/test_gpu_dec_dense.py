@@ -3,7 +3,10 @@
 A spectator dim of extent one makes a field take the table-driven kernels, so
 the same data runs both ways.  Boxes hold one node, an edge pair, and runs
 past a block; strides are the two component orders and reversed lattice axes;
-output boxes are the input's, one smaller, and shifted across its faces.
+output boxes are the input's, one smaller, and shifted across its faces.  The
+Laplacian's marching kernels (3D, and 2D 1-forms, for boxes inside the input)
+meet an exact number of tiles (30 owned nodes along the lanes, 6 rows), one
+more, several runs of planes, and clamped and unclamped upper faces.
 """
 from math import comb
 
@@ -16,6 +19,26 @@ torch = pytest.importorskip("torch")
 
 SHAPES = {1: [(1,), (2,), (300,)], 2: [(1, 2), (3, 5), (2, 131), (37, 6)],
           3: [(1, 1, 2), (3, 2, 4), (4, 5, 67), (9, 3, 3)]}
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("shape,ks", [((7, 31), (1,)), ((67, 62), (1,)), ((301, 241), (1,)), ((5, 13, 61), (1, 2)),
+                                      ((40, 14, 35), (1, 2)), ((41, 12, 30), (1, 2)), ((131, 125, 124), (0, 3))])
+def test_marching_laplacians_equal_the_table_driven_ones(shape, ks, dtype):
+    import similie_b200 as sb
+    n = len(shape)
+    rng = np.random.default_rng(sum(shape))
+    geo = sb.Geometry([np.cumsum(rng.uniform(0.3, 1.7, s + 4)) for s in shape])
+    for k in ks:
+        inp = torch.from_numpy(rng.standard_normal(shape + (comb(n, k),))).cuda().to(dtype)
+        inp.view(-1)[11], inp.view(-1)[97] = float("inf"), float("nan")
+        boxes = [(shape, (0,) * n), (tuple(s - 1 for s in shape), (0,) * n), (tuple(s - 2 for s in shape), (1,) * n)]
+        for oshape, front in boxes if inp.numel() < 10 ** 6 else boxes[:2]:
+            for layout in ("last", "first", "reversed"):
+                got, ref = (_run(sb, "laplacian", geo, shape, k, k, inp, oshape, front, layout, dtype, sp)
+                            for sp in (False, True))
+                assert torch.equal(torch.isnan(got), torch.isnan(ref)), (k, oshape, front, layout)
+                assert torch.equal(torch.nan_to_num(got), torch.nan_to_num(ref)), (k, oshape, front, layout)
 
 
 def _laid_out(t, layout):
