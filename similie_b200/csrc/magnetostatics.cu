@@ -542,6 +542,8 @@ struct Scalars
     double rz_it[2];           // by parity of the iteration: r . z it starts from
     double scale_prev;         // outer residual norm of the previous refinement pass
     int pending;               // 1: x still lacks alpha times the latest direction
+    int cycles;                // resident solve: refinement cycles run
+    int timeout;               // and 1: a wait for the group's other CTAs ran out
 };
 
 // Deterministic block sum of one double per thread.
@@ -1626,6 +1628,346 @@ __global__ void copy_from_vec_kernel(Item const* items, Vecs<T> const* vecs, dou
     for (int64_t row = it.begin + threadIdx.x; row < it.end; row += kThreads) dst[it.prob][row] = static_cast<double>(x[row]);
 }
 
+// ------------------------------------------------------------------ resident solve (2D)
+//
+// The whole refinement loop of a 2D problem in one cooperative launch, its
+// vectors on chip: a group of CTAs, one per multiprocessor, holds consecutive
+// grid rows each, p, nu and D^-1 in shared memory and r, x and q in registers,
+// so an iteration reads nothing from memory but the two neighbour rows of z
+// and the group's partial sums.  An iteration has two waits for the group (after
+// p.q and after r.z), each a counter in global memory; a group whose problem
+// has ended leaves, and groups of several problems run side by side.  The
+// arithmetic is the launch-per-kernel path's, the sums in another order.
+//
+// B200, per iteration against two kernels: four problems of 96^2 .. 161^2 11.2 ->
+// 6.2 us, 512^2 12.7 -> 7.2, 1024^2 19.8 -> 12.5 (FP64), six problems of 128^2 ..
+// 1024^2 41 -> 28, sixty 373 -> 237 (FP64) and 267 -> 137 (FP32).  What bounds it:
+// small problems the two meetings (about 1.7 us each at sixteen CTAs), 1024^2 the
+// shared-memory reads of 7,168 nodes by sixteen warps.
+constexpr int kResThreads = 512;
+// Nodes of a thread at most (r, x and q take three registers of T each): 7,168
+// a CTA in FP64, 14,336 in FP32.
+template <class T>
+constexpr int kResMaxPerThread = sizeof(T) == 8 ? 14 : 28;
+constexpr int kResPollLimit = 1 << 22;                    // polls of a wait before it gives up (seconds)
+
+struct ResidentCta
+{
+    int prob;
+    int g, group;      // CTA number within the problem's group, and the group's size
+    int ja, jb;        // owned rows
+    int nx, ny;
+    int slots;         // first mail slot of the group
+};
+
+// A group meets by mail: each CTA stores its two sums into its own pair of
+// slots and polls everybody's, so the data is its own arrival flag and a
+// meeting costs one trip through L2 after the last arrival (a counter and then
+// the sums would cost two, and all arrivals queue on the counter).  An empty
+// slot holds a NaN no sum is stored as.  Meetings use four sets of slots in
+// turn; a CTA empties its slots of meeting k + 2 after passing meeting k - 1,
+// when everyone has read what they held (meeting k - 2).  Of two meetings in a
+// row at least one carries data, and its release and acquire order the emptying
+// before anyone's poll of meeting k + 2.
+constexpr unsigned long long kNoMail = 0x7ff8decafc0ffee1ull;
+constexpr int kMailSets = 4;
+constexpr int kMailPerLane = 8;   // of a polling lane: groups of up to 256 CTAs
+constexpr int kHaloAhead = 2;   // halo nodes per row that a thread loads ahead
+
+// RELEASE: what the CTA stored before is visible to whoever reads the mail.
+template <bool RELEASE>
+__device__ __forceinline__ void mail_store(unsigned long long* slot, double v)
+{
+    unsigned long long w = static_cast<unsigned long long>(__double_as_longlong(v));
+    if (w == kNoMail) w = 0x7ff8000000000000ull;
+    if constexpr (RELEASE) asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(slot), "l"(w) : "memory");
+    else asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(slot), "l"(w) : "memory");
+}
+__device__ __forceinline__ unsigned long long mail_load(unsigned long long const* slot)
+{
+    unsigned long long w;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(slot) : "memory");
+    return w;
+}
+
+// M: nodes of a thread.  Local node n = tid + m * kResThreads; the arrays are
+// padded to M * kResThreads nodes, whose r and q are zero, so the loops load
+// without a guard.
+template <class T, int M>
+__global__ void __launch_bounds__(kResThreads, 1)
+        cg_resident_kernel(ResidentCta const* ctas, Vecs<T> const* vecs, double const* const* nu64,
+                           double const* const* rhs, double* const* x64, double* const* r64, Scalars* sc,
+                           unsigned long long* mail, double tol2, int max_iter, int chunk, int poll_limit)
+{
+    constexpr int kNodes = M * kResThreads;
+    extern __shared__ __align__(16) unsigned char res_smem[];
+    __shared__ double red[2][kResThreads / 32];
+    __shared__ double sums[2];
+    __shared__ int aborted;
+    ResidentCta const c = ctas[blockIdx.x];
+    Scalars* s = sc + c.prob;
+    if (s->outer_done) return;   // the whole group's
+    int const tid = threadIdx.x, nx = c.nx, ny = c.ny, rows = c.jb - c.ja, count = rows * nx;
+    int64_t const first = static_cast<int64_t>(c.ja) * nx;   // global row number of local node 0
+    T* ps = reinterpret_cast<T*>(res_smem);                  // rows ja-1 .. jb (and padding)
+    T* ns = ps + kNodes + 2 * nx;                            // rows ja-1 .. jb-1
+    T* ds = ns + kNodes + nx;                                // rows ja .. jb-1
+    Vecs<T> const v = vecs[c.prob];
+    unsigned long long* const box = mail + c.slots;          // [set][CTA][2]
+    int meeting = 0;
+    if (tid == 0) aborted = 0;
+
+    // The group's sums of a and, with `data`, of b over all threads, the same
+    // bits in every CTA; with `data` what the CTAs stored to global memory before
+    // is visible after.  False when a wait ran out.
+    auto meet = [&](auto data, double a, double b, double& sum_a, double& sum_b) -> bool {
+        constexpr bool kData = decltype(data)::value, kBoth = kData;
+        for (int o = 16; o > 0; o >>= 1) {
+            a += __shfl_xor_sync(0xffffffffu, a, o);
+            b += __shfl_xor_sync(0xffffffffu, b, o);
+        }
+        if ((tid & 31) == 0) {
+            red[0][tid >> 5] = a;
+            red[1][tid >> 5] = b;
+        }
+        __syncthreads();
+        if (tid < 32) {
+            double ta = tid < kResThreads / 32 ? red[0][tid & 15] : 0.0, tb = tid < kResThreads / 32 ? red[1][tid & 15] : 0.0;
+            for (int o = 8; o > 0; o >>= 1) {
+                ta += __shfl_xor_sync(0xffffffffu, ta, o);
+                tb += __shfl_xor_sync(0xffffffffu, tb, o);
+            }
+            unsigned long long* const now = box + static_cast<int64_t>(meeting & (kMailSets - 1)) * 2 * c.group;
+            unsigned long long* const later = box + static_cast<int64_t>((meeting + 2) & (kMailSets - 1)) * 2 * c.group;
+            if (tid < 2) {
+                later[2 * c.g + tid] = kNoMail;
+                if (kBoth || tid == 0) mail_store<kData>(now + 2 * c.g + tid, tid == 0 ? ta : tb);
+            }
+            // this lane's share of the mail, all of it asked for at once
+            unsigned long long wa[kMailPerLane], wb[kMailPerLane];
+            int tries = 0;
+            bool lost = false, waiting = true;
+#pragma unroll
+            for (int u = 0; u < kMailPerLane; ++u) wa[u] = wb[u] = tid + 32 * u < c.group ? kNoMail : 0ull;
+            while (waiting) {
+                waiting = false;
+#pragma unroll
+                for (int u = 0; u < kMailPerLane; ++u) {
+                    unsigned long long const* slot = now + 2 * (tid + 32 * u);
+                    if (wa[u] == kNoMail) wa[u] = mail_load(slot);
+                    if (kBoth && wb[u] == kNoMail) wb[u] = mail_load(slot + 1);
+                }
+#pragma unroll
+                for (int u = 0; u < kMailPerLane; ++u) waiting = waiting || wa[u] == kNoMail || (kBoth && wb[u] == kNoMail);
+                if (waiting && ++tries > poll_limit) {
+                    lost = true;
+                    break;
+                }
+            }
+            double va = 0.0, vb = 0.0;
+#pragma unroll
+            for (int u = 0; u < kMailPerLane; ++u) {
+                va += __longlong_as_double(static_cast<long long>(wa[u]));
+                if (kBoth) vb += __longlong_as_double(static_cast<long long>(wb[u]));
+            }
+            if constexpr (kData) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+            if (__any_sync(0xffffffffu, lost)) {
+                if (tid == 0) {
+                    aborted = 1;
+                    s->timeout = 1;
+                }
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                va += __shfl_xor_sync(0xffffffffu, va, o);
+                vb += __shfl_xor_sync(0xffffffffu, vb, o);
+            }
+            if (tid == 0) {
+                sums[0] = va;
+                sums[1] = vb;
+            }
+        }
+        ++meeting;
+        __syncthreads();
+        sum_a = sums[0];
+        sum_b = sums[1];
+        return aborted == 0;
+    };
+
+    // which of this thread's nodes are interior, and which lie in a row that
+    // another CTA reads
+    unsigned inner = 0, edge = 0;
+#pragma unroll 1
+    for (int m = 0; m < M; ++m) {
+        int const n = tid + m * kResThreads;
+        if (n >= count) continue;
+        int const jl = n / nx, i = n - jl * nx, j = c.ja + jl;
+        if (i > 0 && i + 1 < nx && j > 0 && j + 1 < ny) inner |= 1u << m;
+        if (jl == 0 || jl == rows - 1) edge |= 1u << m;
+    }
+    auto is = [](unsigned mask, int m) { return ((mask >> m) & 1u) != 0; };
+    bool const lower = c.ja > 0, upper = c.jb < ny;
+    // The reluctivity of the first row and column is zero here: it only enters
+    // the terms that the operator leaves out, which so add a zero.
+    for (int n = tid; n < kNodes + nx; n += kResThreads) {
+        int const jl = n / nx, i = n - jl * nx, j = c.ja - 1 + jl;
+        ns[n] = j > 0 && i > 0 && j < c.jb ? v.nu[first - nx + n] : T(0);
+    }
+    for (int n = tid; n < kNodes; n += kResThreads) ds[n] = n < count ? v.dinv[first + n] : T(0);
+    for (int n = tid; n < kNodes + 2 * nx; n += kResThreads) ps[n] = T(0);
+    double const* const nu = nu64[c.prob] + first;
+    double const* const b = rhs[c.prob] + first;
+    double* const xg = x64[c.prob] + first;
+    double* const rg = r64[c.prob] + first;
+    T* const zg = v.z + first;
+
+    double const bb = s->bb;
+    double scale = s->scale, beta_last = 0.0, rz_cur = 0.0, none;
+    int total_iters = s->total_iters, iters = 0, cycles = 0, nonfinite = 0, outer = 0;
+    bool ok = true;
+    T r[M], x[M], q[M];
+    __syncthreads();
+    while (true) {
+        // r64 = b - A x64, its norm
+        double acc = 0.0;
+#pragma unroll 1
+        for (int n = tid, m = 0; n < count; n += kResThreads, ++m) {
+            double const a0 = __ldcg(xg + n);
+            double ax = a0;
+            if (is(inner, m)) {
+                int const jl = n / nx, i = n - jl * nx, j = c.ja + jl;
+                ax = 0.0;
+                if (j >= 2) ax = ax + (a0 - __ldcg(xg + n - nx)) * nu[n - nx];
+                ax = ax - (__ldcg(xg + n + nx) - a0) * nu[n];
+                if (i >= 2) ax = ax - (__ldcg(xg + n - 1) - a0) * nu[n - 1];
+                ax = ax + (a0 - __ldcg(xg + n + 1)) * nu[n];
+            }
+            double const res = b[n] - ax;
+            rg[n] = res;
+            acc += res * res;
+        }
+        double tot;
+        if (!(ok = meet(std::false_type {}, acc, 0.0, tot, none))) break;
+        double const scale_prev = scale;
+        scale = sqrt(tot);
+        if (!isfinite(tot)) nonfinite = 1;
+        if (tot <= tol2 * bb || !isfinite(tot)) {
+            outer = 1;
+            break;
+        }
+        if (static_cast<int64_t>(cycles) * chunk >= max_iter) break;
+        double const inner_tol2 = 0.25 * tol2 * bb / fmax(tot, 1e-300);
+        // residual replacement (cg_replace_kernel)
+        double rz = 0.0, rr = 0.0;
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            int const n = tid + m * kResThreads;
+            T const rn = n < count ? static_cast<T>(rg[n] / scale) : T(0), z = ds[n] * rn;
+            r[m] = rn;
+            x[m] = T(0);
+            if (is(edge, m)) __stcg(zg + n, z);
+            rz += static_cast<double>(rn) * static_cast<double>(z);
+            rr += static_cast<double>(rn) * static_cast<double>(rn);
+        }
+        double rz0, rr0;
+        if (!(ok = meet(std::true_type {}, rz, rr, rz0, rr0))) break;
+        bool const keep = cycles > 0 && iters > 0 && rz_cur > 0.0 && scale_prev > 0.0;
+        double beta = keep ? beta_last * rz0 / ((scale_prev / scale) * rz_cur) : 0.0;
+        rz_cur = rz0;
+        iters = 0;
+        nonfinite = 0;
+        bool done = rr0 == 0.0 || total_iters >= max_iter;
+        T alpha = T(0);   // of the step x still lacks
+        for (int it = 0; it < chunk && !done; ++it) {
+            // p = z + beta p (and the previous step's x += alpha p), halo rows
+            // too: their z is on its way while the own nodes are formed
+            T const bt = static_cast<T>(beta);
+            T zl[kHaloAhead], zu[kHaloAhead];
+#pragma unroll
+            for (int h = 0; h < kHaloAhead; ++h) {
+                int const i = min(tid + h * kResThreads, nx - 1);
+                zl[h] = lower ? __ldcg(zg - nx + i) : T(0);
+                zu[h] = upper ? __ldcg(zg + count + i) : T(0);
+            }
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                int const n = tid + m * kResThreads;
+                T const po = ps[n + nx];
+                x[m] = x[m] + alpha * po;
+                if (n < count) ps[n + nx] = ds[n] * r[m] + bt * po;
+            }
+#pragma unroll
+            for (int h = 0; h < kHaloAhead; ++h) {
+                int const i = tid + h * kResThreads;
+                if (i < nx) {
+                    if (lower) ps[i] = zl[h] + bt * ps[i];
+                    if (upper) ps[count + nx + i] = zu[h] + bt * ps[count + nx + i];
+                }
+            }
+            for (int i = tid + kHaloAhead * kResThreads; i < nx; i += kResThreads) {
+                if (lower) ps[i] = __ldcg(zg - nx + i) + bt * ps[i];
+                if (upper) ps[count + nx + i] = __ldcg(zg + count + i) + bt * ps[count + nx + i];
+            }
+            __syncthreads();
+            double pq = 0.0;
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                int const n = tid + m * kResThreads;
+                T const* p = ps + n + nx;
+                T const a0 = n < count ? p[0] : T(0), nc = ns[n + nx];
+                T qv = T(0);
+                qv = qv + (a0 - p[-nx]) * ns[n];
+                qv = qv - (p[nx] - a0) * nc;
+                qv = qv - (p[-1] - a0) * ns[n + nx - 1];
+                qv = qv + (a0 - p[1]) * nc;
+                qv = is(inner, m) ? qv : a0;
+                q[m] = qv;
+                pq += static_cast<double>(a0) * static_cast<double>(qv);
+            }
+            double tpq;
+            if (!(ok = meet(std::false_type {}, pq, 0.0, tpq, none))) break;
+            double const a = rz_cur / tpq;
+            alpha = static_cast<T>(a);
+            rz = rr = 0.0;
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                int const n = tid + m * kResThreads;
+                T const rn = r[m] - alpha * q[m], z = ds[n] * rn;
+                r[m] = rn;
+                if (is(edge, m)) __stcg(zg + n, z);
+                rz += static_cast<double>(rn) * static_cast<double>(z);
+                rr += static_cast<double>(rn) * static_cast<double>(rn);
+            }
+            double rz1, rr1;
+            if (!(ok = meet(std::true_type {}, rz, rr, rz1, rr1))) break;
+            beta = beta_last = rz1 / rz_cur;
+            rz_cur = rz1;
+            ++iters;
+            ++total_iters;
+            bool const bad = !isfinite(rr1) || !isfinite(rz1) || !isfinite(a);
+            if (bad) nonfinite = 1;
+            done = rr1 <= inner_tol2 * rr0 || bad || total_iters >= max_iter;
+        }
+        if (!ok) break;
+        // x64 += scale x
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            int const n = tid + m * kResThreads;
+            if (n < count)
+                __stcg(xg + n, __ldcg(xg + n) + scale * static_cast<double>(x[m] + alpha * ps[n + nx]));
+        }
+        if (!(ok = meet(std::true_type {}, 0.0, 0.0, none, none))) break;
+        ++cycles;
+    }
+    if (c.g == 0 && tid == 0) {
+        s->scale = scale;
+        s->total_iters = total_iters;
+        s->iters = iters;
+        s->nonfinite = nonfinite;
+        s->outer_done = outer;
+        s->cycles = cycles;
+    }
+}
+
 // ------------------------------------------------------------------ host driver
 
 struct DeviceBuffer
@@ -1749,6 +2091,130 @@ sil_status build_divergence_gauge(ProblemDesc const& q, ProbInfo const& pi, doub
     return SIL_OK;
 }
 
+// Shared memory of the resident kernel with m nodes per thread, and the rows a
+// CTA can hold of an nx-wide grid.
+template <class T>
+size_t resident_smem(int m, int64_t nx)
+{
+    return (3 * static_cast<size_t>(m) * kResThreads + 3 * static_cast<size_t>(nx)) * sizeof(T);
+}
+template <class T>
+int64_t resident_rows(int64_t nx)
+{
+    constexpr size_t most = 226 * 1024;   // of the 227 KB a CTA can have, less the static part
+    return resident_smem<T>(kResMaxPerThread<T>, nx) <= most ? kResThreads * kResMaxPerThread<T> / nx : 0;
+}
+
+// The kernel's instances by nodes per thread.
+template <class T>
+int resident_nodes(int per_thread)
+{
+    for (int m : {2, 4, 8, 14})
+        if (per_thread <= m) return m;
+    return kResMaxPerThread<T>;
+}
+
+// CTAs a 2D problem needs to be resident (0: it does not fit the GPU).
+template <class T>
+int resident_ctas(ProblemDesc const& q, int sms)
+{
+    if (q.dim != 2 || q.nx * q.ny > static_cast<int64_t>(sms) * kResThreads * kResMaxPerThread<T>) return 0;
+    int64_t const rows = resident_rows<T>(q.nx);
+    if (rows < 1) return 0;
+    int64_t const g = (q.ny + rows - 1) / rows;
+    return g <= sms ? static_cast<int>(g) : 0;
+}
+
+// One cooperative launch: problems side by side, one CTA per multiprocessor.
+struct ResidentWave
+{
+    std::vector<int> probs;
+    std::vector<ResidentCta> ctas;
+    size_t smem = 0;
+    int per_thread = 0;   // nodes of a thread: the kernel's instance
+};
+
+// Nodes per CTA below which another CTA in the group costs more in meetings
+// than it saves: 8 sqrt(nodes), 1,024 at least.  Measured per FP64 iteration:
+// 64^2 with 1,024 nodes a CTA 3.6 us, with 2,048 4.6; 128^2 1,024 4.7, 2,048 4.4,
+// 4,096 5.7; 256^2 1,024 5.7, 2,048 5.3, 4,096 5.8; 512^2 1,771 8.2, 4,096 6.4.
+int64_t resident_enough(ProblemDesc const& q)
+{
+    return std::max<int64_t>(1024, static_cast<int64_t>(8.0 * std::sqrt(static_cast<double>(q.nx * q.ny))));
+}
+
+// Problems into waves (largest first, each into the first wave with room), then
+// a wave's spare CTAs to the problems with the most nodes per CTA.
+template <class T>
+std::vector<ResidentWave> plan_resident(std::vector<ProblemDesc> const& probs, int sms)
+{
+    std::vector<ResidentWave> waves;
+    std::vector<int> order, need(probs.size(), 0), room;
+    for (size_t p = 0; p < probs.size(); ++p) {
+        need[p] = resident_ctas<T>(probs[p], sms);
+        if (need[p] > 0) order.push_back(static_cast<int>(p));
+    }
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+        return probs[a].nx * probs[a].ny > probs[b].nx * probs[b].ny;
+    });
+    for (int p : order) {
+        size_t w = 0;
+        while (w < waves.size() && room[w] < need[p]) ++w;
+        if (w == waves.size()) {
+            waves.emplace_back();
+            room.push_back(sms);
+        }
+        waves[w].probs.push_back(p);
+        room[w] -= need[p];
+    }
+    int slots = 0;
+    for (size_t w = 0; w < waves.size(); ++w) {
+        ResidentWave& wave = waves[w];
+        std::vector<int64_t> g;
+        int64_t widest = 0;
+        for (int p : wave.probs) g.push_back(need[p]);
+        for (int spare = room[w]; spare > 0; --spare) {
+            int64_t most = 0;
+            size_t at = g.size();
+            for (size_t k = 0; k < g.size(); ++k) {
+                ProblemDesc const& q = probs[wave.probs[k]];
+                int64_t const nodes = (q.ny + g[k] - 1) / g[k] * q.nx;
+                if (g[k] < q.ny && nodes > resident_enough(q) && nodes > most) {
+                    most = nodes;
+                    at = k;
+                }
+            }
+            if (at == g.size()) break;
+            ++g[at];
+        }
+        for (size_t k = 0; k < g.size(); ++k) {
+            int const p = wave.probs[k];
+            int const nx = static_cast<int>(probs[p].nx), ny = static_cast<int>(probs[p].ny);
+            int const rows = static_cast<int>((ny + g[k] - 1) / g[k]), group = (ny + rows - 1) / rows;
+            for (int i = 0; i < group; ++i)
+                wave.ctas.push_back({p, i, group, i * rows, std::min(ny, (i + 1) * rows), nx, ny, slots});
+            slots += 2 * kMailSets * group;
+            widest = std::max<int64_t>(widest, nx);
+            wave.per_thread = std::max(wave.per_thread, (rows * nx + kResThreads - 1) / kResThreads);
+        }
+        wave.per_thread = resident_nodes<T>(wave.per_thread);
+        wave.smem = resident_smem<T>(wave.per_thread, widest);
+    }
+    return waves;
+}
+
+template <class T>
+void const* resident_kernel(int per_thread)
+{
+    switch (per_thread) {
+    case 2: return reinterpret_cast<void const*>(cg_resident_kernel<T, 2>);
+    case 4: return reinterpret_cast<void const*>(cg_resident_kernel<T, 4>);
+    case 8: return reinterpret_cast<void const*>(cg_resident_kernel<T, 8>);
+    case 14: return reinterpret_cast<void const*>(cg_resident_kernel<T, 14>);
+    default: return reinterpret_cast<void const*>(cg_resident_kernel<T, kResMaxPerThread<T>>);
+    }
+}
+
 template <class T>
 sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_settings const& set,
                             sil_solve_diagnostics* diag, cudaStream_t stream, nn::Net* learned, int item_rows)
@@ -1826,6 +2292,15 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
             nstrip_ctas += strips_of(info[p].nx, info[p].ny, srows).ctas;
         }
     int const nparts = std::max(std::max(nitems, ntiles), nstrip_ctas);
+    // 2D problems that fit on chip are solved there; the others by the kernels
+    // per iteration.
+    std::vector<ResidentWave> const waves = flat ? plan_resident<T>(probs, sm_count()) : std::vector<ResidentWave> {};
+    size_t nres = 0;
+    std::vector<char> resident(np, 0);
+    for (ResidentWave const& w : waves) {
+        nres += w.ctas.size();
+        for (int p : w.probs) resident[p] = 1;
+    }
     int const nvec = 8;  // x r z p q dinv nu p2 in precision T
     size_t const vec_bytes = ((total_rows * sizeof(T) + 255) / 256) * 256;
     size_t const d_bytes = ((total_rows * sizeof(double) + 255) / 256) * 256;
@@ -1853,7 +2328,8 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
              + 3 * sizeof(double) * nparts + kMaxDirs * sizeof(double) * nitems + 7 * sizeof(void*) * np
              + sp64.size() * (sizeof(double) + sizeof(float)) + sizeof(int) * np + sizeof(int) * nitems
              + (sizeof(Tile) + sizeof(int)) * ntiles + sizeof(Work<T>) * nitems
-             + sizeof(StripWork<T>) * nstrip_ctas + 27 * 256;
+             + sizeof(StripWork<T>) * nstrip_ctas
+             + (sizeof(ResidentCta) + 2 * kMailSets * sizeof(unsigned long long)) * nres + 30 * 256;
     DeviceBuffer buf;
     SIL_CUDA_CHECK(cudaMalloc(&buf.ptr, bytes));
     char* base = static_cast<char*>(buf.ptr);
@@ -1880,6 +2356,8 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
     int* d_active = reinterpret_cast<int*>(take(sizeof(int) * np));
     int* d_act = reinterpret_cast<int*>(take(sizeof(int) * nitems));
     Work<T>* d_work = reinterpret_cast<Work<T>*>(take(sizeof(Work<T>) * nitems));
+    ResidentCta* d_res = reinterpret_cast<ResidentCta*>(take(sizeof(ResidentCta) * nres));
+    auto* d_mail = reinterpret_cast<unsigned long long*>(take(2 * kMailSets * sizeof(unsigned long long) * nres));
     StripWork<T>* d_strips = reinterpret_cast<StripWork<T>*>(take(sizeof(StripWork<T>) * nstrip_ctas));
     Tile* d_tiles = reinterpret_cast<Tile*>(take(sizeof(Tile) * ntiles));
     int* d_tact = reinterpret_cast<int*>(take(sizeof(int) * ntiles));
@@ -1991,7 +2469,7 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
     auto build_open = [&]() {
         open_host.clear();
         for (int i = 0; i < nitems; ++i)
-            if (!hs[items[i].prob].outer_done) open_host.push_back(i);
+            if (!hs[items[i].prob].outer_done && !resident[items[i].prob]) open_host.push_back(i);
         open_tiles.clear();
         for (int i = 0; i < ntiles; ++i)
             if (!hs[tiles[i].prob].outer_done) open_tiles.push_back(i);
@@ -2016,7 +2494,7 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
         }
         swork.clear();
         for (int p = 0; flat && p < np; ++p) {
-            if (hs[p].outer_done) continue;
+            if (hs[p].outer_done || resident[p]) continue;
             ProbInfo const& pi = info[p];
             Vecs<T> const& v = vecs[p];
             Strips const st = strips_of(pi.nx, pi.ny, srows);
@@ -2229,16 +2707,47 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
     // bb = ||b||^2 via an init pass from the right-hand side.
     cg_init_kernel<T><<<nitems, kThreads, 0, stream>>>(d_items, d_info, d_vecs, d_rhs, nullptr, d_sc, part_a, part_b,
                                                        false);
-    int total = 0;
+    int total = 0, resident_cycles = 0;
     if constexpr (std::is_same_v<T, float>) {
         if (learned != nullptr && st == SIL_OK) st = learned_stage(learned, &total, &refinements);
+    }
+    // The resident problems, wave after wave.
+    if (st == SIL_OK && !waves.empty()) {
+        std::vector<ResidentCta> all;
+        for (ResidentWave const& w : waves) all.insert(all.end(), w.ctas.begin(), w.ctas.end());
+        SIL_CUDA_CHECK(cudaMemcpyAsync(d_res, all.data(), sizeof(ResidentCta) * all.size(), cudaMemcpyHostToDevice, stream));
+        std::vector<unsigned long long> const empty(2 * kMailSets * nres, kNoMail);
+        SIL_CUDA_CHECK(cudaMemcpyAsync(d_mail, empty.data(), sizeof(unsigned long long) * empty.size(),
+                                       cudaMemcpyHostToDevice, stream));
+        size_t at = 0;
+        for (ResidentWave const& w : waves) {
+            void const* const kernel = resident_kernel<T>(w.per_thread);
+            SIL_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                static_cast<int>(w.smem)));
+            ResidentCta const* ctas = d_res + at;
+            double tol2 = tol * tol;
+            int budget = max_iter, steps = chunk, polls = kResPollLimit;
+            void* args[] = {&ctas, &d_vecs, &d_nu64, &d_rhs, &d_x64, &d_r64, &d_sc, &d_mail, &tol2, &budget, &steps, &polls};
+            SIL_CUDA_CHECK(cudaLaunchCooperativeKernel(kernel, dim3(static_cast<unsigned>(w.ctas.size())),
+                                                       dim3(kResThreads), args, w.smem, stream));
+            at += w.ctas.size();
+        }
+        st = read_scalars();
+        if (st != SIL_OK) return st;
+        int cycles = 0;
+        for (int p = 0; p < np; ++p) {
+            if (hs[p].timeout) return fail(SIL_ERR_BUDGET, "resident solve: a wait for the group's other blocks ran out");
+            cycles = std::max(cycles, hs[p].cycles);
+        }
+        resident_cycles = cycles;
     }
     // Cycle: FP64 residual (outer check) -> residual replacement -> a chunk
     // of iterations -> x64 += ||r|| x; the host reads the problems' state
     // once per cycle.
     auto const residual_open = any_gauge ? residual64_kernel<true> : residual64_kernel<false>;
+    int const before = refinements;
     build_open();
-    if (!open_host.empty()) st = capture_chunk();
+    if (st == SIL_OK && !open_host.empty()) st = capture_chunk();
     bool fresh = true;
     while (st == SIL_OK && !open_host.empty()) {
         int const n = captured_n;
@@ -2268,6 +2777,7 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
         refine_kernel<T><<<captured_n, kThreads, 0, stream>>>(d_items, d_act, d_vecs, d_x64, d_sc);
         ++refinements;
     }
+    refinements = std::max(refinements, before + resident_cycles);
     if (exec != nullptr) cudaGraphExecDestroy(exec);
     if (graph != nullptr) cudaGraphDestroy(graph);
     if (st == SIL_OK) copy_kernel<<<nitems, kThreads, 0, stream>>>(d_items, d_x64, d_sol, d_sc);
@@ -2336,6 +2846,8 @@ sil_status choose_item_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
         }
     }
     if (total < (int64_t(1) << 22)) return SIL_OK;
+    if (std::all_of(probs.begin(), probs.end(), [](ProblemDesc const& q) { return resident_ctas<T>(q, sm_count()) > 0; }))
+        return SIL_OK;   // solved on chip
     int const key = (sizeof(T) == 8 ? 0 : 2) + (probs.front().dim == 3 ? 1 : 0);
     {
         std::lock_guard<std::mutex> lock(g_item_mutex);
