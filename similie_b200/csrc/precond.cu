@@ -310,11 +310,34 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_group1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
-// Asynchronous halo staging: the level's own tensor (up = false) or the
-// nearest-upsampled coarse tensor gathered to this level (up = true); pixels
-// outside the image (and, for the gather, its border) are zero-filled.
-__device__ __forceinline__ void stage_halo(uint4* halo, Table const& t, int im, int start, int P, bf16 const* src,
-                                           bool up)
+// The level's own tensor.  Four neighbouring lanes copy the four chunks of a
+// pixel, so a warp's copy reads 512 contiguous bytes and walks the row by
+// constant distances; only a row that leaves the image is checked per pixel.
+__device__ __forceinline__ void stage_halo_plain(uint4* halo, Table const& t, int im, int start, int P, bf16 const* src)
+{
+    Img const o = t.img[im];
+    int const npx = P * (o.h + 2);
+    int const c = threadIdx.x & 3, j0 = threadIdx.x >> 2;
+    uint4 const* base = reinterpret_cast<uint4 const*>(src) + o.offset * kChunks + c;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        int const g0 = start + (r - 1) * P - 1;
+        uint4* dst = &halo[(c * 3 + r) * kHalo + j0];
+        uint4 const* p = base + static_cast<int64_t>(g0 + j0) * kChunks;
+        bool const whole = g0 >= 0 && g0 + kHalo <= npx;
+#pragma unroll
+        for (int q = 0; q < (kHalo + 31) / 32; ++q) {
+            if (32 * q + 31 >= kHalo && j0 + 32 * q >= kHalo) continue;
+            int const g = g0 + j0 + 32 * q;
+            bool const valid = whole || (g >= 0 && g < npx);
+            cp_async16(dst + 32 * q, valid ? p + 32 * q * kChunks : base, valid);
+        }
+    }
+}
+
+// The nearest-upsampled coarse tensor gathered to this level; pixels outside
+// the image and on its border are zero-filled.
+__device__ __forceinline__ void stage_halo_up(uint4* halo, Table const& t, int im, int start, int P, bf16 const* src)
 {
     Img const o = t.img[im];
     int const npx = P * (o.h + 2);
@@ -324,14 +347,12 @@ __device__ __forceinline__ void stage_halo(uint4* halo, Table const& t, int im, 
     // the pixel before the image is row -1); within a row they advance by
     // adding, wrapping at the row pitch P.
     int y0[3], x0[3];
-    if (up) {
 #pragma unroll
-        for (int r = 0; r < 3; ++r) {
-            int const g0 = start + (r - 1) * P - 1;
-            int const y = g0 >= 0 ? g0 / P : -1;
-            y0[r] = y;
-            x0[r] = g0 - y * P;
-        }
+    for (int r = 0; r < 3; ++r) {
+        int const g0 = start + (r - 1) * P - 1;
+        int const y = g0 >= 0 ? g0 / P : -1;
+        y0[r] = y;
+        x0[r] = g0 - y * P;
     }
     for (int i = threadIdx.x; i < 3 * kHalo; i += blockDim.x) {
         int const r = i / kHalo, j = i - r * kHalo;
@@ -339,18 +360,14 @@ __device__ __forceinline__ void stage_halo(uint4* halo, Table const& t, int im, 
         bool valid = g >= 0 && g < npx;
         int64_t px = 0;
         if (valid) {
-            if (up) {
-                int y = r == 0 ? y0[0] : (r == 1 ? y0[1] : y0[2]);
-                int x = (r == 0 ? x0[0] : (r == 1 ? x0[1] : x0[2])) + j;
-                while (x >= P) {
-                    x -= P;
-                    ++y;
-                }
-                valid = !(y == 0 || x == 0 || y > o.h || x > o.w);
-                px = ci.offset + static_cast<int64_t>((y - 1) / 2 + 1) * (ci.w + 2) + ((x - 1) / 2 + 1);
-            } else {
-                px = o.offset + g;
+            int y = r == 0 ? y0[0] : (r == 1 ? y0[1] : y0[2]);
+            int x = (r == 0 ? x0[0] : (r == 1 ? x0[1] : x0[2])) + j;
+            while (x >= P) {
+                x -= P;
+                ++y;
             }
+            valid = !(y == 0 || x == 0 || y > o.h || x > o.w);
+            px = ci.offset + static_cast<int64_t>((y - 1) / 2 + 1) * (ci.w + 2) + ((x - 1) / 2 + 1);
         }
         uint4 const* p = valid ? base + px * kChunks : base;
 #pragma unroll
@@ -391,10 +408,8 @@ __global__ void __launch_bounds__(128) conv3x3_kernel(const __grid_constant__ Ta
         s.pre);
     // a CTA without an active tile leaves before staging weights or taking TMEM
     if (static_cast<int64_t>(blockIdx.x) >= s.pre[t.nimg]) return;
-    for (int i = tid; i < kKChunks * kCh; i += 128) {
-        int const co = i & 31, k = i >> 5;
-        s.w[k * kCh + co] = __ldg(reinterpret_cast<uint4 const*>(wt + co * (kTaps * kCh)) + k);
-    }
+#pragma unroll
+    for (int i = 0; i < kKChunks * kCh / 128; ++i) s.w[tid + i * 128] = __ldg(reinterpret_cast<uint4 const*>(wt) + tid + i * 128);
     if (out_taps != nullptr)
         for (int i = tid; i < kCh * 12; i += 128) {
             int const ci = i / 12, tap = i - ci * 12;
@@ -410,7 +425,7 @@ __global__ void __launch_bounds__(128) conv3x3_kernel(const __grid_constant__ Ta
     tc_fence_after();
     uint32_t const tmem = s.tmem;
     uint32_t const halo_addr[2] = {smem_u32(s.halo[0]), smem_u32(s.halo[1])};
-    uint32_t const w_addr = smem_u32(s.w);
+    uint64_t const b0 = umma_desc(smem_u32(s.w), kCh * 16, 128);
     int const nops = mode == kUpAdd ? 2 : 1;
     // kPlain runs a two-stage ring over the two halo buffers: the next tile's
     // cp.async loads are in flight while this tile's MMAs and epilogue run.
@@ -424,7 +439,7 @@ __global__ void __launch_bounds__(128) conv3x3_kernel(const __grid_constant__ Ta
         int const im2 = find_image(t, tl);
         int const P2 = t.img[im2].w + 2;
         int const start2 = P2 + (tl - t.tile_base[im2]) * kTilePx;
-        stage_halo(s.halo[buf], t, im2, start2, P2, in, false);
+        stage_halo_plain(s.halo[buf], t, im2, start2, P2, in);
         cp_async_commit();
     };
     // active tiles handed out round-robin; unit a is tile tile_of(a)
@@ -453,8 +468,8 @@ __global__ void __launch_bounds__(128) conv3x3_kernel(const __grid_constant__ Ta
                 cp_async_wait_all();
             }
         } else if (mode == kUpAdd) {
-            stage_halo(s.halo[0], t, im, start, P, in, false);
-            stage_halo(s.halo[1], t, im, start, P, in2, true);
+            stage_halo_plain(s.halo[0], t, im, start, P, in);
+            stage_halo_up(s.halo[1], t, im, start, P, in2);
             cp_async_wait_all();
         } else {
             load_halo(s.halo[0], mode, t, im, start, P, in, in2, gin);
@@ -463,20 +478,16 @@ __global__ void __launch_bounds__(128) conv3x3_kernel(const __grid_constant__ Ta
         __syncthreads();
         if (tid == 0) {
             tc_fence_after();
-            int step = 0;
-#pragma unroll 1
+            // Descriptors differ from the first tap's by constant distances in
+            // their address field (16-byte units), so each MMA costs two adds.
             for (int op = 0; op < nops; ++op) {
-#pragma unroll 1
-                for (int tap = 0; tap < kTaps; ++tap) {
-                    int const dy = tap / 3, dx = tap % 3;
+                uint64_t const a0 = umma_desc(halo_addr[ring ? cur : op], 3 * kHalo * 16, 128);
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        uint64_t const a = umma_desc(halo_addr[ring ? cur : op] + ((2 * h * 3 + dy) * kHalo + dx) * 16,
-                                                     3 * kHalo * 16, 128);
-                        uint64_t const b = umma_desc(w_addr + (tap * kChunks + 2 * h) * kCh * 16, kCh * 16, 128);
-                        umma_bf16(tmem, a, b, kIdescFwd, step > 0 ? 1u : 0u);
-                        ++step;
-                    }
+                for (int tap = 0; tap < kTaps; ++tap) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        umma_bf16(tmem, a0 + ((2 * h * 3 + tap / 3) * kHalo + tap % 3), b0 + (tap * kChunks + 2 * h) * kCh,
+                                  kIdescFwd, op > 0 || tap > 0 || h > 0 ? 1u : 0u);
                 }
             }
             umma_commit(&s.bar);
@@ -642,8 +653,7 @@ __global__ void __launch_bounds__(128) wgrad_kernel(const __grid_constant__ Tabl
     __syncthreads();
     tc_fence_after();
     uint32_t const tmem = s.tmem;
-    uint32_t const col_addr = smem_u32(s.col);
-    uint32_t const dz_addr = smem_u32(s.dz);
+    uint64_t const a0 = umma_desc(smem_u32(s.col), 128, kTilePx * 16), b0 = umma_desc(smem_u32(s.dz), 128, kTilePx * 16);
     uint32_t phase = 0;
     float db = 0.0f;  // thread co = tid (< 32) accumulates the bias gradient
     bool any = false;
@@ -687,14 +697,12 @@ __global__ void __launch_bounds__(128) wgrad_kernel(const __grid_constant__ Tabl
             __syncthreads();
             if (tid == 0) {
                 tc_fence_after();
-#pragma unroll 1
+#pragma unroll
                 for (int mt = 0; mt < 3; ++mt) {
 #pragma unroll
-                    for (int kk = 0; kk < kTilePx / 16; ++kk) {
-                        uint64_t const a = umma_desc(col_addr + (16 * mt * kTilePx + kk * 16) * 16, 128, kTilePx * 16);
-                        uint64_t const b = umma_desc(dz_addr + kk * 16 * 16, 128, kTilePx * 16);
-                        umma_bf16(tmem + mt * 32, a, b, kIdescWgrad, (any || kk > 0) ? 1u : 0u);
-                    }
+                    for (int kk = 0; kk < kTilePx / 16; ++kk)
+                        umma_bf16(tmem + mt * 32, a0 + (16 * mt * kTilePx + kk * 16), b0 + kk * 16, kIdescWgrad,
+                                  (any || kk > 0) ? 1u : 0u);
                 }
                 umma_commit(&s.bar);
             }
@@ -756,8 +764,10 @@ __global__ void __launch_bounds__(256) reduce_parts_kernel(float const* part, in
     grad[i] = grad[i] + total;
 }
 
-// BF16 weights of the 32->32 convolutions: forward [co][tap][ci] and, for
-// the data gradient, transposed and flipped [ci][8 - tap][co].
+// BF16 weights of the 32->32 convolutions in the order the convolution holds
+// them in shared memory, [K chunk][output channel][8 channels] with K =
+// (tap, input channel), so a CTA copies them straight: forward, and for the
+// data gradient transposed and flipped (K = (8 - tap, co), output ci).
 __global__ void convert_weights_kernel(float const* params, bf16* wf, bf16* wt)
 {
     int const i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -765,8 +775,9 @@ __global__ void convert_weights_kernel(float const* params, bf16* wf, bf16* wt)
     int const j = i / kBigW, r = i % kBigW;
     int const co = r / (kTaps * kCh), tap = (r / kCh) % kTaps, ci = r % kCh;
     bf16 const v = __float2bfloat16_rn(params[kOffBig + j * kBigParams + r]);
-    wf[i] = v;
-    wt[j * kBigW + ci * (kTaps * kCh) + (kTaps - 1 - tap) * kCh + co] = v;
+    auto at = [](int out, int k) { return (k / 8 * kCh + out) * 8 + k % 8; };
+    wf[j * kBigW + at(co, tap * kCh + ci)] = v;
+    wt[j * kBigW + at(ci, (kTaps - 1 - tap) * kCh + co)] = v;
 }
 
 // ------------------------------------------------------------------ thin layers (CUDA cores)

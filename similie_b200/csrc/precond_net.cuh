@@ -106,7 +106,7 @@ public:
     float* grad = nullptr;     // device FP32 [kNumParams]
     float* adam_m = nullptr;
     float* adam_v = nullptr;
-    void* wbf = nullptr;       // device BF16 forward weights [kNumBig][32][9][32]
+    void* wbf = nullptr;       // device BF16 forward weights, in the convolution's shared-memory order
     void* wbf_t = nullptr;     // device BF16 transposed weights for the data gradient
     int adam_t = 0;
     int* error_flag = nullptr;
