@@ -844,35 +844,6 @@ __device__ __forceinline__ Begin cg_begin(Scalars* s, int c, double const* part_
     return b;
 }
 
-// ---- 2D strips: the 2D operator marched down a strip of columns, a warp per
-// strip.  Lane l holds column c0 - 1 + l; lanes 1..30 own theirs.  Walking down
-// the rows a column's operand and reluctivity at rows j - 1 and j stay in
-// registers and its neighbours' come from the next lanes, so a node costs one
-// load per input array where a thread per node made fourteen; four rows' loads
-// are in flight before the first is used.  The values are those of
-// mag_apply_node_ij (an excluded term adds a zero).
-constexpr int kStripCols = 30;
-constexpr int kStripBatch = 4;   // rows whose loads are issued together
-
-// Strips of a problem: strip w % strips of row block w / strips, `rows` rows each.
-struct Strips
-{
-    int strips;    // per row block
-    int rows;      // per strip, a multiple of kStripBatch
-    int count;     // in all
-    int ctas;      // of kThreads / 32 strips
-};
-
-__host__ __device__ inline Strips strips_of(int64_t nx, int64_t ny, int rows)
-{
-    Strips s {};
-    s.strips = static_cast<int>((nx + kStripCols - 1) / kStripCols);
-    s.rows = rows;
-    s.count = s.strips * static_cast<int>((ny + rows - 1) / rows);
-    s.ctas = (s.count + kThreads / 32 - 1) / (kThreads / 32);
-    return s;
-}
-
 // Rows per strip: the fewest, in steps of four, at which the batch fits one
 // wave of two CTAs per multiprocessor; 32 at most (a strip of R rows reads
 // R + 2, and one wave of longer ones leaves too few loads in flight).
@@ -885,59 +856,6 @@ int strip_rows(std::vector<ProbInfo> const& grids)
         if (ctas <= 2 * static_cast<int64_t>(sm_count())) break;
     }
     return rows;
-}
-
-// Src: Raw load(row), T value(Raw), and out(row, q, raw): the result of an
-// owned row and its operand.
-template <class T, class Src, class Out>
-__device__ __forceinline__ void mag2d_strip(Src const& src, T const* __restrict__ nu, int nx, int ny, int c0, int j0,
-                                            int j1, Out const& out)
-{
-    constexpr int U = kStripBatch;
-    int const lane = threadIdx.x & 31, i = c0 - 1 + lane, ic = min(max(i, 0), nx - 1);
-    bool const own = lane > 0 && lane <= kStripCols && i < nx, col_in = i > 0 && i + 1 < nx, left_in = i >= 2;
-    auto row_of = [&](int j) { return ic + nx * min(max(j, 0), ny - 1); };
-    typename Src::Raw const raw_m = src.load(row_of(j0 - 1));
-    typename Src::Raw raw_c = src.load(row_of(j0));
-    T n_m = nu[row_of(j0 - 1)], n_c = nu[row_of(j0)];
-    T below = T(0), centre = T(0);
-    bool first = true;
-    for (int j = j0; j < j1; j += U) {
-        typename Src::Raw raw[U];
-        typename Src::Own mine[U];
-        T n[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            int const at = row_of(j + 1 + u);
-            raw[u] = src.load(at);
-            n[u] = nu[at];
-            mine[u] = src.own(row_of(j + u));
-        }
-        if (first) {
-            below = src.value(raw_m);
-            centre = src.value(raw_c);
-            first = false;
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            T const above = src.value(raw[u]);
-            T const left = __shfl_up_sync(0xffffffffu, centre, 1), right = __shfl_down_sync(0xffffffffu, centre, 1);
-            T const n_l = __shfl_up_sync(0xffffffffu, n_c, 1);
-            int const jj = j + u;
-            T res = T(0);
-            if (jj >= 2) res = res + (centre - below) * n_m;
-            res = res - (above - centre) * n_c;
-            if (left_in) res = res - (left - centre) * n_l;
-            res = res + (centre - right) * n_c;
-            bool const in = col_in && jj > 0 && jj + 1 < ny;
-            if (own && jj < j1) out(ic + nx * jj, in ? res : centre, centre, raw_c, mine[u]);
-            below = centre;
-            centre = above;
-            raw_c = raw[u];
-            n_m = n_c;
-            n_c = n[u];
-        }
-    }
 }
 
 // Operand z + beta p_old of the search direction, x on the side.

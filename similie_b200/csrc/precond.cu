@@ -97,6 +97,30 @@ __device__ __forceinline__ uint4 pack8(float const* f)
     return u;
 }
 
+// Two FP32 fused multiply-adds in one instruction, each rounded as __fmaf_rn.
+struct Float2x
+{
+    uint64_t v;
+};
+__device__ __forceinline__ Float2x pair2(float lo, float hi)
+{
+    Float2x r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 split2(Float2x p)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p.v));
+    return r;
+}
+__device__ __forceinline__ Float2x fma2(Float2x a, Float2x b, Float2x c)
+{
+    Float2x r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+
 __device__ __forceinline__ uint4 ld_chunk(bf16 const* base, int64_t px, int c)
 {
     return __ldg(reinterpret_cast<uint4 const*>(base + px * kCh) + c);
@@ -382,92 +406,275 @@ struct ConvSmem
 {
     uint4 w[kKChunks * kCh];              // B operand: [K chunk][output channel], 18432 B
     float4 wout[kCh][3];                  // output-convolution weights [input channel][tap, 12 with padding]
-    uint64_t bar;
+    uint64_t bar[2];
     uint32_t tmem;
     int abort;
     int64_t pre[kMaxImages + 1];          // prefix of the active images' tiles
     uint4 halo[2][kChunks * 3 * kHalo];   // A operand sources: [chunk][halo row][halo pixel], 2 x 24960 B
 };
 
-// out = act(conv3x3(input) + bias) for the interior pixels of every image of
-// the table; border pixels are written as zero.  out (BF16) may be NULL;
-// out_f32 selects an FP32 output (data gradients), accumulate adds into it;
-// out_taps (with wout) writes the nine partial sums of the 32 -> 1 output
-// convolution per pixel, taps[tap][pixel], for a separate gather.
-__global__ void __launch_bounds__(128) conv3x3_kernel(const __grid_constant__ Table t, int mode, bf16 const* in,
-                                                      bf16 const* in2, float const* gin, bf16 const* wt,
-                                                      float const* bias, int relu, bf16* out, float* out_f32,
-                                                      int accumulate, float* out_taps, float const* wout,
-                                                      int64_t taps_stride, int* error_flag)
+// Where a convolution's results go: bias / ReLU applied, out (BF16), out_f32
+// (with accumulate) and out_taps as conv3x3_kernel describes them.
+struct ConvOut
 {
-    extern __shared__ __align__(1024) unsigned char smem_raw[];
-    ConvSmem& s = *reinterpret_cast<ConvSmem*>(smem_raw);
-    int const tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    scan_active(
-        t.nimg, [&](int k) { return image_active(t, k) ? int64_t(t.tile_base[k + 1] - t.tile_base[k]) : int64_t(0); },
-        s.pre);
-    // a CTA without an active tile leaves before staging weights or taking TMEM
-    if (static_cast<int64_t>(blockIdx.x) >= s.pre[t.nimg]) return;
+    float const* bias;
+    int relu;
+    bf16* out;
+    float* out_f32;
+    int accumulate;
+    float* out_taps;
+    int64_t taps_stride;
+};
+
+// Epilogue of one 128-pixel tile from its accumulator (a pixel per thread).
+__device__ __forceinline__ void conv_epilogue(ConvOut const& w, float const (&bias_r)[32], float4 const (*wout)[3],
+                                              uint32_t tmem, Img const& o, int start)
+{
+    int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31, P = o.w + 2;
+    float acc[32];
+    tmem_ld32(tmem + (static_cast<uint32_t>(warp * 32) << 16), acc);
+    int const g = start + warp * 32 + lane;
+    if (g < P * (o.h + 1)) {
+        int const x = g % P;
+        bool const border = x == 0 || x == P - 1;
+        if (border) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
+        } else {
+            if (w.bias != nullptr) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) acc[i] = acc[i] + bias_r[i];
+            }
+            if (w.relu) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) acc[i] = fmaxf(acc[i], 0.0f);
+            }
+        }
+        int64_t const px = o.offset + g;
+        if (w.out_f32 != nullptr) {
+            float4* dst = reinterpret_cast<float4*>(w.out_f32 + px * kCh);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                float4 v = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+                if (w.accumulate) {
+                    float4 const o4 = dst[q];
+                    v.x = v.x + o4.x;
+                    v.y = v.y + o4.y;
+                    v.z = v.z + o4.z;
+                    v.w = v.w + o4.w;
+                }
+                dst[q] = v;
+            }
+        }
+        if (w.out != nullptr || w.out_taps != nullptr) {
+            uint4 packed[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) packed[q] = pack8(acc + 8 * q);
+            if (w.out != nullptr) {
+                uint4* dst = reinterpret_cast<uint4*>(w.out + px * kCh);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) dst[q] = packed[q];
+            }
+            if (w.out_taps != nullptr) {
+                // partials of the output convolution from the BF16-rounded activations
+                float f[32];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) unpack8(packed[q], f + 8 * q);
+                // nine accumulators side by side, eight of them in pairs; each
+                // tap still sums its 32 channels in order from zero
+                Float2x a2[4];
+                float a[kTaps];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) a2[k] = pair2(0.0f, 0.0f);
+                a[8] = 0.0f;
+#pragma unroll
+                for (int ci = 0; ci < 32; ++ci) {
+                    float4 const w0 = wout[ci][0], w1 = wout[ci][1];
+                    Float2x const v = pair2(f[ci], f[ci]);
+                    a2[0] = fma2(pair2(w0.x, w0.y), v, a2[0]);
+                    a2[1] = fma2(pair2(w0.z, w0.w), v, a2[1]);
+                    a2[2] = fma2(pair2(w1.x, w1.y), v, a2[2]);
+                    a2[3] = fma2(pair2(w1.z, w1.w), v, a2[3]);
+                    a[8] = __fmaf_rn(wout[ci][2].x, f[ci], a[8]);
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    float2 const q = split2(a2[k]);
+                    a[2 * k] = q.x;
+                    a[2 * k + 1] = q.y;
+                }
+#pragma unroll
+                for (int tap = 0; tap < kTaps; ++tap) w.out_taps[tap * w.taps_stride + px] = a[tap];
+            }
+        }
+    }
+}
+
+// The 18 MMAs of one operand, issued by one thread: descriptors differ from the
+// first tap's by constant distances in their address field (16-byte units), so
+// each costs two adds.
+__device__ __forceinline__ void issue_taps(uint32_t tmem, uint32_t halo, uint64_t b0, bool accumulate)
+{
+    uint64_t const a0 = umma_desc(halo, 3 * kHalo * 16, 128);
+#pragma unroll
+    for (int tap = 0; tap < kTaps; ++tap) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            umma_bf16(tmem, a0 + ((2 * h * 3 + tap / 3) * kHalo + tap % 3), b0 + (tap * kChunks + 2 * h) * kCh, kIdescFwd,
+                      accumulate || tap > 0 || h > 0 ? 1u : 0u);
+    }
+}
+
+// What both convolution kernels do before their first tile: weights to shared
+// memory, TMEM columns, the barriers.
+__device__ __forceinline__ void conv_setup(ConvSmem& s, bf16 const* wt, float const* wout, uint32_t columns)
+{
+    int const tid = threadIdx.x;
 #pragma unroll
     for (int i = 0; i < kKChunks * kCh / 128; ++i) s.w[tid + i * 128] = __ldg(reinterpret_cast<uint4 const*>(wt) + tid + i * 128);
-    if (out_taps != nullptr)
+    if (wout != nullptr)
         for (int i = tid; i < kCh * 12; i += 128) {
             int const ci = i / 12, tap = i - ci * 12;
             reinterpret_cast<float*>(s.wout[ci])[tap] = tap < kTaps ? wout[tap * kCh + ci] : 0.0f;
         }
-    if (warp == 0) tmem_alloc(&s.tmem, 32);
+    if (tid < 32) tmem_alloc(&s.tmem, columns);
     if (tid == 0) {
-        mbar_init(&s.bar, 1);
+        mbar_init(&s.bar[0], 1);
+        mbar_init(&s.bar[1], 1);
         s.abort = 0;
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+}
+
+__device__ __forceinline__ void conv_teardown(ConvSmem& s, int* error_flag, uint32_t columns)
+{
+    cp_async_wait_all();  // no copy may still target this CTA's shared memory at exit
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (s.abort && threadIdx.x == 0) atomicExch(error_flag, 1);
+    if (threadIdx.x < 32) tmem_dealloc(s.tmem, columns);
+}
+
+// out = act(conv3x3(in) + bias) of a level's own tensor, for the interior pixels
+// of every active image of the table (border pixels are written as zero; the
+// forms of output are ConvOut's).  Two halo buffers and two accumulators keep
+// one tile ahead: while a tile's epilogue runs, the next tile's MMAs run and
+// the copies of the one after it are on their way, with one barrier a tile.
+// Bound by latency still, with three CTAs of four warps on a multiprocessor.
+// B200, the 32 -> 1 folding decoder of 1 M pixels: 101 us with the MMAs waited
+// for before each epilogue, here 82.
+__global__ void __launch_bounds__(128) conv3x3_plain_kernel(const __grid_constant__ Table t, bf16 const* in, bf16 const* wt,
+                                                            ConvOut const dst, float const* wout, int* error_flag)
+{
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    ConvSmem& s = *reinterpret_cast<ConvSmem*>(smem_raw);
+    int const tid = threadIdx.x;
+    scan_active(
+        t.nimg, [&](int k) { return image_active(t, k) ? int64_t(t.tile_base[k + 1] - t.tile_base[k]) : int64_t(0); },
+        s.pre);
+    // a CTA without an active tile leaves before staging weights or taking TMEM
+    int const nact = static_cast<int>(s.pre[t.nimg]), G = static_cast<int>(gridDim.x);
+    if (static_cast<int>(blockIdx.x) >= nact) return;
+    // active tiles handed out round-robin
+    struct Place
+    {
+        int im, start;
+    };
+    auto place_of = [&](int a) -> Place {
+        int const k = find_unit(s.pre, t.nimg, a);
+        return {k, t.img[k].w + 2 + (a - static_cast<int>(s.pre[k])) * kTilePx};
+    };
+    auto stage = [&](Place const& p, int buf) {
+        stage_halo_plain(s.halo[buf], t, p.im, p.start, t.img[p.im].w + 2, in);
+        cp_async_commit();
+    };
+    Place now = place_of(blockIdx.x), next {};
+    stage(now, 0);
+    int a = blockIdx.x;
+    if (a + G < nact) {
+        next = place_of(a + G);
+        stage(next, 1);
+    }
+    conv_setup(s, wt, dst.out_taps != nullptr ? wout : nullptr, 64);
+    uint32_t const tmem = s.tmem;
+    uint64_t const b0 = umma_desc(smem_u32(s.w), kCh * 16, 128);
+    float bias_r[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) bias_r[i] = dst.bias != nullptr ? __ldg(dst.bias + i) : 0.0f;
+    if (a + G < nact) cp_async_wait_group1();
+    else cp_async_wait_all();
+    fence_async_smem();
+    __syncthreads();
+    if (tid == 0) {
+        tc_fence_after();
+        issue_taps(tmem, smem_u32(s.halo[0]), b0, false);
+        umma_commit(&s.bar[0]);
+    }
+    uint32_t phase = 0;   // bit b: parity of barrier b's next completion
+    bool lost = false;
+    for (int buf = 0; a < nact; a += G, buf ^= 1) {
+        bool const more = a + G < nact;
+        if (more) {
+            // the next tile's copies have landed: its MMAs go to the other accumulator,
+            // whose previous tile every warp has read by this barrier
+            cp_async_wait_all();
+            fence_async_smem();
+            if (__syncthreads_or(lost)) break;
+            if (tid == 0) {
+                tc_fence_after();
+                issue_taps(tmem + (buf ^ 1) * 32, smem_u32(s.halo[buf ^ 1]), b0, false);
+                umma_commit(&s.bar[buf ^ 1]);
+            }
+            __syncwarp();
+        }
+        bool const done = __all_sync(0xffffffffu, mbar_wait(&s.bar[buf], (phase >> buf) & 1u));
+        phase ^= 1u << buf;
+        if (!done) {
+            lost = true;
+            s.abort = 1;
+            continue;
+        }
+        Place after {};
+        if (a + 2 * G < nact) {
+            after = place_of(a + 2 * G);
+            stage(after, buf);   // this tile's MMAs have read the buffer
+        }
+        tc_fence_after();
+        conv_epilogue(dst, bias_r, s.wout, tmem + buf * 32, t.img[now.im], now.start);
+        tc_fence_before();
+        now = next;
+        next = after;
+    }
+    conv_teardown(s, error_flag, 64);
+}
+
+// The other inputs of a convolution (training): kUpAdd, skip + nearest-upsampled
+// coarse tensor as two operands summed in the accumulator, and kMasked, an FP32
+// gradient masked by activity; one tile at a time.
+__global__ void __launch_bounds__(128, 4) conv3x3_kernel(const __grid_constant__ Table t, int mode, bf16 const* in,
+                                                      bf16 const* in2, float const* gin, bf16 const* wt,
+                                                      ConvOut const dst, int* error_flag)
+{
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    ConvSmem& s = *reinterpret_cast<ConvSmem*>(smem_raw);
+    int const tid = threadIdx.x;
+    conv_setup(s, wt, nullptr, 32);
     uint32_t const tmem = s.tmem;
     uint32_t const halo_addr[2] = {smem_u32(s.halo[0]), smem_u32(s.halo[1])};
     uint64_t const b0 = umma_desc(smem_u32(s.w), kCh * 16, 128);
-    int const nops = mode == kUpAdd ? 2 : 1;
-    // kPlain runs a two-stage ring over the two halo buffers: the next tile's
-    // cp.async loads are in flight while this tile's MMAs and epilogue run.
-    bool const ring = mode == kPlain;
     float bias_r[32];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) bias_r[i] = bias != nullptr ? __ldg(bias + i) : 0.0f;
+    for (int i = 0; i < 32; ++i) bias_r[i] = dst.bias != nullptr ? __ldg(dst.bias + i) : 0.0f;
     uint32_t phase = 0;
-    int const ntiles = t.tile_base[t.nimg];
-    auto stage = [&](int tl, int buf) {
-        int const im2 = find_image(t, tl);
-        int const P2 = t.img[im2].w + 2;
-        int const start2 = P2 + (tl - t.tile_base[im2]) * kTilePx;
-        stage_halo_plain(s.halo[buf], t, im2, start2, P2, in);
-        cp_async_commit();
-    };
-    // active tiles handed out round-robin; unit a is tile tile_of(a)
-    int const nact = static_cast<int>(s.pre[t.nimg]);
-    auto tile_of = [&](int a) {
-        int const k = find_unit(s.pre, t.nimg, a);
-        return t.tile_base[k] + (a - static_cast<int>(s.pre[k]));
-    };
-    int tile = static_cast<int>(blockIdx.x) < nact ? tile_of(blockIdx.x) : ntiles;
-    if (ring && tile < ntiles) stage(tile, 0);
-    int iter = 0;
-    for (int a = blockIdx.x; a < nact; a += gridDim.x, ++iter) {
+    for (int tile = blockIdx.x; tile < t.tile_base[t.nimg]; tile += gridDim.x) {
         int const im = find_image(t, tile);
         Img const o = t.img[im];
         int const P = o.w + 2;
         int const start = P + (tile - t.tile_base[im]) * kTilePx;
-        int const an = a + static_cast<int>(gridDim.x);
-        int const nxt = an < nact ? tile_of(an) : ntiles;
-        int cur = 0;
-        if (ring) {
-            cur = iter & 1;
-            if (nxt < ntiles) {
-                stage(nxt, cur ^ 1);
-                cp_async_wait_group1();
-            } else {
-                cp_async_wait_all();
-            }
-        } else if (mode == kUpAdd) {
+        if (mode == kUpAdd) {
             stage_halo_plain(s.halo[0], t, im, start, P, in);
             stage_halo_up(s.halo[1], t, im, start, P, in2);
             cp_async_wait_all();
@@ -478,109 +685,22 @@ __global__ void __launch_bounds__(128) conv3x3_kernel(const __grid_constant__ Ta
         __syncthreads();
         if (tid == 0) {
             tc_fence_after();
-            // Descriptors differ from the first tap's by constant distances in
-            // their address field (16-byte units), so each MMA costs two adds.
-            for (int op = 0; op < nops; ++op) {
-                uint64_t const a0 = umma_desc(halo_addr[ring ? cur : op], 3 * kHalo * 16, 128);
-#pragma unroll
-                for (int tap = 0; tap < kTaps; ++tap) {
-#pragma unroll
-                    for (int h = 0; h < 2; ++h)
-                        umma_bf16(tmem, a0 + ((2 * h * 3 + tap / 3) * kHalo + tap % 3), b0 + (tap * kChunks + 2 * h) * kCh,
-                                  kIdescFwd, op > 0 || tap > 0 || h > 0 ? 1u : 0u);
-                }
-            }
-            umma_commit(&s.bar);
+            issue_taps(tmem, halo_addr[0], b0, false);
+            if (mode == kUpAdd) issue_taps(tmem, halo_addr[1], b0, true);
+            umma_commit(&s.bar[0]);
         }
         __syncwarp();
-        bool const done = mbar_wait(&s.bar, phase);
+        bool const done = mbar_wait(&s.bar[0], phase);
         phase ^= 1u;
         if (!done) s.abort = 1;
         __syncthreads();
         if (s.abort) break;
         tc_fence_after();
-        float acc[32];
-        tmem_ld32(tmem + (static_cast<uint32_t>(warp * 32) << 16), acc);
-        int const g = start + warp * 32 + lane;
-        if (g < P * (o.h + 1)) {
-            int const x = g % P;
-            bool const border = x == 0 || x == P - 1;
-            if (border) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
-            } else {
-                if (bias != nullptr) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) acc[i] = acc[i] + bias_r[i];
-                }
-                if (relu) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) acc[i] = fmaxf(acc[i], 0.0f);
-                }
-            }
-            int64_t const px = o.offset + g;
-            if (out_f32 != nullptr) {
-                float4* dst = reinterpret_cast<float4*>(out_f32 + px * kCh);
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    float4 v = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
-                    if (accumulate) {
-                        float4 const o4 = dst[q];
-                        v.x = v.x + o4.x;
-                        v.y = v.y + o4.y;
-                        v.z = v.z + o4.z;
-                        v.w = v.w + o4.w;
-                    }
-                    dst[q] = v;
-                }
-            }
-            if (out != nullptr || out_taps != nullptr) {
-                uint4 packed[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) packed[q] = pack8(acc + 8 * q);
-                if (out != nullptr) {
-                    uint4* dst = reinterpret_cast<uint4*>(out + px * kCh);
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) dst[q] = packed[q];
-                }
-                if (out_taps != nullptr) {
-                    // partials of the output convolution from the BF16-rounded activations
-                    float f[32];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) unpack8(packed[q], f + 8 * q);
-                    // nine accumulators side by side; each tap still sums its 32
-                    // channels in order from zero
-                    float a[kTaps];
-#pragma unroll
-                    for (int tap = 0; tap < kTaps; ++tap) a[tap] = 0.0f;
-#pragma unroll
-                    for (int ci = 0; ci < 32; ++ci) {
-                        float4 const w0 = s.wout[ci][0], w1 = s.wout[ci][1], w2 = s.wout[ci][2];
-                        a[0] = __fmaf_rn(w0.x, f[ci], a[0]);
-                        a[1] = __fmaf_rn(w0.y, f[ci], a[1]);
-                        a[2] = __fmaf_rn(w0.z, f[ci], a[2]);
-                        a[3] = __fmaf_rn(w0.w, f[ci], a[3]);
-                        a[4] = __fmaf_rn(w1.x, f[ci], a[4]);
-                        a[5] = __fmaf_rn(w1.y, f[ci], a[5]);
-                        a[6] = __fmaf_rn(w1.z, f[ci], a[6]);
-                        a[7] = __fmaf_rn(w1.w, f[ci], a[7]);
-                        a[8] = __fmaf_rn(w2.x, f[ci], a[8]);
-                    }
-#pragma unroll
-                    for (int tap = 0; tap < kTaps; ++tap) out_taps[tap * taps_stride + px] = a[tap];
-                }
-            }
-        }
+        conv_epilogue(dst, bias_r, s.wout, tmem, o, start);
         tc_fence_before();
         __syncthreads();
-        tile = nxt;
     }
-    cp_async_wait_all();  // no copy may still target this CTA's shared memory at exit
-    if (s.abort && tid == 0) atomicExch(error_flag, 1);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    if (warp == 0) tmem_dealloc(tmem, 32);
+    conv_teardown(s, error_flag, 32);
 }
 
 // Output convolution from the tap partials: out[p] = b + sum_tap taps[tap][p + tap] (zero border).
@@ -605,16 +725,37 @@ __global__ void out_gather_kernel(const __grid_constant__ Table t, float const* 
     });
 }
 
-// Coarse tensor = 2x2 average of the finer level (t.img coarse, t.aux fine), BF16.
+// Coarse tensor = 2x2 average of the finer level (t.img coarse, t.aux fine),
+// BF16.  A thread per 16-byte chunk of a pixel, so a warp's loads and stores
+// are runs of whole pixels (a thread per pixel put its lanes 128 bytes apart:
+// 30 us at 1 M pixels, this one 15).
 __global__ void pool_kernel(const __grid_constant__ Table t, bf16 const* fine, bf16* coarse)
 {
     __shared__ int64_t pre[kMaxImages + 1];
-    walk_active(t, pre, 1, [&](int im, int g) {
-        uint4 v[kChunks];
-        load_pixel(kPool, t, im, g, fine, nullptr, nullptr, v);
-        uint4* dst = reinterpret_cast<uint4*>(coarse) + (t.img[im].offset + g) * kChunks;
+    walk_active(t, pre, kChunks, [&](int im, int q) {
+        Img const o = t.img[im], fi = t.aux[im];
+        int const g = q / kChunks, c = q % kChunks, P = o.w + 2;
+        int const y = g / P, x = g - y * P;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (!(y == 0 || x == 0 || y > o.h || x > o.w)) {
+            int const Pf = fi.w + 2;
+            uint4 const* src = reinterpret_cast<uint4 const*>(fine)
+                               + (fi.offset + static_cast<int64_t>(2 * y - 1) * Pf + (2 * x - 1)) * kChunks + c;
+            uint4 const raw[4] = {__ldg(src), __ldg(src + kChunks), __ldg(src + Pf * kChunks), __ldg(src + (Pf + 1) * kChunks)};
+            float f[8], a[8];
 #pragma unroll
-        for (int c = 0; c < kChunks; ++c) dst[c] = v[c];
+            for (int i = 0; i < 8; ++i) f[i] = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                unpack8(raw[k], a);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) f[i] = f[i] + a[i];
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) f[i] = f[i] * 0.25f;
+            v = pack8(f);
+        }
+        reinterpret_cast<uint4*>(coarse)[o.offset * kChunks + q] = v;
     });
 }
 
@@ -783,7 +924,10 @@ __global__ void convert_weights_kernel(float const* params, bf16* wf, bf16* wt)
 // ------------------------------------------------------------------ thin layers (CUDA cores)
 
 // Input convolution 2 -> 32 (+ bias, ReLU) from the FP32 2-channel feature
-// image; weights staged in shared memory, one pixel per thread.
+// image; weights staged in shared memory.  B200, 1 M pixels: 53 us with two
+// pixels of all channels per thread (its stores 128 bytes apart), here 45 with
+// two multiply-adds an instruction.
+constexpr int kIncRun = 4;
 __global__ void __launch_bounds__(256) inc_forward_kernel(const __grid_constant__ Table t, float const* feat,
                                                           float const* params, bf16* out)
 {
@@ -796,77 +940,75 @@ __global__ void __launch_bounds__(256) inc_forward_kernel(const __grid_constant_
         reinterpret_cast<float*>(w4[k])[co] = params[kOffIn + co * kTaps * 2 + k];
     }
     for (int i = threadIdx.x; i < kCh; i += blockDim.x) reinterpret_cast<float*>(b4)[i] = params[kOffIn + kInW + i];
-    // Two horizontally adjacent pixels per thread: their 3 x 3 windows share
-    // six of their nine taps, and each weight read from shared memory serves
-    // both; each pixel's sums keep the single-pixel order.
+    // A thread forms eight channels (chunk c, four neighbouring lanes a pixel) of
+    // kIncRun pixels in a row: their windows slide over one another, each weight
+    // read from shared memory serves all of them, and a warp stores whole pixels.
+    // Each channel's sum is bias, then the 18 inputs in order.
     scan_active(
         t.nimg,
-        [&](int k) { return image_active(t, k) ? (t.px_base[k + 1] - t.px_base[k] + 1) / 2 : int64_t(0); }, pre);
-    walk_range(pre, t.nimg, 1, [&](int im, int q) {
+        [&](int k) { return image_active(t, k) ? (t.px_base[k + 1] - t.px_base[k] + kIncRun - 1) / kIncRun : int64_t(0); },
+        pre);
+    walk_range(pre, t.nimg, kChunks, [&](int im, int e) {
         Img const o = t.img[im];
         int const P = o.w + 2;
         int const npx = P * (o.h + 2);
-        int const g0 = 2 * q;
-        bool inside[2];
+        int const g0 = e / kChunks * kIncRun, c = e % kChunks;
+        bool inside[kIncRun];
+        {
+            int y = g0 / P, x = g0 - y * P;
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            int const g = g0 + u;
-            int const y = g / P, x = g - y * P;
-            inside[u] = g < npx && !(y == 0 || x == 0 || y > o.h || x > o.w);
+            for (int u = 0; u < kIncRun; ++u) {
+                inside[u] = !(y == 0 || x == 0 || y > o.h || x > o.w);
+                if (++x == P) {
+                    x = 0;
+                    ++y;
+                }
+            }
         }
-        uint4* dst = reinterpret_cast<uint4*>(out + (o.offset + g0) * kCh);
         float2 const* f2 = reinterpret_cast<float2 const*>(feat) + o.offset;
-        // window columns g0-1 .. g0+2 of the rows above, at and below
-        float2 win[3][4];
+        // window columns g0-1 .. g0+kIncRun of the rows above, at and below
+        float2 win[3][kIncRun + 2];
 #pragma unroll
         for (int dy = 0; dy < 3; ++dy)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                bool const need = (c < 3 && inside[0]) || (c > 0 && inside[1]);
-                win[dy][c] = need ? f2[g0 + (dy - 1) * P + (c - 1)] : make_float2(0.0f, 0.0f);
+            for (int k = 0; k < kIncRun + 2; ++k) {
+                int const g = g0 + (dy - 1) * P + (k - 1);
+                win[dy][k] = g >= 0 && g < npx ? __ldg(f2 + g) : make_float2(0.0f, 0.0f);
             }
-        float in[2][kTaps * 2];
+        Float2x a[kIncRun][4];
+        float4 const b0 = b4[2 * c], b1 = b4[2 * c + 1];
 #pragma unroll
-        for (int u = 0; u < 2; ++u)
+        for (int u = 0; u < kIncRun; ++u) {
+            a[u][0] = pair2(b0.x, b0.y);
+            a[u][1] = pair2(b0.z, b0.w);
+            a[u][2] = pair2(b1.x, b1.y);
+            a[u][3] = pair2(b1.z, b1.w);
+        }
 #pragma unroll
-            for (int tap = 0; tap < kTaps; ++tap) {
-                float2 const v = win[tap / 3][tap % 3 + u];
-                in[u][2 * tap] = v.x;
-                in[u][2 * tap + 1] = v.y;
+        for (int k = 0; k < kTaps * 2; ++k) {
+            float4 const w0 = w4[k][2 * c], w1 = w4[k][2 * c + 1];
+            Float2x const w[4] = {pair2(w0.x, w0.y), pair2(w0.z, w0.w), pair2(w1.x, w1.y), pair2(w1.z, w1.w)};
+#pragma unroll
+            for (int u = 0; u < kIncRun; ++u) {
+                float2 const in = win[(k / 2) / 3][(k / 2) % 3 + u];
+                float const f = k % 2 == 0 ? in.x : in.y;
+                Float2x const v = pair2(f, f);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) a[u][i] = fma2(w[i], v, a[u][i]);
             }
-        // eight output channels at a time: bias, then the 18 inputs in order
-#pragma unroll 1
-        for (int qq = 0; qq < 4; ++qq) {
-            float a[2][8];
-            float4 const b0 = b4[2 * qq], b1 = b4[2 * qq + 1];
+        }
+        uint4* dst = reinterpret_cast<uint4*>(out + (o.offset + g0) * kCh) + c;
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                a[u][0] = b0.x; a[u][1] = b0.y; a[u][2] = b0.z; a[u][3] = b0.w;
-                a[u][4] = b1.x; a[u][5] = b1.y; a[u][6] = b1.z; a[u][7] = b1.w;
+        for (int u = 0; u < kIncRun; ++u) {
+            if (g0 + u >= npx) continue;
+            float r[8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float2 const q = split2(a[u][i]);
+                r[2 * i] = inside[u] ? fmaxf(q.x, 0.0f) : 0.0f;
+                r[2 * i + 1] = inside[u] ? fmaxf(q.y, 0.0f) : 0.0f;
             }
-#pragma unroll
-            for (int k = 0; k < kTaps * 2; ++k) {
-                float4 const w0 = w4[k][2 * qq], w1 = w4[k][2 * qq + 1];
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    float const v = in[u][k];
-                    a[u][0] = __fmaf_rn(w0.x, v, a[u][0]);
-                    a[u][1] = __fmaf_rn(w0.y, v, a[u][1]);
-                    a[u][2] = __fmaf_rn(w0.z, v, a[u][2]);
-                    a[u][3] = __fmaf_rn(w0.w, v, a[u][3]);
-                    a[u][4] = __fmaf_rn(w1.x, v, a[u][4]);
-                    a[u][5] = __fmaf_rn(w1.y, v, a[u][5]);
-                    a[u][6] = __fmaf_rn(w1.z, v, a[u][6]);
-                    a[u][7] = __fmaf_rn(w1.w, v, a[u][7]);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                if (g0 + u >= npx) continue;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) a[u][i] = inside[u] ? fmaxf(a[u][i], 0.0f) : 0.0f;
-                dst[u * kChunks + qq] = pack8(a[u]);
-            }
+            dst[u * kChunks] = pack8(r);
         }
     });
 }
@@ -1184,15 +1326,26 @@ __global__ void copy_act_kernel(const __grid_constant__ Table t, bf16 const* src
 // convolution reads one operand through the pipelined plain mode.  (The
 // training pass keeps the two operands, which the tensor core sums in FP32,
 // because the weight gradient needs them apart.)
+// A thread per 16-byte chunk, as pool_kernel (33 -> 31 us at 1 M pixels,
+// 10.5 -> 5.2 at 64 k).
 __global__ void upadd_kernel(const __grid_constant__ Table t, bf16 const* skip, bf16 const* coarse, bf16* out)
 {
     __shared__ int64_t pre[kMaxImages + 1];
-    walk_active(t, pre, 1, [&](int im, int g) {
-        uint4 v[kChunks];
-        load_pixel(kUpAdd, t, im, g, skip, coarse, nullptr, v);
-        uint4* dst = reinterpret_cast<uint4*>(out) + (t.img[im].offset + g) * kChunks;
+    walk_active(t, pre, kChunks, [&](int im, int q) {
+        Img const o = t.img[im], ci = t.aux[im];
+        int const g = q / kChunks, c = q % kChunks, P = o.w + 2;
+        int const y = g / P, x = g - y * P;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (!(y == 0 || x == 0 || y > o.h || x > o.w)) {
+            int64_t const cpx = ci.offset + static_cast<int64_t>((y - 1) / 2 + 1) * (ci.w + 2) + ((x - 1) / 2 + 1);
+            float f[8], a[8];
+            unpack8(__ldg(reinterpret_cast<uint4 const*>(skip) + o.offset * kChunks + q), f);
+            unpack8(__ldg(reinterpret_cast<uint4 const*>(coarse) + cpx * kChunks + c), a);
 #pragma unroll
-        for (int c = 0; c < kChunks; ++c) dst[c] = v[c];
+            for (int i = 0; i < 8; ++i) f[i] = f[i] + a[i];
+            v = pack8(f);
+        }
+        reinterpret_cast<uint4*>(out)[o.offset * kChunks + q] = v;
     });
 }
 
@@ -1204,6 +1357,8 @@ struct Samples
     Sample s[kMaxImages];
     Img top[kMaxImages];                 // level-0 network image of each sample
     int32_t item_base[kMaxImages + 1];   // first fused-wrapper work item of each sample
+    int32_t strip_base[kMaxImages + 1];  // first CTA of strips of each sample
+    int32_t strip_rows;                  // rows of a strip
     int const* active;                   // per sample: 0 = skip (NULL: all run)
 };
 
@@ -1217,26 +1372,6 @@ __device__ __forceinline__ bool node_of(Samples const& ss, int64_t& row, Sample&
     sm = ss.s[blockIdx.y];
     row = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     return row < static_cast<int64_t>(sm.nx) * sm.ny;
-}
-
-// dinv = 1 / diag(K) (identity on the boundary); nu given per node.
-__global__ void dinv_kernel(const __grid_constant__ Samples ss, float const* nu, float* dinv)
-{
-    int64_t row;
-    Sample sm;
-    if (!node_of(ss, row, sm)) return;
-    int64_t const nx = sm.nx, ny = sm.ny;
-    int64_t const i = row % nx, j = row / nx;
-    float const* v = nu + sm.offset;
-    float d = 1.0f;
-    if (!(i == 0 || j == 0 || i + 1 == nx || j + 1 == ny)) {
-        d = 0.0f;
-        if (j >= 2) d = d + v[row - nx];
-        d = d + v[row];
-        if (i >= 2) d = d + v[row - 1];
-        d = d + v[row];
-    }
-    dinv[sm.offset + row] = 1.0f / d;
 }
 
 // y = alpha * x + beta * dinv (b - K e)   with optional K e: general Jacobi-type update
@@ -1464,45 +1599,70 @@ __device__ __forceinline__ int item_of(Samples const& ss, int64_t const* pre, in
     return ss.item_base[k] + (a - static_cast<int>(pre[k]));
 }
 
-// r1 = r - K e1 with e1 = w D^-1 r formed on the fly at the row and its
-// neighbours (boundary rows: r1 = r - e1), and the partial sums of
-// |D^-1/2 r1|^2 per item.  A thread's (i, j) advance by adding, without a
-// division per node.
-__global__ void __launch_bounds__(256) wrap_pre_kernel(const __grid_constant__ Samples ss, WrapItem const* items,
-                                                       float const* nu, float const* dinv, float const* r,
-                                                       float* r1, double* part)
+// The active samples' CTAs of strips (mag_ops.cuh): f(sample, strip, j0, j1, c0,
+// cta) for the calling warp's strip of every CTA it is handed; `after(cta)` runs
+// for the whole block after each.
+template <class F, class A>
+__device__ __forceinline__ void walk_strips(Samples const& ss, int64_t* pre, F const& f, A const& after)
+{
+    scan_active(
+        ss.n, [&](int k) { return sample_active(ss, k) ? int64_t(ss.strip_base[k + 1] - ss.strip_base[k]) : int64_t(0); },
+        pre);
+    int const nact = static_cast<int>(pre[ss.n]);
+    for (int a = blockIdx.x; a < nact; a += gridDim.x) {
+        int const k = find_unit(pre, ss.n, a), within = a - static_cast<int>(pre[k]);
+        Sample const sm = ss.s[k];
+        Strips const st = strips_of(sm.nx, sm.ny, ss.strip_rows);
+        int const strip = within * kStripWarps + static_cast<int>(threadIdx.x >> 5);
+        if (strip < st.count) {
+            int const block = strip / st.strips, j0 = block * st.rows;
+            f(sm, (strip - block * st.strips) * kStripCols, j0, min(sm.ny, j0 + st.rows));
+        }
+        after(ss.strip_base[k] + within);
+    }
+}
+
+// Operand e1 = w D^-1 r.
+struct WrapPreSrc
+{
+    struct Raw
+    {
+        float d, r;
+    };
+    struct Own
+    {};
+    float const* __restrict__ d;
+    float const* __restrict__ r;
+    __device__ __forceinline__ Raw load(int row) const { return {d[row], r[row]}; }
+    __device__ __forceinline__ Own own(int) const { return {}; }
+    __device__ __forceinline__ float value(Raw const& v) const { return kOmega * (v.d * v.r); }
+};
+
+// r1 = r - K e1 with e1 = w D^-1 r formed on the fly (boundary rows: r1 = r - e1),
+// and the partial sums of |D^-1/2 r1|^2 per CTA of strips.  B200, 4.1 M nodes: a
+// thread per node with its own stencil 31 us, strips 17.
+__global__ void __launch_bounds__(256) wrap_pre_kernel(const __grid_constant__ Samples ss, float const* nu,
+                                                       float const* dinv, float const* r, float* r1, double* part)
 {
     __shared__ double red[8];
     __shared__ int64_t pre[kMaxImages + 1];
-    int const nact = scan_items(ss, pre);
-    for (int a = blockIdx.x; a < nact; a += gridDim.x) {
-        int const item = item_of(ss, pre, a);
-        WrapItem const it = items[item];
-        Sample const sm = ss.s[it.sample];
-        int const nx = sm.nx, ny = sm.ny;
-        float const* nu_s = nu + sm.offset;
-        float const* d_s = dinv + sm.offset;
-        float const* r_s = r + sm.offset;
-        auto e = [&](int q, int, int) { return kOmega * (d_s[q] * r_s[q]); };
-        double acc = 0.0;
-        int row = it.begin + static_cast<int>(threadIdx.x);
-        int j = row / nx, i = row - j * nx;
-        for (; row < it.end; row += blockDim.x) {
-            float const ev = e(row, i, j);
-            float v;
-            if (i == 0 || j == 0 || i + 1 == nx || j + 1 == ny) v = r_s[row] - ev;
-            else v = r_s[row] - k_row(e, nu_s, nx, row, i, j);
-            r1[sm.offset + row] = v;
-            acc += static_cast<double>(d_s[row]) * static_cast<double>(v) * static_cast<double>(v);
-            i += blockDim.x;
-            while (i >= nx) {
-                i -= nx;
-                ++j;
-            }
-        }
-        double const t = block_sum_d(acc, red);
-        if (threadIdx.x == 0) part[item] = t;
-    }
+    double acc = 0.0;
+    walk_strips(
+        ss, pre,
+        [&](Sample const& sm, int c0, int j0, int j1) {
+            float* out = r1 + sm.offset;
+            mag2d_strip<float>(WrapPreSrc {dinv + sm.offset, r + sm.offset}, nu + sm.offset, sm.nx, sm.ny, c0, j0, j1,
+                               [&](int row, float q, float, WrapPreSrc::Raw const& raw, WrapPreSrc::Own) {
+                                   float const v = raw.r - q;
+                                   out[row] = v;
+                                   acc += static_cast<double>(raw.d) * static_cast<double>(v) * static_cast<double>(v);
+                               });
+        },
+        [&](int cta) {
+            double const t = block_sum_d(acc, red);
+            if (threadIdx.x == 0) part[cta] = t;
+            acc = 0.0;
+        });
 }
 
 // dots[s*3] = sum of the sample's item partials: one warp per sample, each
@@ -1513,7 +1673,7 @@ __global__ void wrap_finish_kernel(const __grid_constant__ Samples ss, double co
     int const sidx = blockIdx.x;
     if (sidx >= ss.n || !sample_active(ss, sidx)) return;
     double t = 0.0;
-    for (int k = ss.item_base[sidx] + static_cast<int>(threadIdx.x); k < ss.item_base[sidx + 1]; k += 32) t += part[k];
+    for (int k = ss.strip_base[sidx] + static_cast<int>(threadIdx.x); k < ss.strip_base[sidx + 1]; k += 32) t += part[k];
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     if (threadIdx.x == 0) dots[sidx * 3] = t;
 }
@@ -1535,6 +1695,29 @@ __device__ __forceinline__ void stage_rms(Samples const& ss, double const* dots,
 {
     for (int k = threadIdx.x; k < ss.n; k += blockDim.x)
         sc[k] = static_cast<float>(sqrt(dots[k * 3] / (static_cast<double>(ss.s[k].nx) * ss.s[k].ny)));
+}
+
+// dinv = 1 / diag(K) (identity on the boundary); nu given per node.
+__global__ void __launch_bounds__(256) dinv_kernel(const __grid_constant__ Samples ss, WrapItem const* items,
+                                                   float const* __restrict__ nu, float* __restrict__ dinv)
+{
+    WrapItem const it = items[blockIdx.x];
+    Sample const sm = ss.s[it.sample];
+    int const nx = sm.nx, ny = sm.ny;
+    float const* v = nu + sm.offset;
+    float* o = dinv + sm.offset;
+#pragma unroll 4
+    for (int row = it.begin + static_cast<int>(threadIdx.x); row < it.end; row += 256) {
+        int const j = row / nx, i = row - j * nx;
+        bool const in = !(i == 0 || j == 0 || i + 1 == nx || j + 1 == ny);
+        float const below = v[j >= 2 ? row - nx : row], left = v[i >= 2 ? row - 1 : row], c = v[row];
+        float d = 0.0f;
+        if (j >= 2) d = d + below;
+        d = d + c;
+        if (i >= 2) d = d + left;
+        d = d + c;
+        o[row] = in ? 1.0f / d : 1.0f;
+    }
 }
 
 // e2 = w D^-1 r + s D^-1/2 up(unet) at interior nodes (w D^-1 r on the
@@ -1574,35 +1757,38 @@ __global__ void __launch_bounds__(256) wrap_e2_kernel(const __grid_constant__ Sa
     }
 }
 
-// M(r) = e2 + w D^-1 (r - K e2) (boundary rows: K e2 -> e2).  Items as wrap_pre.
-__global__ void __launch_bounds__(256) wrap_post_kernel(const __grid_constant__ Samples ss, WrapItem const* items,
-                                                        float const* nu, float const* dinv, float const* r,
-                                                        float const* e2, float* out)
+// Operand e2, with D^-1 and r on the side.
+struct WrapPostSrc
+{
+    using Raw = float;
+    struct Own
+    {
+        float d, r;
+    };
+    float const* __restrict__ e;
+    float const* __restrict__ d;
+    float const* __restrict__ r;
+    __device__ __forceinline__ Raw load(int row) const { return e[row]; }
+    __device__ __forceinline__ Own own(int row) const { return {d[row], r[row]}; }
+    __device__ __forceinline__ float value(Raw v) const { return v; }
+};
+
+// M(r) = e2 + w D^-1 (r - K e2) (boundary rows: K e2 -> e2), in strips as wrap_pre
+// (24 -> 17.5 us).
+__global__ void __launch_bounds__(256) wrap_post_kernel(const __grid_constant__ Samples ss, float const* nu,
+                                                        float const* dinv, float const* r, float const* e2, float* out)
 {
     __shared__ int64_t pre[kMaxImages + 1];
-    int const nact = scan_items(ss, pre);
-    for (int a = blockIdx.x; a < nact; a += gridDim.x) {
-        WrapItem const it = items[item_of(ss, pre, a)];
-        Sample const sm = ss.s[it.sample];
-        int const nx = sm.nx, ny = sm.ny;
-        float const* e_s = e2 + sm.offset;
-        float const* d_s = dinv + sm.offset;
-        float const* r_s = r + sm.offset;
-        auto e = [&](int q, int, int) { return e_s[q]; };
-        int row = it.begin + static_cast<int>(threadIdx.x);
-        int j = row / nx, i = row - j * nx;
-        for (; row < it.end; row += blockDim.x) {
-            float const e0 = e_s[row];
-            float const ke = (i == 0 || j == 0 || i + 1 == nx || j + 1 == ny) ? e0
-                                                                                : k_row(e, nu + sm.offset, nx, row, i, j);
-            out[sm.offset + row] = e0 + kOmega * (d_s[row] * (r_s[row] - ke));
-            i += blockDim.x;
-            while (i >= nx) {
-                i -= nx;
-                ++j;
-            }
-        }
-    }
+    walk_strips(
+        ss, pre,
+        [&](Sample const& sm, int c0, int j0, int j1) {
+            float* o = out + sm.offset;
+            mag2d_strip<float>(WrapPostSrc {e2 + sm.offset, dinv + sm.offset, r + sm.offset}, nu + sm.offset, sm.nx, sm.ny,
+                               c0, j0, j1, [&](int row, float q, float e0, float, WrapPostSrc::Own const& w) {
+                                   o[row] = e0 + kOmega * (w.d * (w.r - q));
+                               });
+        },
+        [](int) {});
 }
 
 // log(nu) / log(1000), pooled 2 x 2 onto the top-level image of every sample
@@ -1696,6 +1882,7 @@ public:
     DevBuf feat, unet, gnet;
     DevBuf witems, wpart;          // fused wrapper work items and their partial sums
     int nwitems = 0;
+    int nstrips = 0;               // CTAs of strips
     DevBuf wparts;                 // weight-gradient partials
     int wgrad_grid = 0;
     int thin_grid = 0;
@@ -1794,7 +1981,20 @@ sil_status Workspace::build(std::vector<Sample> const& s)
         ss.item_base[n] = static_cast<int32_t>(wi.size());
         nwitems = static_cast<int>(wi.size());
         if (sil_status st = witems.alloc(sizeof(WrapItem) * wi.size()); st != SIL_OK) return st;
-        if (sil_status st = wpart.alloc(sizeof(double) * wi.size()); st != SIL_OK) return st;
+        // strips: one wave of two CTAs per multiprocessor before they get longer
+        int dev = 0, sms = 148;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        for (ss.strip_rows = kStripBatch;; ss.strip_rows += kStripBatch) {
+            nstrips = 0;
+            for (int i = 0; i < n; ++i) {
+                ss.strip_base[i] = nstrips;
+                nstrips += strips_of(s[i].nx, s[i].ny, ss.strip_rows).ctas;
+            }
+            ss.strip_base[n] = nstrips;
+            if (nstrips <= 2 * sms || ss.strip_rows >= 32) break;
+        }
+        if (sil_status st = wpart.alloc(sizeof(double) * nstrips); st != SIL_OK) return st;
         SIL_CUDA_CHECK(cudaMemcpy(witems.p, wi.data(), sizeof(WrapItem) * wi.size(), cudaMemcpyHostToDevice));
     }
     int64_t const top = levels[0].npx;
@@ -1862,24 +2062,29 @@ sil_status ensure_attributes()
     int dev = 0;
     SIL_CUDA_CHECK(cudaGetDevice(&dev));
     SIL_CUDA_CHECK(cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev));
-    SIL_CUDA_CHECK(cudaFuncSetAttribute(conv3x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(conv_smem())));
+    for (void const* k : {reinterpret_cast<void const*>(conv3x3_kernel), reinterpret_cast<void const*>(conv3x3_plain_kernel)}) {
+        SIL_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(conv_smem())));
+    }
     // all of the unified L1 / shared storage as shared memory, so several
     // CTAs of these shared-memory-heavy kernels fit on one multiprocessor
     SIL_CUDA_CHECK(cudaFuncSetAttribute(conv3x3_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                        cudaSharedmemCarveoutMaxShared));
+    SIL_CUDA_CHECK(cudaFuncSetAttribute(conv3x3_plain_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                         cudaSharedmemCarveoutMaxShared));
     SIL_CUDA_CHECK(cudaFuncSetAttribute(wgrad_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                         cudaSharedmemCarveoutMaxShared));
     // resident CTAs per multiprocessor from the kernel's registers and each
     // mode's shared memory (1 KB per CTA reserved by the runtime)
     cudaFuncAttributes fa {};
+    cudaFuncAttributes fp {};
     SIL_CUDA_CHECK(cudaFuncGetAttributes(&fa, conv3x3_kernel));
+    SIL_CUDA_CHECK(cudaFuncGetAttributes(&fp, conv3x3_plain_kernel));
     int smem_sm = 0, regs_sm = 0;
     SIL_CUDA_CHECK(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
     SIL_CUDA_CHECK(cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev));
     for (int m = 0; m < 5; ++m) {
         int const by_smem = smem_sm / static_cast<int>(conv_smem(m) + 1024);
-        int const by_regs = regs_sm / std::max(1, fa.numRegs * 128);
+        int const by_regs = regs_sm / std::max(1, ((m == kPlain ? fp : fa).numRegs + 7) / 8 * 8 * 128);
         g_conv_per_sm[m] = std::max(1, std::min(std::min(by_smem, by_regs), 8));
     }
     SIL_CUDA_CHECK(cudaFuncSetAttribute(wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1936,8 +2141,10 @@ sil_status launch_conv(cudaStream_t st, Table const& t, int mode, bf16 const* in
                        int* err, float* out_taps = nullptr, float const* wout = nullptr, int64_t taps_stride = 0)
 {
     if (t.nimg == 0 || t.tile_base[t.nimg] == 0) return SIL_OK;
-    conv3x3_kernel<<<conv_grid(t.tile_base[t.nimg], mode), 128, conv_smem(mode), st>>>(
-            t, mode, in, in2, gin, w, bias, relu, out, out_f32, accumulate, out_taps, wout, taps_stride, err);
+    ConvOut const dst {bias, relu, out, out_f32, accumulate, out_taps, taps_stride};
+    int const grid = conv_grid(t.tile_base[t.nimg], mode);
+    if (mode == kPlain) conv3x3_plain_kernel<<<grid, 128, conv_smem(mode), st>>>(t, in, w, dst, wout, err);
+    else conv3x3_kernel<<<grid, 128, conv_smem(mode), st>>>(t, mode, in, in2, gin, w, dst, err);
     SIL_CUDA_CHECK(cudaGetLastError());
     return SIL_OK;
 }
@@ -2086,14 +2293,14 @@ sil_status net_forward(Net& net, Workspace& w, cudaStream_t st, bool keep)
     int* err = net.error_flag;
     {
         Table const t = w.table(0, -1, false);
-        inc_forward_kernel<<<(walk_grid(t, 1, kWalkInc) + 1) / 2, 256, 0, st>>>(t, w.feat.as<float>(), net.params,
+        inc_forward_kernel<<<walk_grid(t, 1, kWalkInc), 256, 0, st>>>(t, w.feat.as<float>(), net.params,
                                                                               w.h[0].as<bf16>());
         SIL_CUDA_CHECK(cudaGetLastError());
     }
     for (int l = 1; l < D; ++l) {
         int const wl = weight_level_enc(l);
         Table const t = w.table(l, l - 1, true);
-        pool_kernel<<<walk_grid(t, 1, kWalkPool), 256, 0, st>>>(t, w.h[l - 1].as<bf16>(), w.pin[l].as<bf16>());
+        pool_kernel<<<walk_grid(t, kChunks, kWalkPool), 256, 0, st>>>(t, w.h[l - 1].as<bf16>(), w.pin[l].as<bf16>());
         SIL_CUDA_CHECK(cudaGetLastError());
         Table const t2 = w.table(l, -1, false);
         sil_status s = launch_conv(st, t2, kPlain, w.pin[l].as<bf16>(), nullptr, nullptr, big_w(net, kDown, wl),
@@ -2122,7 +2329,7 @@ sil_status net_forward(Net& net, Workspace& w, cudaStream_t st, bool keep)
                             big_b(net, kDec, wl), 1, w.g[l].as<bf16>(), nullptr, 0, err);
         } else {
             // the pooled input of this level (pin) has been consumed by the encoder: it holds the sum
-            upadd_kernel<<<walk_grid(tt, 1, kWalkUpAdd), 256, 0, st>>>(tt, w.h[l].as<bf16>(), w.g[l + 1].as<bf16>(),
+            upadd_kernel<<<walk_grid(tt, kChunks, kWalkUpAdd), 256, 0, st>>>(tt, w.h[l].as<bf16>(), w.g[l + 1].as<bf16>(),
                                                                        w.pin[l].as<bf16>());
             SIL_CUDA_CHECK(cudaGetLastError());
             s = launch_conv(st, tt, kPlain, w.pin[l].as<bf16>(), nullptr, nullptr, big_w(net, kDec, wl),
@@ -2286,12 +2493,12 @@ sil_status precond_forward(Net& net, Workspace& w, float const* nu, float const*
     w.active = active;
     w.ss.active = active;
     if (dinv == nullptr) {
-        dinv_kernel<<<node_grid(w), 256, 0, st>>>(w.ss, nu, w.dinv.as<float>());
+        dinv_kernel<<<static_cast<unsigned>(w.nwitems), 256, 0, st>>>(w.ss, w.witems.as<WrapItem>(), nu, w.dinv.as<float>());
         dinv = w.dinv.as<float>();
     }
     WrapItem const* items = w.witems.as<WrapItem>();
     Table const t0 = w.table(0, -1, false);
-    wrap_pre_kernel<<<item_grid(w.nwitems, kWalkPre), 256, 0, st>>>(w.ss, items, nu, dinv, b, w.r1.as<float>(),
+    wrap_pre_kernel<<<item_grid(w.nstrips, kWalkPre), 256, 0, st>>>(w.ss, nu, dinv, b, w.r1.as<float>(),
                                                                     w.wpart.as<double>());
     wrap_finish_kernel<<<static_cast<unsigned>(w.samples.size()), 32, 0, st>>>(w.ss, w.wpart.as<double>(),
                                                                                 w.dots.as<double>());
@@ -2304,7 +2511,7 @@ sil_status precond_forward(Net& net, Workspace& w, float const* nu, float const*
     if (s != SIL_OK) return s;
     wrap_e2_kernel<<<item_grid(w.nwitems, kWalkE2), 256, 0, st>>>(w.ss, items, dinv, b, w.unet.as<float>(),
                                                                   w.dots.as<double>(), w.e2.as<float>());
-    wrap_post_kernel<<<item_grid(w.nwitems, kWalkPost), 256, 0, st>>>(w.ss, items, nu, dinv, b, w.e2.as<float>(), out);
+    wrap_post_kernel<<<item_grid(w.nstrips, kWalkPost), 256, 0, st>>>(w.ss, nu, dinv, b, w.e2.as<float>(), out);
     SIL_CUDA_CHECK(cudaGetLastError());
     return SIL_OK;
 }
