@@ -1214,6 +1214,49 @@ __global__ void __launch_bounds__(kThreads) fcg_init_kernel(Item const* items, i
     }
 }
 
+// Sums over a problem's CTAs of the K values each thread holds.  A CTA's sums go
+// to parts[k * stride + index]; the last of the problem's n CTAs to count in
+// adds the partials, a warp per value, in a fixed order, and returns true in
+// thread 0 with the totals in `out` (shared).  (With a block-wide sum per value
+// at both ends the eight of fcg_orth_kernel took half of its 33 us.)
+template <int K>
+__device__ __forceinline__ bool fcg_sums(double (&v)[K], double* parts, int64_t stride, int index, int n, int* counter,
+                                         double (&red)[K][kThreads / 32], double (&out)[K])
+{
+    __shared__ int is_last;
+    int const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+        if (lane == 0) red[k][warp] = v[k];
+    }
+    __syncthreads();
+    if (warp == 0) {
+        if (lane < K) {
+            double t = 0.0;
+            for (int w = 0; w < kThreads / 32; ++w) t += red[lane][w];
+            __stcg(parts + lane * stride + index, t);
+            __threadfence();
+        }
+        __syncwarp();
+        if (lane == 0) is_last = atomicAdd(counter, 1) == n - 1;
+    }
+    __syncthreads();
+    if (!is_last) return false;
+    __threadfence();
+    for (int k = warp; k < K; k += kThreads / 32) {
+        double t = 0.0;
+#pragma unroll 4
+        for (int j = lane; j < n; j += 32) t += __ldcg(parts + k * stride + j);
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) out[k] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return false;
+    *counter = 0;
+    return true;
+}
+
 // Partials z.q_j over the stored directions (the first min(iters, m)); the
 // last CTA forms coef_j = (z.q_j)/(p_j.q_j).  M >= m is the compile-time bound.
 template <class T, int M>
@@ -1221,8 +1264,8 @@ __global__ void __launch_bounds__(kThreads) fcg_orth_kernel(Item const* items, i
                                                             Vecs<T> const* vecs, Scalars* sc, double* parts_base,
                                                             int64_t hstride, int m, int nitems_all)
 {
-    __shared__ double red[kThreads / 32];
-    __shared__ double vals[M];
+    __shared__ double red[M][kThreads / 32];
+    __shared__ double tot[M];
     Item const it = items[act != nullptr ? act[blockIdx.x] : blockIdx.x];
     Scalars* s = sc + it.prob;
     if (s->done || s->outer_done || s->fallback) return;
@@ -1230,26 +1273,20 @@ __global__ void __launch_bounds__(kThreads) fcg_orth_kernel(Item const* items, i
     Vecs<T> const v = vecs[it.prob];
     int const nvalid = min(s->iters, m);
     if (nvalid == 0) return;
+    T const* __restrict__ z = v.z;
+    T const* __restrict__ qh = v.qh;
+    int const end = static_cast<int>(it.end);
     double acc[M];
 #pragma unroll
     for (int j = 0; j < M; ++j) acc[j] = 0.0;
-    for (int64_t row = it.begin + threadIdx.x; row < it.end; row += kThreads) {
-        double const z = static_cast<double>(v.z[row]);
+#pragma unroll 2
+    for (int row = static_cast<int>(it.begin) + threadIdx.x; row < end; row += kThreads) {
+        double const zr = static_cast<double>(z[row]);
 #pragma unroll
         for (int j = 0; j < M; ++j)
-            if (j < nvalid) acc[j] += z * static_cast<double>(fcg_slot(v.qh, hstride, j)[row]);
+            if (j < nvalid) acc[j] += zr * static_cast<double>(qh[j * hstride + row]);
     }
-#pragma unroll
-    for (int j = 0; j < M; ++j) {
-        double const t = block_sum(acc[j], red);
-        if (threadIdx.x == 0) vals[j] = t;
-    }
-    __syncthreads();
-    double* parts[M];
-#pragma unroll
-    for (int j = 0; j < M; ++j) parts[j] = parts_base + static_cast<int64_t>(j) * nitems_all;  // one slot per item of the batch
-    double tot[M];
-    if (finish_reduction_k<M>(vals, parts, it.index, pi.first_item, pi.nitems, &s->counter_a, tot)) {
+    if (fcg_sums<M>(acc, parts_base + pi.first_item, nitems_all, it.index, pi.nitems, &s->counter_a, red, tot)) {
         for (int j = 0; j < nvalid; ++j) {
             s->coef[j] = tot[j] / s->pq_hist[j];
             if (!isfinite(s->coef[j])) s->nonfinite = 1;
@@ -1273,80 +1310,108 @@ __global__ void __launch_bounds__(kThreads) fcg_direction_kernel(Item const* ite
     T c[M];
 #pragma unroll
     for (int j = 0; j < M; ++j) c[j] = j < nvalid ? static_cast<T>(s->coef[j]) : T(0);
-    T* const out = fcg_slot(v.ph, hstride, slot);
-    for (int64_t row = it.begin + threadIdx.x; row < it.end; row += kThreads) {
-        T p = v.z[row];
+    T const* __restrict__ z = v.z;
+    T* ph = v.ph;
+    int const end = static_cast<int>(it.end);
+    // the rows' loads go out in batches: a row's store may not wait for the next row's loads
+    constexpr int U = M > 8 ? 1 : 2;
+    for (int row = static_cast<int>(it.begin) + threadIdx.x; row < end; row += U * kThreads) {
+        T p[U], h[U][M];
 #pragma unroll
-        for (int j = 0; j < M; ++j)
-            if (j < nvalid) p -= c[j] * fcg_slot(v.ph, hstride, j)[row];
-        out[row] = p;
+        for (int u = 0; u < U; ++u) {
+            int const at = min(row + u * kThreads, end - 1);
+            p[u] = z[at];
+#pragma unroll
+            for (int j = 0; j < M; ++j) h[u][j] = j < nvalid ? ph[j * hstride + at] : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+#pragma unroll
+            for (int j = 0; j < M; ++j)
+                if (j < nvalid) p[u] -= c[j] * h[u][j];
+            if (row + u * kThreads < end) ph[slot * hstride + row + u * kThreads] = p[u];
+        }
     }
 }
 
-// q_slot = A p_slot, partials p.q and p.r; the last CTA stores p.q for the
-// slot and forms alpha.
+// The direction p_slot as a strip's operand, r on the side.
 template <class T>
-__global__ void __launch_bounds__(kThreads) fcg_apply_kernel(Item const* items, int const* act, ProbInfo const* info,
-                                                             Vecs<T> const* vecs, Scalars* sc, double* part_a,
-                                                             double* part_b, int64_t hstride, int m)
+struct StripSlot
 {
-    __shared__ double red[kThreads / 32];
-    Item const it = items[act != nullptr ? act[blockIdx.x] : blockIdx.x];
-    Scalars* s = sc + it.prob;
+    using Raw = T;
+    using Own = T;
+    T const* __restrict__ p;
+    T const* __restrict__ r;
+    __device__ __forceinline__ Raw load(int row) const { return p[row]; }
+    __device__ __forceinline__ Own own(int row) const { return r[row]; }
+    __device__ __forceinline__ T value(Raw v) const { return v; }
+};
+
+// q_slot = A p_slot in strips, partials p.q and p.r; the last CTA stores p.q
+// for the slot and forms alpha.
+template <class T>
+__global__ void __launch_bounds__(kThreads) fcg_apply_kernel(StripWork<T> const* work, Vecs<T> const* vecs, int64_t hstride,
+                                                             int m, int64_t part_stride)
+{
+    __shared__ double red[2][kThreads / 32];
+    __shared__ double tot[2];
+    StripWork<T> const w = work[blockIdx.x];
+    Scalars* s = w.s;
     if (s->done || s->outer_done || s->fallback) return;
-    ProbInfo const pi = info[it.prob];
-    Vecs<T> const v = vecs[it.prob];
+    Vecs<T> const v = vecs[w.prob];
     int const slot = s->iters % m;
-    T const* const p = fcg_slot(v.ph, hstride, slot);
-    T* const qo = fcg_slot(v.qh, hstride, slot);
-    double pq = 0.0, pr = 0.0;
-    for (int64_t row = it.begin + threadIdx.x; row < it.end; row += kThreads) {
-        T const q = mag_apply_row(p, v.nu, pi, row);
-        qo[row] = q;
-        double const pv = static_cast<double>(p[row]);
-        pq += pv * static_cast<double>(q);
-        pr += pv * static_cast<double>(v.r[row]);
+    T* __restrict__ q = v.qh + slot * hstride;
+    double sums[2] = {0.0, 0.0};
+    int const strip = w.first + static_cast<int>(threadIdx.x) / 32;
+    if (strip < w.count) {
+        int const block = strip / w.strips, j0 = block * w.rows;
+        mag2d_strip<T>(StripSlot<T> {v.ph + slot * hstride, v.r}, w.nu, w.nx, w.ny, (strip - block * w.strips) * kStripCols,
+                       j0, min(w.ny, j0 + w.rows), [&](int row, T qr, T p, T, T r) {
+                           q[row] = qr;
+                           sums[0] += static_cast<double>(p) * static_cast<double>(qr);
+                           sums[1] += static_cast<double>(p) * static_cast<double>(r);
+                       });
     }
-    double const pq_b = block_sum(pq, red);
-    double const pr_b = block_sum(pr, red);
-    double const vals[2] = {pq_b, pr_b};
-    double* parts[2] = {part_a, part_b};
-    double tot[2];
-    if (finish_reduction_k<2>(vals, parts, it.index, pi.first_item, pi.nitems, &s->counter_a, tot)) {
-        double const tpq = tot[0], tot_pr = tot[1];
-        s->pq_hist[slot] = tpq;
-        s->alpha = tot_pr / tpq;
+    int const ctas = (w.count + kThreads / 32 - 1) / (kThreads / 32);
+    if (fcg_sums<2>(sums, w.part_pq, part_stride, w.index, ctas, &s->counter_a, red, tot)) {
+        s->pq_hist[slot] = tot[0];
+        s->alpha = tot[1] / tot[0];
         if (!isfinite(s->alpha)) s->nonfinite = 1;
     }
 }
 
 // x += alpha p_slot, r -= alpha q_slot, partial r.r; the last CTA advances
-// the iteration (and so the slot) and checks convergence and the stall window.
+// the iteration (and so the slot), checks convergence and the stall window, and
+// switches the problem off for the network (`active`) once it stops.
 template <class T>
 __global__ void __launch_bounds__(kThreads) fcg_update_kernel(Item const* items, int const* act, ProbInfo const* info,
                                                               Vecs<T> const* vecs, Scalars* sc, double* part,
-                                                              int window, int64_t hstride, int m)
+                                                              int window, int64_t hstride, int m, int* active)
 {
-    __shared__ double red[kThreads / 32];
+    __shared__ double red[1][kThreads / 32];
+    __shared__ double total[1];
     Item const it = items[act != nullptr ? act[blockIdx.x] : blockIdx.x];
     Scalars* s = sc + it.prob;
     if (s->done || s->outer_done || s->fallback) return;
     ProbInfo const pi = info[it.prob];
     Vecs<T> const v = vecs[it.prob];
     int const slot = s->iters % m;
-    T const* const p = fcg_slot(v.ph, hstride, slot);
-    T const* const q = fcg_slot(v.qh, hstride, slot);
+    T const* __restrict__ p = v.ph + slot * hstride;
+    T const* __restrict__ q = v.qh + slot * hstride;
+    T* __restrict__ rv = v.r;
+    T* __restrict__ xv = v.x;
     T const alpha = static_cast<T>(s->alpha);
-    double rr = 0.0;
-    for (int64_t row = it.begin + threadIdx.x; row < it.end; row += kThreads) {
-        T const r = v.r[row] - alpha * q[row];
-        v.x[row] = v.x[row] + alpha * p[row];
-        v.r[row] = r;
-        rr += static_cast<double>(r) * static_cast<double>(r);
+    int const end = static_cast<int>(it.end);
+    double rr[1] = {0.0};
+#pragma unroll 4
+    for (int row = static_cast<int>(it.begin) + threadIdx.x; row < end; row += kThreads) {
+        T const r = rv[row] - alpha * q[row];
+        xv[row] = xv[row] + alpha * p[row];
+        rv[row] = r;
+        rr[0] += static_cast<double>(r) * static_cast<double>(r);
     }
-    double const rr_b = block_sum(rr, red);
-    double tot = 0.0;
-    if (finish_reduction(rr_b, part, it.index, pi.first_item, pi.nitems, &s->counter_c, &tot)) {
+    if (fcg_sums<1>(rr, part + pi.first_item, 0, it.index, pi.nitems, &s->counter_c, red, total)) {
+        double const tot = total[0];
         s->rr = tot;
         s->iters += 1;
         s->total_iters += 1;
@@ -1361,6 +1426,7 @@ __global__ void __launch_bounds__(kThreads) fcg_update_kernel(Item const* items,
             s->win_rr = tot;
             s->win_iters = 0;
         }
+        if (s->done) active[it.prob] = 0;
     }
 }
 
@@ -2392,6 +2458,20 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
         for (int i = 0; i < ntiles; ++i)
             if (!hs[tiles[i].prob].outer_done) open_tiles.push_back(i);
     };
+    // The strips of the open problems of a 2D batch.
+    auto build_strips = [&](std::vector<char> const& open) {
+        swork.clear();
+        for (int p = 0; flat && p < np; ++p) {
+            if (!open[p]) continue;
+            ProbInfo const& pi = info[p];
+            Vecs<T> const& v = vecs[p];
+            Strips const st = strips_of(pi.nx, pi.ny, srows);
+            for (int k = 0; k < st.ctas; ++k)
+                swork.push_back({v.x, v.z, v.p, v.p2, v.q, v.nu, d_sc + p, part_a + strip_part[p], part_b + pi.first_item,
+                                 part_c + pi.first_item, static_cast<int>(pi.nx), static_cast<int>(pi.ny), st.strips,
+                                 st.rows, st.count, k * kStripWarps, k, p, pi.nitems, pi.max_iters});
+        }
+    };
     auto capture_chunk = [&]() -> sil_status {
         if (exec != nullptr) cudaGraphExecDestroy(exec);
         if (graph != nullptr) cudaGraphDestroy(graph);
@@ -2410,17 +2490,9 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
                             static_cast<int>(it.end), it.index, pi.nitems,
                             march ? pi.ntiles : (flat ? strips_of(pi.nx, pi.ny, srows).ctas : pi.nitems), pi.max_iters});
         }
-        swork.clear();
-        for (int p = 0; flat && p < np; ++p) {
-            if (hs[p].outer_done || resident[p]) continue;
-            ProbInfo const& pi = info[p];
-            Vecs<T> const& v = vecs[p];
-            Strips const st = strips_of(pi.nx, pi.ny, srows);
-            for (int k = 0; k < st.ctas; ++k)
-                swork.push_back({v.x, v.z, v.p, v.p2, v.q, v.nu, d_sc + p, part_a + strip_part[p], part_b + pi.first_item,
-                                 part_c + pi.first_item, static_cast<int>(pi.nx), static_cast<int>(pi.ny), st.strips,
-                                 st.rows, st.count, k * (kThreads / 32), k, p, pi.nitems, pi.max_iters});
-        }
+        std::vector<char> open(np, 0);
+        for (int i : open_host) open[items[i].prob] = 1;
+        build_strips(open);
         int const ns = static_cast<int>(swork.size());
         if (ns > 0)
             SIL_CUDA_CHECK(cudaMemcpyAsync(d_strips, swork.data(), sizeof(StripWork<T>) * ns, cudaMemcpyHostToDevice,
@@ -2542,17 +2614,21 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
                 lexec = nullptr;
                 lgraph = nullptr;
                 ln = static_cast<int>(lopen.size());
+                std::vector<char> open(np, 0);
+                for (int i : lopen) open[items[i].prob] = 1;
+                build_strips(open);
+                int const lstrips = static_cast<int>(swork.size());
+                SIL_CUDA_CHECK(cudaMemcpyAsync(d_strips, swork.data(), sizeof(StripWork<T>) * lstrips,
+                                               cudaMemcpyHostToDevice, stream));
                 SIL_CUDA_CHECK(cudaMemcpyAsync(d_act, lopen.data(), sizeof(int) * ln, cudaMemcpyHostToDevice, stream));
                 cudaStream_t cs;
                 SIL_CUDA_CHECK(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
                 sil_status cst = SIL_OK;
                 cudaError_t err = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
                 for (int c = 0; c < lchunk && err == cudaSuccess && cst == SIL_OK; ++c) {
-                    fcg_apply_kernel<T><<<ln, kThreads, 0, cs>>>(d_items, d_act, d_info, d_vecs, d_sc, part_a, part_b,
-                                                                 hstride, fdirs);
+                    fcg_apply_kernel<T><<<lstrips, kThreads, 0, cs>>>(d_strips, d_vecs, hstride, fdirs, part_b - part_a);
                     fcg_update_kernel<T><<<ln, kThreads, 0, cs>>>(d_items, d_act, d_info, d_vecs, d_sc, part_c, window,
-                                                                  hstride, fdirs);
-                    fcg_active_kernel<<<(np + 63) / 64, 64, 0, cs>>>(d_sc, np, d_active);
+                                                                  hstride, fdirs, d_active);
                     cst = net->forward(ws, nuf, dv, rv, zv, cs, d_active);
                     new_direction(cs);
                 }
