@@ -15,10 +15,6 @@
 // from global memory each load touches six 128-byte lines).  The moments and
 // sums are those of mag3d_curl_rows in the same order, so the values are the
 // same.
-//
-// In the direction form the operand is p = z + beta p_old, formed once per
-// element between the copies and the ring (halo elements by each tile that
-// reads them), with p and the pending x += alpha p_old written by the owner.
 #pragma once
 
 #include <cstdint>
@@ -60,49 +56,24 @@ constexpr int kMarchWarps = 8;
 constexpr int kMarchThreads = kMarchX * kMarchWarps;
 constexpr int kMarchOwnRows = kMarchWarps - 1;   // owned columns along y
 
-// Operand sources.  MarchPlain: the array itself.  MarchDirection: the new
-// search direction z + beta p_old; p_new receives it and, when `pending`, x
-// gets the previous iteration's alpha p_old.
 template <class T>
-struct MarchPlain
-{
-    static constexpr int kFields = 0;
-    T const* a;
-    __device__ __forceinline__ T at(int row) const { return a[row]; }
-};
-template <class T>
-struct MarchDirection
-{
-    static constexpr int kFields = 3;
-    T const* z;
-    T const* pold;
-    T* pnew;
-    T* x;
-    T alpha, beta;
-    bool pending;
-    __device__ __forceinline__ T at(int row) const { return z[row] + beta * pold[row]; }
-};
-
-template <class T, class Src>
 struct MarchSmem
 {
     static constexpr int kElems = (kMarchWarps + 1) * kMarchNodes * 3;
     T a[kMarchRing * kElems];             // operand planes, [slot][row][node][component]
     T h[2 * 2 * kMarchThreads];           // H_x and H_z of the current plane, double-buffered
-    T raw[Src::kFields ? Src::kFields : 1][Src::kFields ? kElems : 1];   // a plane's copied fields
 };
 
 // One run of planes [k0, k1) of the tile whose first owned column is (i0, j0):
-// out(row, q, p) takes a result and its operand.  Rows are below 2^31.  EDGE:
+// out(row, q, a) takes a result and its operand.  Rows are below 2^31.  EDGE:
 // the tile touches the grid's boundary columns, so columns and elements are
 // tested; the others test planes only.
-template <bool EDGE, class T, class Src, class Out>
-__device__ __forceinline__ void mag3d_march_tile(MarchSmem<T, Src>& sm, Grid3<T> const& g, T const* __restrict__ nu,
-                                                 Src const& src, int i0, int j0, int k0, int k1, Out const& out)
+template <bool EDGE, class T, class Out>
+__device__ __forceinline__ void mag3d_march_tile(MarchSmem<T>& sm, Grid3<T> const& g, T const* __restrict__ nu,
+                                                 T const* __restrict__ a, int i0, int j0, int k0, int k1, Out const& out)
 {
-    constexpr bool kDirect = Src::kFields == 0;
     constexpr int kRow = kMarchNodes * 3;
-    constexpr int kElems = MarchSmem<T, Src>::kElems;
+    constexpr int kElems = MarchSmem<T>::kElems;
     constexpr int kFull = kElems / kMarchThreads;     // slots every thread fills
     constexpr int kSlots = kFull + (kElems % kMarchThreads != 0);
     int const tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
@@ -110,69 +81,30 @@ __device__ __forceinline__ void mag3d_march_tile(MarchSmem<T, Src>& sm, Grid3<T>
     int const nodes2 = g.nx * g.ny, plane = 3 * nodes2;
     bool const tail = tid < kElems % kMarchThreads;   // fills the last, partial slot
 
-    // the elements this thread stages: row offset in a plane, and whether it
-    // lies in the grid, is an interior (nonzero) and an owned one
+    // the elements this thread stages: row offset in a plane, and whether it is
+    // an interior one (the others are zero)
     int off[kSlots];
-    unsigned grid = 0, inner = 0, owned = 0;
+    unsigned inner = 0;
 #pragma unroll
     for (int s = 0; s < kSlots; ++s) {
         int const e = min(tid + s * kMarchThreads, kElems - 1), r = e / kRow, c = e - r * kRow;
         int const ii = i0 - 1 + c / 3, jj = j0 - 1 + r;
-        bool const in = !EDGE || (ii >= 0 && jj >= 0 && ii < g.nx && jj < g.ny);
         bool const deep = !EDGE || (ii > 0 && jj > 0 && ii + 1 < g.nx && jj + 1 < g.ny);
-        off[s] = (kDirect ? deep : in) ? 3 * (ii + g.nx * jj) + c % 3 : 0;
-        if (in) grid |= 1u << s;
+        off[s] = deep ? 3 * (ii + g.nx * jj) + c % 3 : 0;
         if (deep) inner |= 1u << s;
-        if (in && ii >= i0 && jj >= j0 && ii < i0 + kMarchCols && jj < j0 + kMarchOwnRows) owned |= 1u << s;
     }
-    auto for_slots = [&](auto const& f) {
-#pragma unroll
-        for (int s = 0; s < kSlots; ++s)
-            if (s < kFull || tail) f(s, tid + s * kMarchThreads);
-    };
-    // Copies of plane k: into its ring slot (plain; `to` its first element), or
-    // of its fields.
+    // Copies of plane k into the ring slot whose first element is `to`.
     auto fetch = [&](int k, int to) {
-        if constexpr (kDirect) {
-            if (k <= k1) {
-                bool const deep = k > 0 && k + 1 < g.nz;
-                T const* from = src.a + static_cast<int64_t>(plane) * (deep ? k : 0);
-                for_slots([&](int s, int e) {
-                    march_copy(&sm.a[to + e], from + off[s],
+        if (k <= k1) {
+            bool const deep = k > 0 && k + 1 < g.nz;
+            T const* from = a + static_cast<int64_t>(plane) * (deep ? k : 0);
+#pragma unroll
+            for (int s = 0; s < kSlots; ++s)
+                if (s < kFull || tail)
+                    march_copy(&sm.a[to + tid + s * kMarchThreads], from + off[s],
                                deep && (!EDGE || ((inner >> s) & 1u)) ? static_cast<int>(sizeof(T)) : 0);
-                });
-            }
-        } else if (k >= 0 && k <= k1 && k < g.nz) {
-            int const at = plane * k;
-            bool const mine = src.pending && k >= k0 && k < k1;
-            for_slots([&](int s, int e) {
-                int const n = !EDGE || ((grid >> s) & 1u) ? static_cast<int>(sizeof(T)) : 0;
-                march_copy(&sm.raw[0][e], src.z + (off[s] + at), n);
-                march_copy(&sm.raw[1][e], src.pold + (off[s] + at), n);
-                if (mine && ((owned >> s) & 1u)) march_copy(&sm.raw[2][e], src.x + (off[s] + at), n);
-            });
         }
         march_commit();
-    };
-    // Direction form: the copied fields of plane k (this thread's own slots)
-    // become its operand.
-    auto combine = [&](int k, int to) {
-        if constexpr (!kDirect) {
-            bool const deep = k > 0 && k + 1 < g.nz, there = k >= 0 && k < g.nz, mine = k >= k0 && k < k1;
-            int const at = plane * k;
-            for_slots([&](int s, int e) {
-                T v = T(0);
-                if (there && (!EDGE || ((grid >> s) & 1u))) {
-                    T const po = sm.raw[1][e], p = sm.raw[0][e] + src.beta * po;
-                    if (mine && ((owned >> s) & 1u)) {
-                        src.pnew[off[s] + at] = p;
-                        if (src.pending) src.x[off[s] + at] = sm.raw[2][e] + src.alpha * po;
-                    }
-                    if (deep && (!EDGE || ((inner >> s) & 1u))) v = p;
-                }
-                sm.a[to + e] = v;
-            });
-        }
     };
 
     // the thread's column
@@ -184,18 +116,9 @@ __device__ __forceinline__ void mag3d_march_tile(MarchSmem<T, Src>& sm, Grid3<T>
 
     int slot0 = 0, slot1 = kElems, slot2 = 2 * kElems;   // of planes k, k + 1, k + 2
     fetch(k0 - 1, slot0);
-    if constexpr (kDirect) {
-        fetch(k0, slot1);
-        fetch(k0 + 1, slot2);
-        march_wait<1>();
-    } else {
-        march_wait<0>();
-        combine(k0 - 1, slot0);
-        fetch(k0, 0);
-        march_wait<0>();
-        combine(k0, slot1);
-        fetch(k0 + 1, 0);
-    }
+    fetch(k0, slot1);
+    fetch(k0 + 1, slot2);
+    march_wait<1>();
     __syncthreads();
 
     int const at = (ty * kMarchNodes + tx) * 3;
@@ -224,14 +147,9 @@ __device__ __forceinline__ void mag3d_march_tile(MarchSmem<T, Src>& sm, Grid3<T>
         sm.h[hs] = hx;
         sm.h[hs + kMarchThreads] = hz;
         march_wait<0>();
-        if constexpr (!kDirect) {
-            // plane k + 2 takes the slot of plane k - 1, last read before the previous barrier
-            if (k + 2 <= k1) combine(k + 2, slot2);
-            fetch(k + 3, 0);
-        }
         __syncthreads();
         // plane k's slot is free now
-        if constexpr (kDirect) fetch(k + kMarchRing, slot0);
+        fetch(k + kMarchRing, slot0);
         T const hy_left = __shfl_up_sync(0xffffffffu, hy, 1), hz_left = __shfl_up_sync(0xffffffffu, hz, 1);
         T hx_low = T(0), hz_low = T(0);
         if (ty > 0) {
@@ -247,9 +165,9 @@ __device__ __forceinline__ void mag3d_march_tile(MarchSmem<T, Src>& sm, Grid3<T>
                 q2 = (((hx_low - hx) + hy) - hy_left) + (g.gamma * ((lx * ly) * ilz)) * az;
             } else {
                 // identity row of a boundary node: the operand itself
-                q0 = p0 = src.at(row);
-                q1 = p1 = src.at(row + 1);
-                q2 = p2 = src.at(row + 2);
+                q0 = p0 = a[row];
+                q1 = p1 = a[row + 1];
+                q2 = p2 = a[row + 2];
             }
             out(row, q0, p0);
             out(row + 1, q1, p1);
@@ -272,13 +190,13 @@ __device__ __forceinline__ void mag3d_march_tile(MarchSmem<T, Src>& sm, Grid3<T>
     march_wait<0>();   // nothing still targets shared memory when the block reuses it or exits
 }
 
-template <class T, class Src, class Out>
-__device__ __forceinline__ void mag3d_march(MarchSmem<T, Src>& sm, Grid3<T> const& g, T const* nu, Src const& src, int i0,
-                                            int j0, int k0, int k1, Out const& out)
+template <class T, class Out>
+__device__ __forceinline__ void mag3d_march(MarchSmem<T>& sm, Grid3<T> const& g, T const* nu, T const* a, int i0, int j0,
+                                            int k0, int k1, Out const& out)
 {
     bool const inside = i0 > 1 && j0 > 1 && i0 + kMarchCols < g.nx - 1 && j0 + kMarchOwnRows < g.ny - 1;
-    if (inside) mag3d_march_tile<false>(sm, g, nu, src, i0, j0, k0, k1, out);
-    else mag3d_march_tile<true>(sm, g, nu, src, i0, j0, k0, k1, out);
+    if (inside) mag3d_march_tile<false>(sm, g, nu, a, i0, j0, k0, k1, out);
+    else mag3d_march_tile<true>(sm, g, nu, a, i0, j0, k0, k1, out);
 }
 
 } // namespace sil

@@ -79,7 +79,7 @@ struct Vecs
     T* nu;
     T* ph;  // flexible CG: m stored directions p_j at ph + j * hstride
     T* qh;  // and their images q_j = A p_j
-    T* p2;  // persistent CG: the direction's second buffer (p and p2 alternate)
+    T* p2;  // 2D CG: the direction's second buffer (p and p2 alternate)
 };
 
 struct ProbInfo
@@ -717,9 +717,9 @@ struct Tile
 
 // ------------------------------------------------------------------ CG iteration
 //
-// One Jacobi-CG iteration is two kernels over the items of the problems that
-// still iterate (`act`, one CTA per item, so converged problems launch
-// nothing):
+// One Jacobi-CG iteration is two kernels in 2D over the CTAs of the problems
+// that still iterate (converged problems launch nothing), and three in 3D,
+// where the direction is a pass before the apply:
 //   direction  p = z + beta p_old (formed on the fly at the row and at its
 //              stencil neighbours; p double-buffered), x += alpha p_old of the
 //              previous iteration, q = A p, partial p.q
@@ -802,8 +802,9 @@ struct Begin
 // Start of iteration c of a chunk (c > 0: completes iteration c - 1 from its
 // partials).  lead: this CTA records the problem's state.  Every thread of the
 // block calls it; smem holds 2 * kThreads / 32 doubles.
+// in_place: the problem's directions all live in p (3D), not in p and p2 by turns.
 __device__ __forceinline__ Begin cg_begin(Scalars* s, int c, double const* part_rz, double const* part_rr, int npart,
-                                          int max_iters, bool lead, double* smem)
+                                          int max_iters, bool lead, double* smem, bool in_place)
 {
     Begin b {};
     int const now = c & 1, before = now ^ 1;
@@ -811,7 +812,7 @@ __device__ __forceinline__ Begin cg_begin(Scalars* s, int c, double const* part_
         if (lead && threadIdx.x == 0) s->stopped[now] = 1;
         return b;
     }
-    b.pbuf = s->pbuf0 ^ now;
+    b.pbuf = in_place ? 0 : s->pbuf0 ^ now;
     if (c == 0) {
         b.run = true;
         b.beta = s->beta;
@@ -916,7 +917,7 @@ __global__ void __launch_bounds__(kThreads, 2) cg_direction2_kernel(StripWork<T>
 {
     __shared__ double red[2 * kThreads / 32];
     StripWork<T> const w = work[blockIdx.x];
-    Begin const b = cg_begin(w.s, c, w.part_rz, w.part_rr, w.npart, w.max_iters, w.index == 0, red);
+    Begin const b = cg_begin(w.s, c, w.part_rz, w.part_rr, w.npart, w.max_iters, w.index == 0, red, false);
     if (!b.run) return;
     T* __restrict__ pnew = b.pbuf == 0 ? w.p2 : w.p;
     T* __restrict__ x = w.x;
@@ -940,7 +941,8 @@ __global__ void __launch_bounds__(kThreads, 2) cg_direction2_kernel(StripWork<T>
     if (threadIdx.x == 0) w.part_pq[w.index] = t;
 }
 
-template <class T>
+// Z: z is stored for the 2D stencil; the 3D direction forms it again from r.
+template <class T, bool Z>
 __global__ void __launch_bounds__(kThreads) cg_update_kernel(Work<T> const* work, int c)
 {
     __shared__ double red[2 * kThreads / 32];
@@ -980,7 +982,7 @@ __global__ void __launch_bounds__(kThreads) cg_update_kernel(Work<T> const* work
             if (row + u * kThreads >= w.end) continue;
             T const rn = rv[u] - alpha * qv[u], zn = dv[u] * rn;
             r[row + u * kThreads] = rn;
-            z[row + u * kThreads] = zn;
+            if constexpr (Z) z[row + u * kThreads] = zn;
             rz += static_cast<double>(rn) * static_cast<double>(zn);
             rr += static_cast<double>(rn) * static_cast<double>(rn);
         }
@@ -996,13 +998,13 @@ __global__ void __launch_bounds__(kThreads) cg_update_kernel(Work<T> const* work
 
 // End of a chunk of `c` iterations: completes the last one (one CTA per item;
 // only each problem's first works).
-template <class T>
+template <class T, bool IN_PLACE>
 __global__ void __launch_bounds__(kThreads) cg_close_kernel(Work<T> const* work, int c)
 {
     __shared__ double red[2 * kThreads / 32];
     Work<T> const w = work[blockIdx.x];
     if (w.index != 0) return;
-    Begin const b = cg_begin(w.s, c, w.part_rz, w.part_rr, w.npart, w.max_iters, true, red);
+    Begin const b = cg_begin(w.s, c, w.part_rz, w.part_rr, w.npart, w.max_iters, true, red, IN_PLACE);
     __syncthreads();
     if (threadIdx.x == 0 && !w.s->outer_done) {
         w.s->done = b.run ? 0 : 1;
@@ -1010,61 +1012,81 @@ __global__ void __launch_bounds__(kThreads) cg_close_kernel(Work<T> const* work,
     }
 }
 
-// The direction kernel for batches of 3D penalty-gauge problems, in marching
-// tiles (mag3d_march.cuh): p = z + beta p_old, x += alpha p_old on the read of
-// p_old, q = A p, the partials of p.q.  B200, per iteration of one 160^3 problem
-// against a direction pass, a node-per-thread apply and x in the update: FP64
-// 392 -> 293 us, FP32 270 -> 217 (this kernel 155 and 106 us of it).
-template <class T>
-__global__ void __launch_bounds__(kMarchThreads, sizeof(T) == 8 ? 3 : 4)
-        cg_march_kernel(Tile const* tiles, int const* act, ProbInfo const* info, Vecs<T> const* vecs, Scalars* sc,
-                        double* part_pq, double const* part_rz, double const* part_rr, int c)
-{
-    extern __shared__ __align__(16) unsigned char march_smem[];
-    auto& sm = *reinterpret_cast<MarchSmem<T, MarchDirection<T>>*>(march_smem);
-    __shared__ double red[2 * kThreads / 32];
-    static_assert(kMarchThreads == kThreads, "block_sum covers the block");
-    Tile const t = tiles[act[blockIdx.x]];
-    ProbInfo const& pi = info[t.prob];
-    Begin const b = cg_begin(sc + t.prob, c, part_rz + pi.first_item, part_rr + pi.first_item, pi.nitems, pi.max_iters,
-                             t.index == 0, red);
-    if (!b.run) return;
-    Vecs<T> const v = vecs[t.prob];
-    bool const first = b.pbuf == 0;
-    MarchDirection<T> const src {v.z, first ? v.p : v.p2, first ? v.p2 : v.p, v.x, static_cast<T>(b.alpha),
-                                 static_cast<T>(b.beta), b.pending};
-    double pq = 0.0;
-    mag3d_march(sm, march_grid<T>(pi), static_cast<T const*>(v.nu), src, t.i0, t.j0, t.k0, t.k1, [&](int row, T q, T p) {
-        v.q[row] = q;
-        pq += static_cast<double>(p) * static_cast<double>(q);
-    });
-    __syncthreads();
-    double const pq_b = block_sum(pq, red);
-    if (threadIdx.x == 0) part_pq[pi.first_tile + t.index] = pq_b;
-}
-
-// Batches with the divergence gauge, whose stencil reaches two nodes: the
-// direction as a pass of its own, then the apply, a thread per node.
+// 3D problems: p = D^-1 r + beta p in place and x += alpha p_old as a pass of
+// their own, then the apply.  z is not stored and p not double-buffered, so an
+// iteration of a medium batch stays in L2: at the 4.9 M rows of 64^3 + 80^3 + 96^3
+// in FP32 its six vectors are 118 MB, with z and the second p 157.  Forming the
+// direction inside the marching apply (between its copies and its planes) moves
+// two vectors less but costs more instructions than this pass costs memory: one
+// 160^3 problem, per iteration, FP64 292 -> 265 us, FP32 217 -> 157.  Bound by
+// memory (6.4 TB/s at 160^3 in FP64); two rows in flight a thread instead of
+// four cost 8% of an FP64 iteration.
 template <class T>
 __global__ void __launch_bounds__(kThreads) cg_direction3_kernel(Work<T> const* work, int c)
 {
     __shared__ double red[2 * kThreads / 32];
     Work<T> const w = work[blockIdx.x];
-    Begin const b = cg_begin(w.s, c, w.part_rz, w.part_rr, w.npart, w.max_iters, w.index == 0, red);
-    if (!b.run) return;
-    T const* __restrict__ z = w.z;
-    T const* __restrict__ pold = b.pbuf == 0 ? w.p : w.p2;
-    T* __restrict__ pnew = b.pbuf == 0 ? w.p2 : w.p;
+    T const* __restrict__ r = w.r;
+    T const* __restrict__ dinv = w.dinv;
     T* __restrict__ x = w.x;
+    T* __restrict__ p = w.p;
+    // the first rows are on their way while the partials are summed
+    constexpr int U = 4;
+    T rv[U], dv[U], xv[U], pv[U];
+    int row = w.begin + static_cast<int>(threadIdx.x);
+    auto fetch = [&](int from) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            int const at = min(from + u * kThreads, w.end - 1);
+            rv[u] = r[at];
+            dv[u] = dinv[at];
+            xv[u] = x[at];
+            pv[u] = p[at];
+        }
+    };
+    fetch(row);
+    Begin const b = cg_begin(w.s, c, w.part_rz, w.part_rr, w.npart, w.max_iters, w.index == 0, red, true);
+    if (!b.run) return;
     T const beta = static_cast<T>(b.beta), alpha = static_cast<T>(b.alpha);
-#pragma unroll 4
-    for (int row = w.begin + static_cast<int>(threadIdx.x); row < w.end; row += kThreads) {
-        T const po = pold[row];
-        pnew[row] = z[row] + beta * po;
-        if (b.pending) x[row] = x[row] + alpha * po;
+    for (; row < w.end; row += U * kThreads) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            int const at = row + u * kThreads;
+            if (at >= w.end) continue;
+            p[at] = dv[u] * rv[u] + beta * pv[u];
+            if (b.pending) x[at] = xv[u] + alpha * pv[u];
+        }
+        fetch(row + U * kThreads);
     }
 }
 
+// q = A p and the partials of p.q for batches of penalty-gauge problems, in
+// marching tiles (mag3d_march.cuh).
+template <class T>
+__global__ void __launch_bounds__(kMarchThreads, 4)
+        cg_march_kernel(Tile const* tiles, int const* act, ProbInfo const* info, Vecs<T> const* vecs, Scalars const* sc,
+                        double* part_pq, int c)
+{
+    __shared__ MarchSmem<T> sm;
+    __shared__ double red[kThreads / 32];
+    static_assert(kMarchThreads == kThreads, "block_sum covers the block");
+    Tile const t = tiles[act[blockIdx.x]];
+    Scalars const* s = sc + t.prob;
+    if (s->stopped[c & 1]) return;
+    ProbInfo const& pi = info[t.prob];
+    Vecs<T> const v = vecs[t.prob];
+    T const* p = v.p;
+    double pq = 0.0;
+    mag3d_march(sm, march_grid<T>(pi), static_cast<T const*>(v.nu), p, t.i0, t.j0, t.k0, t.k1, [&](int row, T q, T pv) {
+        v.q[row] = q;
+        pq += static_cast<double>(pv) * static_cast<double>(q);
+    });
+    double const pq_b = block_sum(pq, red);
+    if (threadIdx.x == 0) part_pq[pi.first_tile + t.index] = pq_b;
+}
+
+// The apply of batches with the divergence gauge, whose stencil reaches two
+// nodes: a thread per node.
 template <class T>
 __global__ void __launch_bounds__(kThreads) cg_apply3_kernel(Item const* items, int const* act, ProbInfo const* info,
                                                              Vecs<T> const* vecs, Scalars const* sc, double* part_pq,
@@ -1076,7 +1098,7 @@ __global__ void __launch_bounds__(kThreads) cg_apply3_kernel(Item const* items, 
     if (s->stopped[c & 1]) return;
     ProbInfo const pi = info[it.prob];
     Vecs<T> const v = vecs[it.prob];
-    T const* p = (s->pbuf0 ^ (c & 1)) == 0 ? v.p2 : v.p;
+    T const* p = v.p;
     double pq = 0.0;
     for (int64_t node = it.begin / 3 + threadIdx.x; node < it.end / 3; node += kThreads) {
         T q[3];
@@ -1528,7 +1550,7 @@ __global__ void __launch_bounds__(kMarchThreads, 4)
                                 double const* const* rhs, double* const* x64, double* const* r64, Scalars* sc,
                                 double* part, double tol2, double floor2, int mark)
 {
-    __shared__ MarchSmem<double, MarchPlain<double>> sm;
+    __shared__ MarchSmem<double> sm;
     __shared__ double red[kThreads / 32];
     Tile const t = tiles[act[blockIdx.x]];
     Scalars* s = sc + t.prob;
@@ -1537,7 +1559,7 @@ __global__ void __launch_bounds__(kMarchThreads, 4)
     double const* b = rhs[t.prob];
     double* r64p = r64[t.prob];
     double rr = 0.0;
-    mag3d_march(sm, march_grid<double>(pi), nu64[t.prob], MarchPlain<double> {x64[t.prob]}, t.i0, t.j0, t.k0, t.k1,
+    mag3d_march(sm, march_grid<double>(pi), nu64[t.prob], static_cast<double const*>(x64[t.prob]), t.i0, t.j0, t.k0, t.k1,
                 [&](int row, double ax, double) {
                     double const r = b[row] - ax;
                     r64p[row] = r;
@@ -2226,9 +2248,14 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
         pi.max_iters = set.max_iterations > 0 ? set.max_iterations : 100000;
         pi.first_item = static_cast<int>(items.size());
         int idx = 0;
-        // 3D items: whole nodes (3 rows each), four times the 2D item, so
-        // the per-CTA prologue is amortised over more of the costlier 3D rows
-        int64_t const step = q.dim == 3 ? (4 * item_rows / 3) * 3 : item_rows;
+        // 3D divergence-gauge items: whole nodes (3 rows each), four times the
+        // others, so the per-CTA prologue is amortised over the costlier apply.
+        // A problem has at most one wave of four CTAs a multiprocessor, as every
+        // CTA sums its partials (64^3 + 80^3 + 96^3, an iteration: at most 592
+        // items 62 us FP32 and 104 FP64, at most 1,024 65 and 107)
+        int64_t const most = 4 * static_cast<int64_t>(sm_count());
+        int64_t const rows = std::max<int64_t>(item_rows, (pi.n / most + kThreads) / kThreads * kThreads);
+        int64_t const step = q.dim == 3 && q.gauge != 0 ? (4 * rows / 3) * 3 : rows / 3 * 3;
         for (int64_t b = 0; b < pi.n; b += step, ++idx) items.push_back({p, idx, b, std::min(pi.n, b + step)});
         pi.nitems = idx;
         total_rows += pi.n;
@@ -2249,7 +2276,7 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
     });
     std::vector<Tile> tiles;
     if (march) {
-        int const planes = march_planes(info, static_cast<int64_t>(sizeof(T) == 8 ? 3 : 4) * sm_count());
+        int const planes = march_planes(info, 4 * static_cast<int64_t>(sm_count()));
         for (int p = 0; p < np; ++p) {
             ProbInfo& pi = info[p];
             pi.first_tile = static_cast<int>(tiles.size());
@@ -2261,8 +2288,6 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
                                          static_cast<int>(std::min(pi.nz, k + planes))});
             pi.ntiles = idx;
         }
-        SIL_CUDA_CHECK(cudaFuncSetAttribute(cg_march_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            static_cast<int>(sizeof(MarchSmem<T, MarchDirection<T>>))));
     }
     int const ntiles = static_cast<int>(tiles.size());
     // Strips of a 2D batch.
@@ -2505,17 +2530,19 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
         cudaError_t err = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
         for (int c = 0; c < chunk && err == cudaSuccess; ++c) {
             if (march) {
-                cg_march_kernel<T><<<nt, kMarchThreads, sizeof(MarchSmem<T, MarchDirection<T>>), cs>>>(
-                        d_tiles, d_tact, d_info, d_vecs, d_sc, part_a, part_b, part_c, c);
+                cg_direction3_kernel<T><<<n, kThreads, 0, cs>>>(d_work, c);
+                cg_march_kernel<T><<<nt, kMarchThreads, 0, cs>>>(d_tiles, d_tact, d_info, d_vecs, d_sc, part_a, c);
             } else if (any_gauge) {
                 cg_direction3_kernel<T><<<n, kThreads, 0, cs>>>(d_work, c);
                 cg_apply3_kernel<T><<<n, kThreads, 0, cs>>>(d_items, d_act, d_info, d_vecs, d_sc, part_a, c);
             } else {
                 cg_direction2_kernel<T><<<ns, kThreads, 0, cs>>>(d_strips, c);
             }
-            cg_update_kernel<T><<<n, kThreads, 0, cs>>>(d_work, c);
+            if (flat) cg_update_kernel<T, true><<<n, kThreads, 0, cs>>>(d_work, c);
+            else cg_update_kernel<T, false><<<n, kThreads, 0, cs>>>(d_work, c);
         }
-        cg_close_kernel<T><<<n, kThreads, 0, cs>>>(d_work, chunk);
+        if (flat) cg_close_kernel<T, false><<<n, kThreads, 0, cs>>>(d_work, chunk);
+        else cg_close_kernel<T, true><<<n, kThreads, 0, cs>>>(d_work, chunk);
         cudaError_t const err2 = cudaStreamEndCapture(cs, &graph);
         if (err == cudaSuccess) err = err2;
         if (err == cudaSuccess) err = cudaGraphInstantiate(&exec, graph, 0);
@@ -3053,10 +3080,10 @@ __global__ void __launch_bounds__(kMarchThreads, kApplyCtas)
         mag3d_march_kernel(Grid3<double> g, double const* nu, double const* a, double* y, int tiles_x, int tiles_y,
                            int planes)
 {
-    __shared__ MarchSmem<double, MarchPlain<double>> sm;
+    __shared__ MarchSmem<double> sm;
     int const t = blockIdx.x / tiles_x, bx = blockIdx.x - t * tiles_x, bz = t / tiles_y, by = t - bz * tiles_y;
     int const k0 = bz * planes;
-    mag3d_march(sm, g, nu, MarchPlain<double> {a}, bx * kMarchCols, by * kMarchOwnRows, k0, min(g.nz, k0 + planes),
+    mag3d_march(sm, g, nu, a, bx * kMarchCols, by * kMarchOwnRows, k0, min(g.nz, k0 + planes),
                 [&](int row, double q, double) { y[row] = q; });
 }
 
