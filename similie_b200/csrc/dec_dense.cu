@@ -15,7 +15,7 @@
 // Measured on a B200, table-driven -> here: 1-form Laplacian 161x144x130 FP64
 // 2,366 -> 145 us, 1999x2741 FP32 1,016 -> 46 us; d + star + codifferential of
 // a 150x171x128 1-form FP64 651 -> 122 us (the star is one kernel on both
-// sides).
+// sides; the codifferential's march takes it to 112).
 #include <algorithm>
 #include <cstdint>
 #include <cstdlib>
@@ -637,6 +637,107 @@ __global__ void __launch_bounds__(kMarchZ* Y, CTAS)
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
+// The 3D codifferential, marched the same way: S from the ring's plane, its y
+// and z neighbours through a double-buffered plane, its x neighbour kept.  Only
+// lower neighbours are read, so the tile owns 31 x (Y - 1) columns.
+//
+// Bound by its loads in flight and the idle threads of its tiles (63 % of the
+// copy rate at 150x171x128, FP64).  B200, node kernel -> march at that size: 2-form
+// FP64 52.8 -> 39.8 us, FP32 47.2 -> 27.5; 1-form 34.5 -> 30.1, 32.0 -> 24.1;
+// 3-form 36.2 -> 30.2, 33.4 -> 20.1.
+template <class T, int K, int Y>
+struct Codiff3Smem
+{
+    T w[3][Y * kMarchZ * Stages<3, K>::kIn];
+    T s[2][Stages<3, K>::kIn][kMarchZ * Y];
+};
+
+template <class T, int K, int Y, int CTAS>
+__global__ void __launch_bounds__(kMarchZ* Y, CTAS)
+        codiff3_march_kernel(const __grid_constant__ Dense<T, 3> a, int tiles_z, int tiles_y, int planes)
+{
+    using St = Stages<3, K>;
+    constexpr int kThreads = kMarchZ * Y, kRow = kMarchZ * St::kIn, kSlots = St::kIn;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    auto& sm = *reinterpret_cast<Codiff3Smem<T, K, Y>*>(smem_raw);
+    int const tid = threadIdx.x, tz = tid & 31, ty = tid >> 5;
+    int const t = blockIdx.x / tiles_z, bz = blockIdx.x - t * tiles_z, bx = t / tiles_y, by = t - bx * tiles_y;
+    int const oz = bz * (kMarchZ - 1), oy = by * (Y - 1), ox0 = bx * planes, ox1 = min(a.oext[0], ox0 + planes);
+    int const z = oz + a.off[2] - 1 + tz, y = oy + a.off[1] - 1 + ty;
+    int const X = a.iext[0], Ny = a.iext[1], Nz = a.iext[2];
+    auto clampi = [](int v, int n) { return min(max(v, 0), n - 1); };
+    bool const col_in = z >= 0 && y >= 0 && z < Nz && y < Ny;
+    bool const own = tz > 0 && ty > 0 && oz + tz - 1 < a.oext[2] && oy + ty - 1 < a.oext[1];
+    int src[kSlots];
+#pragma unroll
+    for (int q = 0; q < kSlots; ++q) {
+        int const e = tid + q * kThreads, r = e / kRow, c = e - r * kRow;
+        src[q] = clampi(oy + a.off[1] - 1 + r, Ny) * a.istr[1]
+                 + clampi(oz + a.off[2] - 1 + c / St::kIn, Nz) * a.istr[2] + c % St::kIn * a.ics;
+    }
+    int const x_first = ox0 + a.off[0] - 1, x_last = ox1 - 1 + a.off[0];
+    auto fetch = [&](int x, int slot) {
+        if (x <= x_last) {
+            T const* plane = a.in + static_cast<int64_t>(clampi(x, X)) * a.istr[0];
+#pragma unroll
+            for (int q = 0; q < kSlots; ++q)
+                copy_async(&sm.w[slot][tid + q * kThreads], plane + src[q], Int<static_cast<int>(sizeof(T))> {});
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(x_first, 0);
+    fetch(x_first + 1, 1);
+    fetch(x_first + 2, 2);
+    T h[3], ih[3];
+    h[1] = __ldg(a.h[1] + clampi(y, Ny));
+    ih[1] = __ldg(a.ih[1] + clampi(y, Ny));
+    h[2] = __ldg(a.h[2] + clampi(z, Nz));
+    ih[2] = __ldg(a.ih[2] + clampi(z, Nz));
+    asm volatile("cp.async.wait_group 2;" ::: "memory");
+    __syncthreads();
+    int const at = tid * St::kIn, back_z = tz > 0 ? tid - 1 : tid, back_y = ty > 0 ? tid - kMarchZ : tid;
+    T* o = a.out + static_cast<int64_t>(ox0) * a.ostr[0] + (oy + ty - 1) * a.ostr[1] + (oz + tz - 1) * a.ostr[2];
+    Vals<T, St::kIn> s0;
+#pragma unroll
+    for (int c = 0; c < St::kIn; ++c) s0.v[c] = T(0);
+    int slot0 = 0, slot1 = 1, slot2 = 2;
+    for (int x = x_first; x <= x_last; ++x) {
+        int const buf = x & 1;
+        h[0] = __ldg(a.h[0] + clampi(x, X));
+        ih[0] = __ldg(a.ih[0] + clampi(x, X));
+        Vals<T, St::kIn> w;
+#pragma unroll
+        for (int c = 0; c < St::kIn; ++c) w.v[c] = sm.w[slot0][at + c];
+        Vals<T, St::kIn> const s1 = stage_s<3, K, T>(w, h, ih, col_in && x >= 0 && x < X);
+#pragma unroll
+        for (int c = 0; c < St::kIn; ++c) sm.s[buf][c][tid] = s1.v[c];
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        // every thread is past plane x's slot: plane x + 3 takes it
+        fetch(x + 3, slot0);
+        if (x > x_first && own) {
+            Vals<T, St::kE> const e = stage_e<3, K, T>(
+                    [&](auto dim, auto shift, auto comp) -> T {
+                        constexpr int C = decltype(comp)::value;
+                        if constexpr (decltype(shift)::value == 0) return s1.v[C];
+                        else if constexpr (decltype(dim)::value == 0) return s0.v[C];
+                        else if constexpr (decltype(dim)::value == 1) return sm.s[buf][C][back_y];
+                        else return sm.s[buf][C][back_z];
+                    },
+                    h, ih);
+#pragma unroll
+            for (int c = 0; c < St::kE; ++c) o[c * a.ocs] = e.v[c];
+            o += a.ostr[0];
+        }
+        s0 = s1;
+        int const q = slot0;
+        slot0 = slot1;
+        slot1 = slot2;
+        slot2 = q;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
 // ---- 2D 1-forms: a warp per strip of 30 owned columns (y along the lanes), no
 // shared memory: the y neighbours' values come from the next lanes.  Four
 // planes' loads are in flight before the first is used.
@@ -874,6 +975,43 @@ bool launch_lap3(cudaStream_t stream, Dense<T, 3> const& a)
     return true;
 }
 
+// At 150x171x128 the FP64 2-form took 39.8 us with four CTAs of 8 rows, 39.1
+// with three (FP32 and the other ranks 3 % slower), 48.2 with five, 45.7 with
+// three of 12 rows and 47.5 with two of 16.
+constexpr int kCodiff3Y = 8, kCodiff3Ctas = 4;
+
+// Whether the 3D codifferential marches: boxes of 500,000 nodes on, below which
+// too few planes are in flight (FP64, node kernel -> march: 32^3 2-form 3.2 ->
+// 3.8 us, 64^3 7.7 -> 7.6, 1-form 5.7 -> 6.5; 80^3 11.5 -> 8.6 and 8.1 -> 6.9),
+// whose columns the tiles cover without too many idle ones: 300x300x24 2-form
+// 51.0 -> 28.0 (tiles of 1.30 times its columns), 200x9x400 11.3 -> 12.9 (1.57);
+// a 1-form writes one component and gains less: 96^3 12.4 -> 13.3 (1.32),
+// 110^3 15.0 -> 14.4 (1.14).
+template <int K, class T>
+bool codiff3_marches(Dense<T, 3> const& a)
+{
+    int64_t const columns = static_cast<int64_t>(a.oext[1]) * a.oext[2];
+    int64_t const tz = (a.oext[2] + kMarchZ - 2) / (kMarchZ - 1), ty = (a.oext[1] + kCodiff3Y - 2) / (kCodiff3Y - 1);
+    int64_t const covered = tz * (kMarchZ - 1) * ty * (kCodiff3Y - 1);
+    return columns * a.oext[0] >= 500000 && covered * 4 <= columns * (K == 1 ? 5 : 6) && box_inside(a);
+}
+
+template <class T, int K>
+bool launch_codiff3(cudaStream_t stream, Dense<T, 3> const& a)
+{
+    constexpr size_t smem = sizeof(Codiff3Smem<T, K, kCodiff3Y>);
+    auto const kernel = codiff3_march_kernel<T, K, kCodiff3Y, kCodiff3Ctas>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
+        return false;
+    int const tz = (a.oext[2] + kMarchZ - 2) / (kMarchZ - 1), ty = (a.oext[1] + kCodiff3Y - 2) / (kCodiff3Y - 1);
+    int64_t const columns = static_cast<int64_t>(tz) * ty;
+    int const planes = run_length(columns, a.oext[0], static_cast<int64_t>(kCodiff3Ctas) * multiprocessors());
+    int64_t const blocks = columns * ((a.oext[0] + planes - 1) / planes);
+    if (blocks >= (int64_t(1) << 31)) return false;
+    kernel<<<static_cast<unsigned>(blocks), kMarchZ * kCodiff3Y, smem, stream>>>(a, tz, ty, planes);
+    return true;
+}
+
 template <class T>
 bool launch_lap2(cudaStream_t stream, Dense<T, 2> const& a)
 {
@@ -899,6 +1037,8 @@ bool launch_rank(cudaStream_t stream, Geometry const* geo, int k, sil_field cons
             auto const a = dense_args<T, N>(geo, in, out, total);
             if constexpr (OP == kLaplacian && N == 3)
                 if (total >= kLap3Min<K> && box_inside(a) && launch_lap3<T, K>(stream, a)) return true;
+            if constexpr (OP == kCodiff && N == 3)
+                if (codiff3_marches<K>(a) && launch_codiff3<T, K>(stream, a)) return true;
             if constexpr (OP == kLaplacian && N == 2 && K == 1)
                 if (box_inside(a) && launch_lap2<T>(stream, a)) return true;
             unsigned const blocks = static_cast<unsigned>((total + kDenseBlock - 1) / kDenseBlock);

@@ -41,6 +41,26 @@ def test_marching_laplacians_equal_the_table_driven_ones(shape, ks, dtype):
                 assert torch.equal(torch.nan_to_num(got), torch.nan_to_num(ref)), (k, oshape, front, layout)
 
 
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("shape,ks", [((83, 77, 92), (1, 2, 3)), ((84, 78, 94), (2,)), ((78, 84, 93), (1, 3)),
+                                      ((3, 447, 400), (2, 3))])
+def test_marching_codifferentials_equal_the_table_driven_ones(shape, ks, dtype):
+    """Tiles of 31 x 7 owned nodes: just under, exactly, and one over a whole number of them; few planes."""
+    import similie_b200 as sb
+    rng = np.random.default_rng(sum(shape))
+    geo = sb.Geometry([np.cumsum(rng.uniform(0.3, 1.7, s + 4)) for s in shape])
+    for k in ks:
+        inp = torch.from_numpy(rng.standard_normal(shape + (comb(3, k),))).cuda().to(dtype)
+        inp.view(-1)[11], inp.view(-1)[-97] = float("inf"), float("nan")
+        for oshape, front in ((shape, (0, 0, 0)), ((shape[0],) + tuple(s - 1 for s in shape[1:]), (0, 1, 0)),
+                              (tuple(s - 1 for s in shape), (1, 0, 1))):
+            for layout in ("last", "first", "reversed"):
+                got, ref = (_run(sb, "codifferential", geo, shape, k, k - 1, inp, oshape, front, layout, dtype, sp)
+                            for sp in (False, True))
+                assert torch.equal(torch.isnan(got), torch.isnan(ref)), (k, oshape, front, layout)
+                assert torch.equal(torch.nan_to_num(got), torch.nan_to_num(ref)), (k, oshape, front, layout)
+
+
 def _laid_out(t, layout):
     """The same values under another layout: component last, component first, lattice axes reversed in memory."""
     n = t.dim() - 1
