@@ -525,7 +525,7 @@ struct Scalars
     int iters;        // iterations of the current solve
     int total_iters;  // all inner iterations
     int nonfinite;
-    int counter_a, counter_b, counter_c;
+    int counter_a, counter_c;
     // flexible CG with the learned preconditioner
     double win_rr;    // r . r at the start of the stall window
     int win_iters;    // iterations into the stall window
@@ -1641,8 +1641,8 @@ __global__ void copy_from_vec_kernel(Item const* items, Vecs<T> const* vecs, dou
 // grid rows each, p, nu and D^-1 in shared memory and r, x and q in registers,
 // so an iteration reads nothing from memory but the two neighbour rows of z
 // and the group's partial sums.  An iteration has two waits for the group (after
-// p.q and after r.z), each a counter in global memory; a group whose problem
-// has ended leaves, and groups of several problems run side by side.  The
+// p.q and after r.z), where its sums pass through global memory; a group whose
+// problem has ended leaves, and groups of several problems run side by side.  The
 // arithmetic is the launch-per-kernel path's, the sums in another order.
 //
 // B200, per iteration against two kernels: four problems of 96^2 .. 161^2 11.2 ->
@@ -2810,7 +2810,7 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
     SIL_CUDA_CHECK(cudaStreamSynchronize(stream));
     for (int p = 0; p < np; ++p) {
         hs2[p].outer_done = 0;
-        hs2[p].counter_a = hs2[p].counter_b = hs2[p].counter_c = 0;
+        hs2[p].counter_a = hs2[p].counter_c = 0;
     }
     SIL_CUDA_CHECK(cudaMemcpyAsync(d_sc, hs2.data(), sizeof(Scalars) * np, cudaMemcpyHostToDevice, stream));
     residual64<<<nitems, kThreads, 0, stream>>>(d_items, nullptr, d_info, d_nu64, d_rhs, d_sol, d_scratch, d_sc,

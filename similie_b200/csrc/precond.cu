@@ -74,8 +74,8 @@ __device__ __forceinline__ bool image_active(Table const& t, int im)
 // upsampled coarse tensor (two operands summed by the tensor core); kMasked a
 // FP32 gradient masked by ReLU activity (data and weight gradients);
 // kUpOnly the upsampled coarse tensor alone (second pass of kUpAdd's weight
-// gradient); kPool a 2x2 average of the finer level.
-enum InMode { kPlain = 0, kPool = 1, kUpAdd = 2, kMasked = 3, kUpOnly = 4 };
+// gradient).
+enum InMode { kPlain = 0, kUpAdd, kMasked, kUpOnly };
 
 __device__ __forceinline__ void unpack8(uint4 u, float* f)
 {
@@ -217,8 +217,9 @@ __device__ __forceinline__ void walk_active(Table const& t, int64_t* pre, int pe
 }
 
 // The 32 channels (four 16-byte chunks) of the convolution input at padded
-// flat pixel g of image im, per input mode.  Zero outside the padded image
-// and on its border.  32-bit pixel arithmetic (images below 2^31 pixels).
+// flat pixel g of image im, per input mode (kUpAdd's operands are staged apart
+// or taken in two passes).  Zero outside the padded image and on its border.
+// 32-bit pixel arithmetic (images below 2^31 pixels).
 __device__ __forceinline__ void load_pixel(int mode, Table const& t, int im, int g, bf16 const* in, bf16 const* in2,
                                            float const* gin, uint4 (&v)[kChunks])
 {
@@ -252,60 +253,12 @@ __device__ __forceinline__ void load_pixel(int mode, Table const& t, int im, int
         }
         return;
     }
-    if (mode == kPool) {
-        Img const fi = t.aux[im];
-        int const Pf = fi.w + 2;
-        int64_t const base = fi.offset + static_cast<int64_t>(2 * y - 1) * Pf + (2 * x - 1);
-        int64_t const px[4] = {base, base + 1, base + Pf, base + Pf + 1};
-        uint4 const* src = reinterpret_cast<uint4 const*>(in);
-        uint4 raw[4][kChunks];
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-            for (int c = 0; c < kChunks; ++c) raw[q][c] = __ldg(src + px[q] * kChunks + c);
-#pragma unroll
-        for (int c = 0; c < kChunks; ++c) {
-            float f[8], a[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] = 0.0f;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                unpack8(raw[q][c], a);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) f[i] = f[i] + a[i];
-            }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] = f[i] * 0.25f;
-            v[c] = pack8(f);
-        }
-        return;
-    }
     Img const ci = t.aux[im];
     int64_t const cpx = ci.offset + static_cast<int64_t>((y - 1) / 2 + 1) * (ci.w + 2) + ((x - 1) / 2 + 1);
-    if (mode == kUpOnly) {
-        uint4 const* cp = reinterpret_cast<uint4 const*>(in2) + cpx * kChunks;
-#pragma unroll
-        for (int c = 0; c < kChunks; ++c) v[c] = __ldg(cp + c);
-        return;
-    }
-    // kUpAdd: skip (this level) + nearest-upsampled coarse features
-    uint4 const* sp = reinterpret_cast<uint4 const*>(in) + (o.offset + g) * kChunks;
+    // kUpOnly
     uint4 const* cp = reinterpret_cast<uint4 const*>(in2) + cpx * kChunks;
-    uint4 a4[kChunks], b4[kChunks];
 #pragma unroll
-    for (int c = 0; c < kChunks; ++c) {
-        a4[c] = __ldg(sp + c);
-        b4[c] = __ldg(cp + c);
-    }
-#pragma unroll
-    for (int c = 0; c < kChunks; ++c) {
-        float f[8], a[8];
-        unpack8(a4[c], f);
-        unpack8(b4[c], a);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) f[i] = f[i] + a[i];
-        v[c] = pack8(f);
-    }
+    for (int c = 0; c < kChunks; ++c) v[c] = __ldg(cp + c);
 }
 
 // Stage the three 130-pixel halo rows of the tile starting at flat pixel
@@ -2081,7 +2034,7 @@ size_t wgrad_smem() { return sizeof(WgradSmem) + 1024; }
 
 bool g_attr_done = false;
 int g_sms = 0;  // multiprocessor count, read once (outside any stream capture)
-int g_conv_per_sm[5] = {0, 0, 0, 0, 0};  // resident conv CTAs per SM, by input mode
+int g_conv_per_sm[kUpOnly + 1] = {};  // resident conv CTAs per SM, by input mode
 // Grid-stride kernels of the forward pass and their resident blocks per SM.
 enum WalkKind { kWalkInc = 0, kWalkOut, kWalkGather, kWalkPool, kWalkCopy, kWalkFeat, kWalkPre, kWalkPost, kWalkLogNu,
                 kWalkE2, kWalkUpAdd, kWalkKinds };
@@ -2113,7 +2066,7 @@ sil_status ensure_attributes()
     int smem_sm = 0, regs_sm = 0;
     SIL_CUDA_CHECK(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
     SIL_CUDA_CHECK(cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev));
-    for (int m = 0; m < 5; ++m) {
+    for (int m = 0; m <= kUpOnly; ++m) {
         int const by_smem = smem_sm / static_cast<int>(conv_smem(m) + 1024);
         int const by_regs = regs_sm / std::max(1, ((m == kPlain ? fp : fa).numRegs + 7) / 8 * 8 * 128);
         g_conv_per_sm[m] = std::max(1, std::min(std::min(by_smem, by_regs), 8));
