@@ -1982,6 +1982,74 @@ struct DeviceBuffer
     ~DeviceBuffer() { cudaFree(ptr); }
 };
 
+// Memory of small solves comes from a pool of the device that keeps up to
+// kPoolKeep bytes between calls (the rest goes back to the device at the next
+// synchronisation, and all of it when a larger solve finds no memory).  The pool
+// is stream-ordered, so threads and streams can share it.  cudaMalloc and
+// cudaFree map and unmap at every call, 0.4 ms each: four 2D problems of 96^2 ..
+// 161^2 5.4 -> 4.6 ms a solve, one 32^3 5.4 -> 4.7.  Larger solves, of whose time
+// that is a percent or two, do not hold on to memory.
+constexpr size_t kPoolKeep = size_t(64) << 20;
+
+cudaMemPool_t solve_pool()
+{
+    static std::mutex mutex;
+    static cudaMemPool_t pools[16] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= 16) return nullptr;
+    std::lock_guard<std::mutex> lock(mutex);
+    if (pools[dev] == nullptr) {
+        cudaMemPoolProps props {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        uint64_t keep = kPoolKeep;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        pools[dev] = pool;
+    }
+    return pools[dev];
+}
+
+struct SolveBuffer
+{
+    void* ptr = nullptr;
+    cudaStream_t stream = nullptr;
+    bool pooled = false;
+
+    cudaError_t take(size_t bytes, cudaStream_t st)
+    {
+        stream = st;
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        cudaMemPool_t pool = nullptr;
+        if (cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) pool = solve_pool();
+        if (pool != nullptr && bytes <= kPoolKeep) {
+            pooled = cudaMallocFromPoolAsync(&ptr, bytes, pool, st) == cudaSuccess;
+            if (pooled) return cudaSuccess;
+            cudaGetLastError();
+            ptr = nullptr;
+        }
+        cudaError_t e = cudaMalloc(&ptr, bytes);
+        if (e == cudaErrorMemoryAllocation && pool != nullptr) {
+            cudaGetLastError();
+            cudaMemPoolTrimTo(pool, 0);
+            e = cudaMalloc(&ptr, bytes);
+        }
+        return e;
+    }
+    ~SolveBuffer()
+    {
+        if (pooled) {
+            cudaStreamSynchronize(stream);   // as cudaFree: nothing of the call runs on
+            cudaFreeAsync(ptr, stream);
+        } else cudaFree(ptr);
+    }
+};
+
 // One problem of a batch, 2D or 3D, as the solver driver sees it.
 struct ProblemDesc
 {
@@ -2339,8 +2407,8 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
              + (sizeof(Tile) + sizeof(int)) * ntiles + sizeof(Work<T>) * nitems
              + sizeof(StripWork<T>) * nstrip_ctas
              + (sizeof(ResidentCta) + 2 * kMailSets * sizeof(unsigned long long)) * nres + 30 * 256;
-    DeviceBuffer buf;
-    SIL_CUDA_CHECK(cudaMalloc(&buf.ptr, bytes));
+    SolveBuffer buf;
+    SIL_CUDA_CHECK(buf.take(bytes, stream));
     char* base = static_cast<char*>(buf.ptr);
     auto take = [&](size_t b) {
         char* r = base;
