@@ -352,16 +352,18 @@ __device__ __forceinline__ void stage_halo_up(uint4* halo, Table const& t, int i
     }
 }
 
-// The apply's kernels follow one another by programmatic dependent launch: a
-// kernel's CTAs may take their places, and do what needs no predecessor (the
-// convolutions their weights, TMEM and barriers), while the previous kernel's
-// last CTAs run.  after_previous comes before anything the previous kernel
-// wrote is read and before anything is written, in every CTA, and lets the next
-// kernel start only from there: so when a kernel starts, every kernel before
-// its predecessor has finished and two at most are under way.  The pointers to
-// what the predecessor wrote pass through the wait, so no load by them can be
-// moved ahead of it.  B200, 36 launches an apply: eight samples of 256^2 ..
-// 1024^2 552 -> 468 us, a learned solve of five problems 149 -> 139 ms.
+// The kernels of an apply and of a gradient's backward pass follow one another
+// by programmatic dependent launch: a kernel's CTAs may take their places, and do
+// what needs no predecessor (the convolutions their weights, TMEM and barriers),
+// while the previous kernel's last CTAs run.  after_previous comes before
+// anything the previous kernel wrote is read and before anything is written, in
+// every CTA, and lets the next kernel start only from there: so when a kernel
+// starts, every kernel before its predecessor has finished and two at most are
+// under way.  The pointers to what the predecessor wrote pass through the wait,
+// so no load by them can be moved ahead of it.  B200: an apply of 36 launches,
+// eight samples of 256^2 .. 1024^2, 552 -> 468 us; a gradient of eight 256^2
+// samples, about 120 launches, 984 -> 836 us; a learned solve of five problems
+// 149 -> 139 ms.
 template <class... P>
 __device__ __forceinline__ void after_previous(P const*&... read)
 {
@@ -637,6 +639,7 @@ __global__ void __launch_bounds__(128, 4) conv3x3_kernel(const __grid_constant__
     ConvSmem& s = *reinterpret_cast<ConvSmem*>(smem_raw);
     int const tid = threadIdx.x;
     conv_setup(s, wt, nullptr, 32);
+    after_previous(in, in2, gin);
     uint32_t const tmem = s.tmem;
     uint32_t const halo_addr[2] = {smem_u32(s.halo[0]), smem_u32(s.halo[1])};
     uint64_t const b0 = umma_desc(smem_u32(s.w), kCh * 16, 128);
@@ -770,6 +773,7 @@ __global__ void __launch_bounds__(128) wgrad_kernel(const __grid_constant__ Tabl
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    after_previous(in, in2, dy, y);
     uint32_t const tmem = s.tmem;
     uint64_t const a0 = umma_desc(smem_u32(s.col), 128, kTilePx * 16), b0 = umma_desc(smem_u32(s.dz), 128, kTilePx * 16);
     uint32_t phase = 0;
@@ -865,6 +869,7 @@ __global__ void __launch_bounds__(128) wgrad_kernel(const __grid_constant__ Tabl
 __global__ void __launch_bounds__(256) reduce_parts_kernel(float const* part, int nparts, int n, float* grad)
 {
     __shared__ float red[8][32];
+    after_previous(part);
     int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int const i = blockIdx.x * 32 + lane;
     int const per = (nparts + 7) / 8, p1 = min(nparts, (warp + 1) * per);
@@ -995,6 +1000,7 @@ __global__ void __launch_bounds__(256) inc_forward_kernel(const __grid_constant_
 __global__ void __launch_bounds__(256) out_forward_kernel(const __grid_constant__ Table t, bf16 const* in,
                                                           float const* params, float* out)
 {
+    after_previous(in);
     __shared__ float w[kOutW + 1];
     __shared__ int64_t pre[kMaxImages + 1];
     for (int i = threadIdx.x; i < kOutW + 1; i += blockDim.x) w[i] = params[kOffOut + i];
@@ -1028,6 +1034,7 @@ __global__ void __launch_bounds__(256) out_forward_kernel(const __grid_constant_
 // Data gradient of the output convolution: dg[p][ci] = sum_tap du[p - tap] w[tap][ci].
 __global__ void out_backward_data_kernel(const __grid_constant__ Table t, float const* du, float const* params, float* dg)
 {
+    after_previous(du);
     int const im = blockIdx.y;
     if (im >= t.nimg) return;
     Img const o = t.img[im];
@@ -1093,6 +1100,7 @@ __global__ void __launch_bounds__(kThinBlock) out_wgrad_kernel(const __grid_cons
     constexpr int NV = kTaps + 1;
     __shared__ float win[3][kHalo + 2];
     __shared__ float red[kThinWarps * NV * 32];
+    after_previous(du, in);
     int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float acc[NV] = {};
     for (int tile = blockIdx.x; tile < t.tile_base[t.nimg]; tile += gridDim.x) {
@@ -1148,6 +1156,7 @@ __global__ void __launch_bounds__(kThinBlock) inc_wgrad_kernel(const __grid_cons
     constexpr int NV = 2 * kTaps + 1;
     __shared__ float2 win[3][kHalo + 2];
     __shared__ float red[kThinWarps * NV * 32];
+    after_previous(dh, h, feat);
     int const warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float acc[NV] = {};
     for (int tile = blockIdx.x; tile < t.tile_base[t.nimg]; tile += gridDim.x) {
@@ -1211,6 +1220,7 @@ __global__ void __launch_bounds__(kThinBlock) inc_wgrad_kernel(const __grid_cons
 // dfine[p] += 0.25 * dcoarse[parent(p)] (adjoint of the 2x2 average pool).
 __global__ void pool_adjoint_kernel(const __grid_constant__ Table t, float const* dcoarse, float* dfine)
 {
+    after_previous(dcoarse);
     // t.img: fine level; t.aux: coarse level
     int const im = blockIdx.y;
     if (im >= t.nimg) return;
@@ -1236,6 +1246,7 @@ __global__ void pool_adjoint_kernel(const __grid_constant__ Table t, float const
 // Adjoint of skip + up(coarse): dskip[p] += dx[p]; dcoarse[q] += sum of dx over q's children.
 __global__ void upadd_adjoint_skip_kernel(const __grid_constant__ Table t, float const* dx, float* dskip)
 {
+    after_previous(dx);
     int const im = blockIdx.y;
     if (im >= t.nimg) return;
     Img const f = t.img[im];
@@ -1257,6 +1268,7 @@ __global__ void upadd_adjoint_skip_kernel(const __grid_constant__ Table t, float
 
 __global__ void upadd_adjoint_coarse_kernel(const __grid_constant__ Table t, float const* dx, float* dcoarse)
 {
+    after_previous(dx);
     // t.img: coarse level; t.aux: fine level
     int const im = blockIdx.y;
     if (im >= t.nimg) return;
@@ -2119,13 +2131,13 @@ unsigned item_grid(int nitems, int kind)
 
 // Launch of a kernel that calls after_previous.
 template <class... P, class... A>
-cudaError_t launch_after(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A const&... args)
+cudaError_t launch_after(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, A const&... args)
 {
     cudaLaunchAttribute early {};
     early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     early.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -2146,7 +2158,8 @@ sil_status launch_conv(cudaStream_t st, Table const& t, int mode, bf16 const* in
     int const grid = conv_grid(t.tile_base[t.nimg], mode);
     if (mode == kPlain) SIL_CUDA_CHECK(launch_after(conv3x3_plain_kernel, grid, 128, conv_smem(mode), st, t, in, w,
                                                     dst, wout, err));
-    else conv3x3_kernel<<<grid, 128, conv_smem(mode), st>>>(t, mode, in, in2, gin, w, dst, err);
+    else SIL_CUDA_CHECK(launch_after(conv3x3_kernel, grid, 128, conv_smem(mode), st, t, mode, in, in2, gin, w, dst,
+                                     err));
     SIL_CUDA_CHECK(cudaGetLastError());
     return SIL_OK;
 }
@@ -2343,7 +2356,8 @@ sil_status net_forward(Net& net, Workspace& w, cudaStream_t st, bool keep)
     }
     if (keep) {
         Table const t = w.table(0, -1, false);
-        out_forward_kernel<<<walk_grid(t, 1, kWalkOut), 256, 0, st>>>(t, w.g[0].as<bf16>(), net.params, w.unet.as<float>());
+        SIL_CUDA_CHECK(launch_after(out_forward_kernel, walk_grid(t, 1, kWalkOut), 256, 0, st, t, w.g[0].as<bf16>(),
+                                    net.params, w.unet.as<float>()));
     } else {
         Table const td = dec_table(w, 0);
         if (td.nimg > 0)
@@ -2351,7 +2365,8 @@ sil_status net_forward(Net& net, Workspace& w, cudaStream_t st, bool keep)
                                         w.taps.as<float>(), top, net.params, w.unet.as<float>()));
         Table const t1 = deepest_table(w, 0);  // single-level images: no decoder
         if (t1.nimg > 0)
-            out_forward_kernel<<<walk_grid(t1, 1, kWalkOut), 256, 0, st>>>(t1, w.g[0].as<bf16>(), net.params, w.unet.as<float>());
+            SIL_CUDA_CHECK(launch_after(out_forward_kernel, walk_grid(t1, 1, kWalkOut), 256, 0, st, t1,
+                                        w.g[0].as<bf16>(), net.params, w.unet.as<float>()));
     }
     SIL_CUDA_CHECK(cudaGetLastError());
     return SIL_OK;
@@ -2399,8 +2414,10 @@ sil_status wgrad(Net& net, Workspace& w, cudaStream_t st, Table const& t, int mo
 {
     if (t.nimg == 0 || t.tile_base[t.nimg] == 0) return SIL_OK;
     int const grid = std::min(w.wgrad_grid, t.tile_base[t.nimg]);
-    wgrad_kernel<<<grid, 128, wgrad_smem(), st>>>(t, mode, in, in2, dy, y, w.wparts.as<float>(), net.error_flag);
-    reduce_parts_kernel<<<(kWgradParts + 31) / 32, 256, 0, st>>>(w.wparts.as<float>(), grid, kWgradParts, grad_out);
+    SIL_CUDA_CHECK(launch_after(wgrad_kernel, grid, 128, wgrad_smem(), st, t, mode, in, in2, dy, y,
+                                w.wparts.as<float>(), net.error_flag));
+    SIL_CUDA_CHECK(launch_after(reduce_parts_kernel, (kWgradParts + 31) / 32, 256, 0, st, w.wparts.as<float>(), grid,
+                                kWgradParts, grad_out));
     SIL_CUDA_CHECK(cudaGetLastError());
     return SIL_OK;
 }
@@ -2418,10 +2435,12 @@ sil_status net_backward(Net& net, Workspace& w, cudaStream_t st)
     Table const t0 = w.table(0, -1, false);
     int const thin_blocks = std::min(w.thin_grid, t0.tile_base[t0.nimg]);
     // output convolution
-    out_backward_data_kernel<<<image_grid(t0, 1, 0), 256, 0, st>>>(t0, w.gnet.as<float>(), net.params, w.dg[0].as<float>());
-    out_wgrad_kernel<<<thin_blocks, kThinBlock, 0, st>>>(t0, w.gnet.as<float>(), w.g[0].as<bf16>(), w.wparts.as<float>());
-    reduce_parts_kernel<<<(kOutW + 1 + 31) / 32, 256, 0, st>>>(w.wparts.as<float>(), thin_blocks, kOutW + 1,
-                                                                 net.grad + kOffOut);
+    SIL_CUDA_CHECK(launch_after(out_backward_data_kernel, image_grid(t0, 1, 0), 256, 0, st, t0, w.gnet.as<float>(),
+                                net.params, w.dg[0].as<float>()));
+    SIL_CUDA_CHECK(launch_after(out_wgrad_kernel, thin_blocks, kThinBlock, 0, st, t0, w.gnet.as<float>(),
+                                w.g[0].as<bf16>(), w.wparts.as<float>()));
+    SIL_CUDA_CHECK(launch_after(reduce_parts_kernel, (kOutW + 1 + 31) / 32, 256, 0, st, w.wparts.as<float>(),
+                                thin_blocks, kOutW + 1, net.grad + kOffOut));
     SIL_CUDA_CHECK(cudaGetLastError());
     // decoder, top-down
     for (int l = 0; l <= D - 2; ++l) {
@@ -2434,7 +2453,8 @@ sil_status net_backward(Net& net, Workspace& w, cudaStream_t st)
         s = launch_conv(st, t, kMasked, w.g[l].as<bf16>(), w.g[l].as<bf16>(), w.dg[l].as<float>(), big_wt(net, kDec, wl),
                         nullptr, 0, nullptr, w.dx[l].as<float>(), 0, err);
         if (s != SIL_OK) return s;
-        upadd_adjoint_skip_kernel<<<image_grid(t, 8, 0), 256, 0, st>>>(t, w.dx[l].as<float>(), w.dh[l].as<float>());
+        SIL_CUDA_CHECK(launch_after(upadd_adjoint_skip_kernel, image_grid(t, 8, 0), 256, 0, st, t, w.dx[l].as<float>(),
+                                    w.dh[l].as<float>()));
         // coarse part: table over level l+1 with aux = level l
         Table tc {};
         tc.nimg = t.nimg;
@@ -2442,14 +2462,16 @@ sil_status net_backward(Net& net, Workspace& w, cudaStream_t st)
             tc.img[k] = t.aux[k];
             tc.aux[k] = t.img[k];
         }
-        upadd_adjoint_coarse_kernel<<<image_grid(tc, 8, 0), 256, 0, st>>>(tc, w.dx[l].as<float>(), w.dg[l + 1].as<float>());
+        SIL_CUDA_CHECK(launch_after(upadd_adjoint_coarse_kernel, image_grid(tc, 8, 0), 256, 0, st, tc,
+                                    w.dx[l].as<float>(), w.dg[l + 1].as<float>()));
         SIL_CUDA_CHECK(cudaGetLastError());
     }
     // deepest level of each image: g = h
     for (int l = 0; l < D; ++l) {
         Table const t = deepest_table(w, l);
         if (t.nimg == 0) continue;
-        upadd_adjoint_skip_kernel<<<image_grid(t, 8, 0), 256, 0, st>>>(t, w.dg[l].as<float>(), w.dh[l].as<float>());
+        SIL_CUDA_CHECK(launch_after(upadd_adjoint_skip_kernel, image_grid(t, 8, 0), 256, 0, st, t, w.dg[l].as<float>(),
+                                    w.dh[l].as<float>()));
         SIL_CUDA_CHECK(cudaGetLastError());
     }
     // encoder, bottom-up
@@ -2476,14 +2498,15 @@ sil_status net_backward(Net& net, Workspace& w, cudaStream_t st)
             tf.img[k] = tp.aux[k];   // fine level l-1
             tf.aux[k] = tp.img[k];   // coarse level l
         }
-        pool_adjoint_kernel<<<image_grid(tf, 8, 0), 256, 0, st>>>(tf, w.dg[l].as<float>(), w.dh[l - 1].as<float>());
+        SIL_CUDA_CHECK(launch_after(pool_adjoint_kernel, image_grid(tf, 8, 0), 256, 0, st, tf, w.dg[l].as<float>(),
+                                    w.dh[l - 1].as<float>()));
         SIL_CUDA_CHECK(cudaGetLastError());
     }
     // input convolution
-    inc_wgrad_kernel<<<thin_blocks, kThinBlock, 0, st>>>(t0, w.dh[0].as<float>(), w.h[0].as<bf16>(), w.feat.as<float>(),
-                                                         w.wparts.as<float>());
-    reduce_parts_kernel<<<(kInW + kCh + 31) / 32, 256, 0, st>>>(w.wparts.as<float>(), thin_blocks, kInW + kCh,
-                                                                  net.grad + kOffIn);
+    SIL_CUDA_CHECK(launch_after(inc_wgrad_kernel, thin_blocks, kThinBlock, 0, st, t0, w.dh[0].as<float>(),
+                                w.h[0].as<bf16>(), w.feat.as<float>(), w.wparts.as<float>()));
+    SIL_CUDA_CHECK(launch_after(reduce_parts_kernel, (kInW + kCh + 31) / 32, 256, 0, st, w.wparts.as<float>(),
+                                thin_blocks, kInW + kCh, net.grad + kOffIn));
     SIL_CUDA_CHECK(cudaGetLastError());
     return SIL_OK;
 }
