@@ -2165,6 +2165,12 @@ sil_status build_divergence_gauge(ProblemDesc const& q, ProbInfo const& pi, doub
     return SIL_OK;
 }
 
+// Dynamic shared memory of the resident kernel at most: the 227 KB a CTA can
+// have less its static part.  Every launch allows its instance this much: the
+// attribute belongs to the kernel and the device, not to the call, so a smaller
+// value of one host thread would refuse another's launch of the same instance.
+constexpr size_t kResSmemMost = 226 * 1024;
+
 // Shared memory of the resident kernel with m nodes per thread, and the rows a
 // CTA can hold of an nx-wide grid.
 template <class T>
@@ -2175,8 +2181,7 @@ size_t resident_smem(int m, int64_t nx)
 template <class T>
 int64_t resident_rows(int64_t nx)
 {
-    constexpr size_t most = 226 * 1024;   // of the 227 KB a CTA can have, less the static part
-    return resident_smem<T>(kResMaxPerThread<T>, nx) <= most ? kResThreads * kResMaxPerThread<T> / nx : 0;
+    return resident_smem<T>(kResMaxPerThread<T>, nx) <= kResSmemMost ? kResThreads * kResMaxPerThread<T> / nx : 0;
 }
 
 // The kernel's instances by nodes per thread.
@@ -2812,7 +2817,7 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
         for (ResidentWave const& w : waves) {
             void const* const kernel = resident_kernel<T>(w.per_thread);
             SIL_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                static_cast<int>(w.smem)));
+                                                static_cast<int>(kResSmemMost)));
             ResidentCta const* ctas = d_res + at;
             double tol2 = tol * tol;
             int budget = max_iter, steps = chunk, polls = kResPollLimit;
