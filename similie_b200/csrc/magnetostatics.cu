@@ -1703,7 +1703,7 @@ template <class T, int M>
 __global__ void __launch_bounds__(kResThreads, 1)
         cg_resident_kernel(ResidentCta const* ctas, Vecs<T> const* vecs, double const* const* nu64,
                            double const* const* rhs, double* const* x64, double* const* r64, Scalars* sc,
-                           unsigned long long* mail, double tol2, int max_iter, int chunk, int poll_limit)
+                           unsigned long long* mail, double tol2, int max_iter, int spent, int chunk, int poll_limit)
 {
     constexpr int kNodes = M * kResThreads;
     extern __shared__ __align__(16) unsigned char res_smem[];
@@ -1860,7 +1860,8 @@ __global__ void __launch_bounds__(kResThreads, 1)
             outer = 1;
             break;
         }
-        if (static_cast<int64_t>(cycles) * chunk >= max_iter) break;
+        // the batch's budget, of which an earlier stage has used `spent`
+        if (spent + static_cast<int64_t>(cycles) * chunk >= max_iter) break;
         double const inner_tol2 = 0.25 * tol2 * bb / fmax(tot, 1e-300);
         // residual replacement (cg_replace_kernel)
         double rz = 0.0, rr = 0.0;
@@ -2820,8 +2821,8 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
                                                 static_cast<int>(kResSmemMost)));
             ResidentCta const* ctas = d_res + at;
             double tol2 = tol * tol;
-            int budget = max_iter, steps = chunk, polls = kResPollLimit;
-            void* args[] = {&ctas, &d_vecs, &d_nu64, &d_rhs, &d_x64, &d_r64, &d_sc, &d_mail, &tol2, &budget, &steps, &polls};
+            int budget = max_iter, spent = total, steps = chunk, polls = kResPollLimit;
+            void* args[] = {&ctas, &d_vecs, &d_nu64, &d_rhs, &d_x64, &d_r64, &d_sc, &d_mail, &tol2, &budget, &spent, &steps, &polls};
             SIL_CUDA_CHECK(cudaLaunchCooperativeKernel(kernel, dim3(static_cast<unsigned>(w.ctas.size())),
                                                        dim3(kResThreads), args, w.smem, stream));
             at += w.ctas.size();
