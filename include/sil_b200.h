@@ -309,6 +309,21 @@ sil_status sil_mag2d_solve_batch(const sil_mag2d_problem* problems, int nproblem
                                  const sil_solve_settings* settings, sil_solve_diagnostics* diag,
                                  sil_stream stream);
 
+/* What a 2D solve may use of the GPU for its on-chip part: problems that fit
+ * the multiprocessors' memory are solved there in one cooperative launch, the
+ * others by kernels per iteration. */
+typedef struct sil_chip_limits {
+    int32_t blocks;        /* blocks of a launch: -1 one per multiprocessor, 0 nothing on chip, 256 at most */
+    int32_t solved;        /* written: problems whose plain solve ran on chip */
+} sil_chip_limits;
+
+/* sil_mag2d_solve_batch within limits, for callers that leave a part of the
+ * GPU to other work and for the tests of either path; no counterpart in the
+ * reference. */
+sil_status sil_mag2d_solve_batch_within(sil_chip_limits* limits, const sil_mag2d_problem* problems, int nproblems,
+                                        const sil_solve_settings* settings, sil_solve_diagnostics* diag,
+                                        sil_stream stream);
+
 /* ---------------------------------------------------------------------- */
 /* 2D magnetostatics with a nonlinear (saturating) ferromagnetic material.  */
 /* A node whose ferromagnetic fraction (share of adjacent cells made of the */

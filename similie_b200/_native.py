@@ -145,6 +145,13 @@ class SilSolveDiagnostics(ctypes.Structure):
     ]
 
 
+class SilChipLimits(ctypes.Structure):
+    _fields_ = [
+        ("blocks", ctypes.c_int32),
+        ("solved", ctypes.c_int32),
+    ]
+
+
 class SilError(RuntimeError):
     def __init__(self, status, message):
         super().__init__(f"{STATUS_NAMES.get(status, status)}: {message}")
@@ -192,6 +199,9 @@ SIGNATURES = [
     ("sil_mag2d_solve_batch", ctypes.c_int, [ctypes.POINTER(SilMag2dProblem), ctypes.c_int,
                                              ctypes.POINTER(SilSolveSettings),
                                              ctypes.POINTER(SilSolveDiagnostics), _P]),
+    ("sil_mag2d_solve_batch_within", ctypes.c_int, [ctypes.POINTER(SilChipLimits), ctypes.POINTER(SilMag2dProblem),
+                                                    ctypes.c_int, ctypes.POINTER(SilSolveSettings),
+                                                    ctypes.POINTER(SilSolveDiagnostics), _P]),
     ("sil_fill_discrete_hodge_star_metric", ctypes.c_int, [_P, ctypes.c_int, ctypes.c_int, _F, _F, _F]),
     ("sil_hodge_star_stored", ctypes.c_int, [_P, ctypes.c_int, ctypes.c_int, _F, _F, _F]),
     ("sil_precond_num_params", ctypes.c_int64, []),

@@ -2316,9 +2316,17 @@ void const* resident_kernel(int per_thread)
     }
 }
 
+// Blocks the resident solve may take: one per multiprocessor, or the caller's
+// limit (a lane polls kMailPerLane of a group's slots).
+int chip_blocks(sil_chip_limits const& limits)
+{
+    return limits.blocks < 0 ? sm_count() : std::min(limits.blocks, 32 * kMailPerLane);
+}
+
 template <class T>
 sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_settings const& set,
-                            sil_solve_diagnostics* diag, cudaStream_t stream, nn::Net* learned, int item_rows)
+                            sil_solve_diagnostics* diag, cudaStream_t stream, nn::Net* learned,
+                            sil_chip_limits& limits, int item_rows)
 {
     int const np = static_cast<int>(probs.size());
     // Work items: contiguous row ranges of item_rows rows per problem (3D:
@@ -2398,7 +2406,7 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
     int const nparts = std::max(std::max(nitems, ntiles), nstrip_ctas);
     // 2D problems that fit on chip are solved there; the others by the kernels
     // per iteration.
-    std::vector<ResidentWave> const waves = flat ? plan_resident<T>(probs, sm_count()) : std::vector<ResidentWave> {};
+    std::vector<ResidentWave> const waves = flat ? plan_resident<T>(probs, chip_blocks(limits)) : std::vector<ResidentWave> {};
     size_t nres = 0;
     std::vector<char> resident(np, 0);
     for (ResidentWave const& w : waves) {
@@ -2857,6 +2865,7 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
         }
         resident_cycles = cycles;
     }
+    limits.solved = static_cast<int>(std::count(resident.begin(), resident.end(), 1));
     // Cycle: FP64 residual (outer check) -> residual replacement -> a chunk
     // of iterations -> x64 += ||r|| x; the host reads the problems' state
     // once per cycle.
@@ -2945,7 +2954,7 @@ int g_item_rows_tuned[4] = {0, 0, 0, 0};  // [precision FP64 / FP32][first probl
 
 template <class T>
 sil_status choose_item_rows(std::vector<ProblemDesc> const& probs, sil_solve_settings const& set, cudaStream_t stream,
-                            int* rows)
+                            sil_chip_limits const& limits, int* rows)
 {
     int64_t total = 0;
     for (ProblemDesc const& q : probs) total += (q.dim == 3 ? 3 : 1) * q.nx * q.ny * (q.dim == 3 ? q.nz : 1);
@@ -2962,7 +2971,8 @@ sil_status choose_item_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
         }
     }
     if (total < (int64_t(1) << 22)) return SIL_OK;
-    if (std::all_of(probs.begin(), probs.end(), [](ProblemDesc const& q) { return resident_ctas<T>(q, sm_count()) > 0; }))
+    int const blocks = chip_blocks(limits);
+    if (std::all_of(probs.begin(), probs.end(), [&](ProblemDesc const& q) { return resident_ctas<T>(q, blocks) > 0; }))
         return SIL_OK;   // solved on chip
     int const key = (sizeof(T) == 8 ? 0 : 2) + (probs.front().dim == 3 ? 1 : 0);
     {
@@ -2981,7 +2991,8 @@ sil_status choose_item_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
     int best_rows = kItemNodes;
     for (int c : kItemCandidates) {
         auto const t0 = std::chrono::steady_clock::now();
-        sil_status const st = solve_batch_rows<T>(probs, probe, scratch.data(), stream, nullptr, c);
+        sil_chip_limits within = limits;
+        sil_status const st = solve_batch_rows<T>(probs, probe, scratch.data(), stream, nullptr, within, c);
         if (st != SIL_OK) return st;
         double const sec = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
         if (sec < best) {
@@ -2997,12 +3008,12 @@ sil_status choose_item_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
 
 template <class T>
 sil_status solve_batch(std::vector<ProblemDesc> const& probs, sil_solve_settings const& set, sil_solve_diagnostics* diag,
-                       cudaStream_t stream, nn::Net* learned = nullptr)
+                       cudaStream_t stream, sil_chip_limits& limits, nn::Net* learned = nullptr)
 {
     int rows = kItemNodes;
-    sil_status const st = choose_item_rows<T>(probs, set, stream, &rows);
+    sil_status const st = choose_item_rows<T>(probs, set, stream, limits, &rows);
     if (st != SIL_OK) return st;
-    return solve_batch_rows<T>(probs, set, diag, stream, learned, rows);
+    return solve_batch_rows<T>(probs, set, diag, stream, learned, limits, rows);
 }
 
 } // namespace
@@ -3100,6 +3111,17 @@ sil_status sil_mag2d_apply_noalloc(sil_stream stream, int64_t nx, int64_t ny, co
 sil_status sil_mag2d_solve_batch(const sil_mag2d_problem* problems, int nproblems, const sil_solve_settings* settings,
                                  sil_solve_diagnostics* diag, sil_stream stream)
 {
+    sil_chip_limits limits = {-1, 0};
+    return sil_mag2d_solve_batch_within(&limits, problems, nproblems, settings, diag, stream);
+}
+
+sil_status sil_mag2d_solve_batch_within(sil_chip_limits* limits, const sil_mag2d_problem* problems, int nproblems,
+                                        const sil_solve_settings* settings, sil_solve_diagnostics* diag,
+                                        sil_stream stream)
+{
+    if (limits == nullptr || limits->blocks < -1)
+        return fail(SIL_ERR_INVALID, "sil_mag2d_solve_batch_within: NULL limits or bad block count");
+    limits->solved = 0;
     if (problems == nullptr || settings == nullptr || diag == nullptr || nproblems < 1)
         return fail(SIL_ERR_INVALID, "sil_mag2d_solve_batch: NULL argument or empty batch");
     std::vector<ProblemDesc> descs(nproblems);
@@ -3114,14 +3136,14 @@ sil_status sil_mag2d_solve_batch(const sil_mag2d_problem* problems, int nproblem
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     std::memset(diag, 0, sizeof(sil_solve_diagnostics) * nproblems);
-    if (settings->solver == SIL_SOLVER_CG_F64) return solve_batch<double>(descs, *settings, diag, s);
-    if (settings->solver == SIL_SOLVER_MIXED_IR) return solve_batch<float>(descs, *settings, diag, s);
+    if (settings->solver == SIL_SOLVER_CG_F64) return solve_batch<double>(descs, *settings, diag, s, *limits);
+    if (settings->solver == SIL_SOLVER_MIXED_IR) return solve_batch<float>(descs, *settings, diag, s, *limits);
     if (settings->solver == SIL_SOLVER_LEARNED) {
         if (settings->preconditioner == nullptr)
             return fail(SIL_ERR_INVALID, "sil_mag2d_solve_batch: the learned solver needs a preconditioner");
         if (nproblems > nn::kMaxImages)
             return fail(SIL_ERR_INVALID, "sil_mag2d_solve_batch: the learned solver takes at most 64 problems per call");
-        return solve_batch<float>(descs, *settings, diag, s, &settings->preconditioner->net);
+        return solve_batch<float>(descs, *settings, diag, s, *limits, &settings->preconditioner->net);
     }
     return fail(SIL_ERR_INVALID, "sil_mag2d_solve_batch: unknown solver kind");
 }
@@ -3403,8 +3425,9 @@ sil_status sil_mag3d_solve_batch(const sil_mag3d_problem* problems, int nproblem
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     std::memset(diag, 0, sizeof(sil_solve_diagnostics) * nproblems);
-    if (settings->solver == SIL_SOLVER_CG_F64) return solve_batch<double>(descs, *settings, diag, s);
-    if (settings->solver == SIL_SOLVER_MIXED_IR) return solve_batch<float>(descs, *settings, diag, s);
+    sil_chip_limits none = {0, 0};   // nothing of a 3D solve runs on chip
+    if (settings->solver == SIL_SOLVER_CG_F64) return solve_batch<double>(descs, *settings, diag, s, none);
+    if (settings->solver == SIL_SOLVER_MIXED_IR) return solve_batch<float>(descs, *settings, diag, s, none);
     return fail(SIL_ERR_INVALID, "sil_mag3d_solve_batch: unknown solver kind (the learned solver is 2D only)");
 }
 

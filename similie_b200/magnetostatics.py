@@ -145,6 +145,27 @@ def solve_batch(mus, rhss, sols, shapes, solver="cg", tol=1e-10, max_iterations=
     `flexible_directions` (1..16) A-orthogonal directions, then the mixed
     solver for problems whose preconditioned residual stalls).
     Returns one Diagnostics per problem."""
+    return _solve_batch(None, mus, rhss, sols, shapes, solver, tol, max_iterations, inner_iterations, inner_tolerance,
+                        stream, preconditioner, stall_window, flexible_directions)
+
+
+@dataclass
+class ChipLimits:
+    """What a solve may use of the GPU for its on-chip part (sil_chip_limits)."""
+    blocks: int = -1   # blocks of a launch: -1 one per multiprocessor, 0 nothing on chip, 256 at most
+    solved: int = 0    # written: problems whose plain solve ran on chip
+
+
+def solve_batch_within(limits, mus, rhss, sols, shapes, solver="cg", tol=1e-10, max_iterations=200000,
+                       inner_iterations=4000, inner_tolerance=1e-4, stream=None, preconditioner=None, stall_window=200,
+                       flexible_directions=8):
+    """solve_batch within `limits`, a ChipLimits, for callers that leave a part of the GPU to other work."""
+    return _solve_batch(limits, mus, rhss, sols, shapes, solver, tol, max_iterations, inner_iterations,
+                        inner_tolerance, stream, preconditioner, stall_window, flexible_directions)
+
+
+def _solve_batch(limits, mus, rhss, sols, shapes, solver, tol, max_iterations, inner_iterations, inner_tolerance,
+                 stream, preconditioner, stall_window, flexible_directions):
     import torch
     n = len(shapes)
     probs = (_native.SilMag2dProblem * n)()
@@ -165,7 +186,12 @@ def solve_batch(mus, rhss, sols, shapes, solver="cg", tol=1e-10, max_iterations=
         st.preconditioner = preconditioner._h.value
     diag = (_native.SilSolveDiagnostics * n)()
     s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream if stream is None else stream)
-    rc = lib().sil_mag2d_solve_batch(probs, n, ctypes.byref(st), diag, s)
+    if limits is None:
+        rc = lib().sil_mag2d_solve_batch(probs, n, ctypes.byref(st), diag, s)
+    else:
+        lim = _native.SilChipLimits(limits.blocks)
+        rc = lib().sil_mag2d_solve_batch_within(ctypes.byref(lim), probs, n, ctypes.byref(st), diag, s)
+        limits.solved = lim.solved
     out = [Diagnostics(d.iterations, bool(d.converged), d.refinements, d.status, d.initial_residual_l2,
                        d.final_residual_l2, d.final_relative_residual, d.learned_iterations, bool(d.fallback))
            for d in diag]
