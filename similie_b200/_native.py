@@ -149,6 +149,7 @@ class SilChipLimits(ctypes.Structure):
     _fields_ = [
         ("blocks", ctypes.c_int32),
         ("solved", ctypes.c_int32),
+        ("handed_over", ctypes.c_int32),
     ]
 
 

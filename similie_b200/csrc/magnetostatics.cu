@@ -2846,14 +2846,22 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
         size_t at = 0;
         for (ResidentWave const& w : waves) {
             void const* const kernel = resident_kernel<T>(w.per_thread);
-            SIL_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                static_cast<int>(kResSmemMost)));
             ResidentCta const* ctas = d_res + at;
             double tol2 = tol * tol;
             int budget = max_iter, spent = total, steps = chunk, polls = kResPollLimit;
             void* args[] = {&ctas, &d_vecs, &d_nu64, &d_rhs, &d_x64, &d_r64, &d_sc, &d_mail, &tol2, &budget, &spent, &steps, &polls};
-            SIL_CUDA_CHECK(cudaLaunchCooperativeKernel(kernel, dim3(static_cast<unsigned>(w.ctas.size())),
-                                                       dim3(kResThreads), args, w.smem, stream));
+            cudaError_t refused = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       static_cast<int>(kResSmemMost));
+            if (refused == cudaSuccess)
+                refused = cudaLaunchCooperativeKernel(kernel, dim3(static_cast<unsigned>(w.ctas.size())),
+                                                      dim3(kResThreads), args, w.smem, stream);
+            if (refused != cudaSuccess) {
+                // not run: the kernels per iteration take its problems (an error
+                // that outlasts the launch comes back from the next call)
+                cudaGetLastError();
+                for (int p : w.probs) resident[p] = 0;
+                limits.handed_over += static_cast<int>(w.probs.size());
+            }
             at += w.ctas.size();
         }
         st = read_scalars();
@@ -3111,7 +3119,7 @@ sil_status sil_mag2d_apply_noalloc(sil_stream stream, int64_t nx, int64_t ny, co
 sil_status sil_mag2d_solve_batch(const sil_mag2d_problem* problems, int nproblems, const sil_solve_settings* settings,
                                  sil_solve_diagnostics* diag, sil_stream stream)
 {
-    sil_chip_limits limits = {-1, 0};
+    sil_chip_limits limits = {-1, 0, 0};
     return sil_mag2d_solve_batch_within(&limits, problems, nproblems, settings, diag, stream);
 }
 
@@ -3121,7 +3129,7 @@ sil_status sil_mag2d_solve_batch_within(sil_chip_limits* limits, const sil_mag2d
 {
     if (limits == nullptr || limits->blocks < -1)
         return fail(SIL_ERR_INVALID, "sil_mag2d_solve_batch_within: NULL limits or bad block count");
-    limits->solved = 0;
+    limits->solved = limits->handed_over = 0;
     if (problems == nullptr || settings == nullptr || diag == nullptr || nproblems < 1)
         return fail(SIL_ERR_INVALID, "sil_mag2d_solve_batch: NULL argument or empty batch");
     std::vector<ProblemDesc> descs(nproblems);
@@ -3425,7 +3433,7 @@ sil_status sil_mag3d_solve_batch(const sil_mag3d_problem* problems, int nproblem
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     std::memset(diag, 0, sizeof(sil_solve_diagnostics) * nproblems);
-    sil_chip_limits none = {0, 0};   // nothing of a 3D solve runs on chip
+    sil_chip_limits none = {0, 0, 0};   // nothing of a 3D solve runs on chip
     if (settings->solver == SIL_SOLVER_CG_F64) return solve_batch<double>(descs, *settings, diag, s, none);
     if (settings->solver == SIL_SOLVER_MIXED_IR) return solve_batch<float>(descs, *settings, diag, s, none);
     return fail(SIL_ERR_INVALID, "sil_mag3d_solve_batch: unknown solver kind (the learned solver is 2D only)");

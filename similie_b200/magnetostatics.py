@@ -154,6 +154,7 @@ class ChipLimits:
     """What a solve may use of the GPU for its on-chip part (sil_chip_limits)."""
     blocks: int = -1   # blocks of a launch: -1 one per multiprocessor, 0 nothing on chip, 256 at most
     solved: int = 0    # written: problems whose plain solve ran on chip
+    handed_over: int = 0   # written: problems meant for the chip whose launch the device refused
 
 
 def solve_batch_within(limits, mus, rhss, sols, shapes, solver="cg", tol=1e-10, max_iterations=200000,
@@ -191,7 +192,7 @@ def _solve_batch(limits, mus, rhss, sols, shapes, solver, tol, max_iterations, i
     else:
         lim = _native.SilChipLimits(limits.blocks)
         rc = lib().sil_mag2d_solve_batch_within(ctypes.byref(lim), probs, n, ctypes.byref(st), diag, s)
-        limits.solved = lim.solved
+        limits.solved, limits.handed_over = lim.solved, lim.handed_over
     out = [Diagnostics(d.iterations, bool(d.converged), d.refinements, d.status, d.initial_residual_l2,
                        d.final_residual_l2, d.final_relative_residual, d.learned_iterations, bool(d.fallback))
            for d in diag]

@@ -1,0 +1,29 @@
+"""When the on-chip part of a 2D solve cannot run, the kernels per iteration solve its problems.
+
+The launch is refused here by planning for more blocks than the device can hold at once: two grids of 800 x 800
+nodes take 100 blocks of 7,168 FP64 nodes each, one to a multiprocessor, in one cooperative launch of 200, which
+the runtime answers with an error before anything runs.
+"""
+import numpy as np
+import pytest
+
+from test_gpu_mag2d_steps import _batch, _check, _solve
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+def test_refused_launch():
+    shapes = [(800, 800), (800, 800), (64, 48)]
+    mus, rhss = _batch(shapes, 13)
+    sols, diag, limits = _solve(shapes, mus, rhss, blocks=256, solver="cg", tol=1e-8)
+    assert limits.handed_over == len(shapes) and limits.solved == 0
+    _check(shapes, mus, rhss, sols, diag, 1e-8)
+    want, _, _ = _solve(shapes, mus, rhss, blocks=0, solver="cg", tol=1e-8)
+    for a, b in zip(sols, want):
+        np.testing.assert_array_equal(a, b)
+    # and the device still takes what fits it
+    sols, diag, limits = _solve(shapes, mus, rhss, blocks=-1, solver="cg", tol=1e-8)
+    assert limits.handed_over == 0 and limits.solved == len(shapes)
+    _check(shapes, mus, rhss, sols, diag, 1e-8)
