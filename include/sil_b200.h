@@ -314,9 +314,12 @@ sil_status sil_mag2d_solve_batch(const sil_mag2d_problem* problems, int nproblem
  * others by kernels per iteration. */
 typedef struct sil_chip_limits {
     int32_t blocks;        /* blocks of a launch: -1 one per multiprocessor, 0 nothing on chip, 256 at most */
+    int32_t wait_polls;    /* bound of each wait of a block for the others of its problem, in polls (-1: the
+                            * default, 4,194,304; 0: every wait runs out at once) */
     int32_t solved;        /* written: problems whose plain solve ran on chip */
     int32_t handed_over;   /* written: problems meant for the chip that the kernels per iteration took, as the
-                            * device refused the launch (a process may have fewer multiprocessors than the device) */
+                            * device refused the launch (a process may have fewer multiprocessors than the
+                            * device) or a wait ran out */
 } sil_chip_limits;
 
 /* sil_mag2d_solve_batch within limits, for callers that leave a part of the

@@ -148,6 +148,7 @@ class SilSolveDiagnostics(ctypes.Structure):
 class SilChipLimits(ctypes.Structure):
     _fields_ = [
         ("blocks", ctypes.c_int32),
+        ("wait_polls", ctypes.c_int32),
         ("solved", ctypes.c_int32),
         ("handed_over", ctypes.c_int32),
     ]

@@ -1772,7 +1772,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
             // this lane's share of the mail, all of it asked for at once
             unsigned long long wa[kMailPerLane], wb[kMailPerLane];
             int tries = 0;
-            bool lost = false, waiting = true;
+            bool lost = poll_limit == 0, waiting = !lost;
 #pragma unroll
             for (int u = 0; u < kMailPerLane; ++u) wa[u] = wb[u] = tid + 32 * u < c.group ? kNoMail : 0ull;
             while (waiting) {
@@ -1785,7 +1785,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
                 }
 #pragma unroll
                 for (int u = 0; u < kMailPerLane; ++u) waiting = waiting || wa[u] == kNoMail || (kBoth && wb[u] == kNoMail);
-                if (waiting && ++tries > poll_limit) {
+                if (waiting && ++tries >= poll_limit) {
                     lost = true;
                     break;
                 }
@@ -2848,7 +2848,8 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
             void const* const kernel = resident_kernel<T>(w.per_thread);
             ResidentCta const* ctas = d_res + at;
             double tol2 = tol * tol;
-            int budget = max_iter, spent = total, steps = chunk, polls = kResPollLimit;
+            int budget = max_iter, spent = total, steps = chunk;
+            int polls = limits.wait_polls < 0 ? kResPollLimit : limits.wait_polls;
             void* args[] = {&ctas, &d_vecs, &d_nu64, &d_rhs, &d_x64, &d_r64, &d_sc, &d_mail, &tol2, &budget, &spent, &steps, &polls};
             cudaError_t refused = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                        static_cast<int>(kResSmemMost));
@@ -2868,8 +2869,13 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
         if (st != SIL_OK) return st;
         int cycles = 0;
         for (int p = 0; p < np; ++p) {
-            if (hs[p].timeout) return fail(SIL_ERR_BUDGET, "resident solve: a wait for the group's other blocks ran out");
             cycles = std::max(cycles, hs[p].cycles);
+            if (!resident[p] || !hs[p].timeout || hs[p].outer_done) continue;
+            // A wait ran out (the group's blocks were kept from running for
+            // seconds): the kernels per iteration go on from its x64, of whose
+            // rows some may hold a correction that the others still lack.
+            resident[p] = 0;
+            ++limits.handed_over;
         }
         resident_cycles = cycles;
     }
@@ -3119,7 +3125,7 @@ sil_status sil_mag2d_apply_noalloc(sil_stream stream, int64_t nx, int64_t ny, co
 sil_status sil_mag2d_solve_batch(const sil_mag2d_problem* problems, int nproblems, const sil_solve_settings* settings,
                                  sil_solve_diagnostics* diag, sil_stream stream)
 {
-    sil_chip_limits limits = {-1, 0, 0};
+    sil_chip_limits limits = {-1, -1, 0, 0};
     return sil_mag2d_solve_batch_within(&limits, problems, nproblems, settings, diag, stream);
 }
 
@@ -3127,8 +3133,8 @@ sil_status sil_mag2d_solve_batch_within(sil_chip_limits* limits, const sil_mag2d
                                         const sil_solve_settings* settings, sil_solve_diagnostics* diag,
                                         sil_stream stream)
 {
-    if (limits == nullptr || limits->blocks < -1)
-        return fail(SIL_ERR_INVALID, "sil_mag2d_solve_batch_within: NULL limits or bad block count");
+    if (limits == nullptr || limits->blocks < -1 || limits->wait_polls < -1)
+        return fail(SIL_ERR_INVALID, "sil_mag2d_solve_batch_within: NULL or bad limits");
     limits->solved = limits->handed_over = 0;
     if (problems == nullptr || settings == nullptr || diag == nullptr || nproblems < 1)
         return fail(SIL_ERR_INVALID, "sil_mag2d_solve_batch: NULL argument or empty batch");
@@ -3433,7 +3439,7 @@ sil_status sil_mag3d_solve_batch(const sil_mag3d_problem* problems, int nproblem
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     std::memset(diag, 0, sizeof(sil_solve_diagnostics) * nproblems);
-    sil_chip_limits none = {0, 0, 0};   // nothing of a 3D solve runs on chip
+    sil_chip_limits none = {0, 0, 0, 0};   // nothing of a 3D solve runs on chip
     if (settings->solver == SIL_SOLVER_CG_F64) return solve_batch<double>(descs, *settings, diag, s, none);
     if (settings->solver == SIL_SOLVER_MIXED_IR) return solve_batch<float>(descs, *settings, diag, s, none);
     return fail(SIL_ERR_INVALID, "sil_mag3d_solve_batch: unknown solver kind (the learned solver is 2D only)");

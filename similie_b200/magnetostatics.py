@@ -152,9 +152,11 @@ def solve_batch(mus, rhss, sols, shapes, solver="cg", tol=1e-10, max_iterations=
 @dataclass
 class ChipLimits:
     """What a solve may use of the GPU for its on-chip part (sil_chip_limits)."""
-    blocks: int = -1   # blocks of a launch: -1 one per multiprocessor, 0 nothing on chip, 256 at most
-    solved: int = 0    # written: problems whose plain solve ran on chip
-    handed_over: int = 0   # written: problems meant for the chip whose launch the device refused
+    blocks: int = -1       # blocks of a launch: -1 one per multiprocessor, 0 nothing on chip, 256 at most
+    wait_polls: int = -1   # bound of a wait between blocks, in polls (-1: the default; 0: it runs out at once)
+    solved: int = 0        # written: problems whose plain solve ran on chip
+    handed_over: int = 0   # written: problems meant for the chip that the kernels per iteration took (the launch was
+                           # refused, or a wait ran out)
 
 
 def solve_batch_within(limits, mus, rhss, sols, shapes, solver="cg", tol=1e-10, max_iterations=200000,
@@ -190,7 +192,7 @@ def _solve_batch(limits, mus, rhss, sols, shapes, solver, tol, max_iterations, i
     if limits is None:
         rc = lib().sil_mag2d_solve_batch(probs, n, ctypes.byref(st), diag, s)
     else:
-        lim = _native.SilChipLimits(limits.blocks)
+        lim = _native.SilChipLimits(limits.blocks, limits.wait_polls)
         rc = lib().sil_mag2d_solve_batch_within(ctypes.byref(lim), probs, n, ctypes.byref(st), diag, s)
         limits.solved, limits.handed_over = lim.solved, lim.handed_over
     out = [Diagnostics(d.iterations, bool(d.converged), d.refinements, d.status, d.initial_residual_l2,

@@ -18,9 +18,9 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 
-def _solve(shapes, mus, rhss, blocks=0, **kw):
+def _solve(shapes, mus, rhss, blocks=0, wait_polls=-1, **kw):
     from similie_b200 import magnetostatics as m2
-    limits = m2.ChipLimits(blocks)
+    limits = m2.ChipLimits(blocks, wait_polls)
     sols = [torch.full((len(b),), float("nan"), device="cuda", dtype=torch.float64) for b in rhss]
     diag = m2.solve_batch_within(limits, [torch.from_numpy(m).cuda() for m in mus],
                                  [torch.from_numpy(b).cuda() for b in rhss], sols, shapes, **kw)
@@ -78,6 +78,8 @@ def test_limits_are_checked():
 
     import similie_b200 as sil
     from similie_b200 import _native
-    lim = _native.SilChipLimits(-2)
-    assert sil.lib().sil_mag2d_solve_batch_within(ctypes.byref(lim), None, 0, None, None, None) == 1
+    for bad in ((-2, -1), (-1, -2)):
+        lim = _native.SilChipLimits(*bad)
+        assert sil.lib().sil_mag2d_solve_batch_within(ctypes.byref(lim), None, 0, None, None, None) == 1
+        assert b"limits" in sil.lib().sil_last_error()
     assert sil.lib().sil_mag2d_solve_batch_within(None, None, 0, None, None, None) == 1
