@@ -911,6 +911,10 @@ Dense<T, N> dense_args(Geometry const* geo, sil_field const& in, sil_field const
     return a;
 }
 
+// Dynamic shared memory a kernel may take without asking for it, so that the
+// marching launches have no call that can fail before them.
+constexpr size_t kPlainSmem = 48 * 1024;
+
 // Planes per run: `columns` tiles of `length` planes over `resident` CTAs at a
 // time, a run of n planes costing n + 2 steps: the cheapest total of whole waves.
 int run_length(int64_t columns, int64_t length, int64_t resident)
@@ -963,9 +967,8 @@ template <class T, int K>
 bool launch_lap3(cudaStream_t stream, Dense<T, 3> const& a)
 {
     constexpr size_t smem = sizeof(Lap3Smem<T, K, kLap3Y>);
+    static_assert(smem <= kPlainSmem);
     auto const kernel = lap3_march_kernel<T, K, kLap3Y, kLap3Ctas<T, K>>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-        return false;
     int const tz = (a.oext[2] + kMarchZ - 3) / (kMarchZ - 2), ty = (a.oext[1] + kLap3Y - 3) / (kLap3Y - 2);
     int64_t const columns = static_cast<int64_t>(tz) * ty;
     int const planes = run_length(columns, a.oext[0], static_cast<int64_t>(kLap3Ctas<T, K>) * multiprocessors());
@@ -1000,9 +1003,8 @@ template <class T, int K>
 bool launch_codiff3(cudaStream_t stream, Dense<T, 3> const& a)
 {
     constexpr size_t smem = sizeof(Codiff3Smem<T, K, kCodiff3Y>);
+    static_assert(smem <= kPlainSmem);
     auto const kernel = codiff3_march_kernel<T, K, kCodiff3Y, kCodiff3Ctas>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-        return false;
     int const tz = (a.oext[2] + kMarchZ - 2) / (kMarchZ - 1), ty = (a.oext[1] + kCodiff3Y - 2) / (kCodiff3Y - 1);
     int64_t const columns = static_cast<int64_t>(tz) * ty;
     int const planes = run_length(columns, a.oext[0], static_cast<int64_t>(kCodiff3Ctas) * multiprocessors());
