@@ -26,6 +26,7 @@
 #include <mutex>
 #include <vector>
 
+#include "item_rows.cuh"
 #include "mag3d_march.cuh"
 #include "mag_ops.cuh"
 #include "precond_net.cuh"
@@ -949,18 +950,19 @@ __global__ void __launch_bounds__(kThreads) cg_update_kernel(Work<T> const* work
     Work<T> const w = work[blockIdx.x];
     Scalars* s = w.s;
     if (s->stopped[c & 1]) return;
-    T* __restrict__ r = w.r;
-    T* __restrict__ z = w.z;
-    T const* __restrict__ q = w.q;
-    T const* __restrict__ dinv = w.dinv;
+    ItemRows const rows(w.begin, w.end);
+    T* __restrict__ r = rows.of(w.r);
+    T* __restrict__ z = rows.of(w.z);
+    T const* __restrict__ q = rows.of(w.q);
+    T const* __restrict__ dinv = rows.of(w.dinv);
     // the first rows' loads are issued before the partials are summed
     constexpr int U = 4;
     T rv[U], qv[U], dv[U];
-    int row = w.begin + static_cast<int>(threadIdx.x);
+    int row = static_cast<int>(threadIdx.x);
     auto fetch = [&](int from) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            int const at = min(from + u * kThreads, w.end - 1);
+            int const at = rows.ahead(from, u * kThreads);
             rv[u] = r[at];
             qv[u] = q[at];
             dv[u] = dinv[at];
@@ -976,10 +978,10 @@ __global__ void __launch_bounds__(kThreads) cg_update_kernel(Work<T> const* work
     }
     T const alpha = static_cast<T>(a);
     double rz = 0.0, rr = 0.0;
-    for (; row < w.end; row += U * kThreads) {
+    for (; row < rows.count; row += U * kThreads) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            if (row + u * kThreads >= w.end) continue;
+            if (row + u * kThreads >= rows.count) continue;
             T const rn = rv[u] - alpha * qv[u], zn = dv[u] * rn;
             r[row + u * kThreads] = rn;
             if constexpr (Z) z[row + u * kThreads] = zn;
@@ -1026,18 +1028,19 @@ __global__ void __launch_bounds__(kThreads) cg_direction3_kernel(Work<T> const* 
 {
     __shared__ double red[2 * kThreads / 32];
     Work<T> const w = work[blockIdx.x];
-    T const* __restrict__ r = w.r;
-    T const* __restrict__ dinv = w.dinv;
-    T* __restrict__ x = w.x;
-    T* __restrict__ p = w.p;
+    ItemRows const rows(w.begin, w.end);
+    T const* __restrict__ r = rows.of(w.r);
+    T const* __restrict__ dinv = rows.of(w.dinv);
+    T* __restrict__ x = rows.of(w.x);
+    T* __restrict__ p = rows.of(w.p);
     // the first rows are on their way while the partials are summed
     constexpr int U = 4;
     T rv[U], dv[U], xv[U], pv[U];
-    int row = w.begin + static_cast<int>(threadIdx.x);
+    int row = static_cast<int>(threadIdx.x);
     auto fetch = [&](int from) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            int const at = min(from + u * kThreads, w.end - 1);
+            int const at = rows.ahead(from, u * kThreads);
             rv[u] = r[at];
             dv[u] = dinv[at];
             xv[u] = x[at];
@@ -1048,11 +1051,11 @@ __global__ void __launch_bounds__(kThreads) cg_direction3_kernel(Work<T> const* 
     Begin const b = cg_begin(w.s, c, w.part_rz, w.part_rr, w.npart, w.max_iters, w.index == 0, red, true);
     if (!b.run) return;
     T const beta = static_cast<T>(b.beta), alpha = static_cast<T>(b.alpha);
-    for (; row < w.end; row += U * kThreads) {
+    for (; row < rows.count; row += U * kThreads) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             int const at = row + u * kThreads;
-            if (at >= w.end) continue;
+            if (at >= rows.count) continue;
             p[at] = dv[u] * rv[u] + beta * pv[u];
             if (b.pending) x[at] = xv[u] + alpha * pv[u];
         }
@@ -1154,15 +1157,16 @@ __global__ void __launch_bounds__(kThreads) cg_replace_kernel(Item const* items,
     ProbInfo const pi = info[it.prob];
     Vecs<T> const v = vecs[it.prob];
     double const scale = s->scale;
-    double const* __restrict__ src = r64[it.prob];
-    T const* __restrict__ dinv = v.dinv;
-    T* __restrict__ x = v.x;
-    T* __restrict__ rv = v.r;
-    T* __restrict__ zv = v.z;
-    T* __restrict__ pold = s->pbuf == 0 ? v.p : v.p2;
+    ItemRows const rows(it.begin, it.end);
+    double const* __restrict__ src = rows.of(r64[it.prob]);
+    T const* __restrict__ dinv = rows.of(v.dinv);
+    T* __restrict__ x = rows.of(v.x);
+    T* __restrict__ rv = rows.of(v.r);
+    T* __restrict__ zv = rows.of(v.z);
+    T* __restrict__ pold = rows.of(s->pbuf == 0 ? v.p : v.p2);
     double rz = 0.0, rr = 0.0;
 #pragma unroll 4
-    for (int row = static_cast<int>(it.begin) + threadIdx.x; row < static_cast<int>(it.end); row += kThreads) {
+    for (int row = static_cast<int>(threadIdx.x); row < rows.count; row += kThreads) {
         T const r = static_cast<T>(src[row] / scale);
         T const z = dinv[row] * r;
         x[row] = T(0);
@@ -1599,21 +1603,21 @@ __global__ void __launch_bounds__(kThreads) refine_kernel(Item const* items, int
     Item const it = items[act != nullptr ? act[blockIdx.x] : blockIdx.x];
     Scalars const* s = sc + it.prob;
     if (s->outer_done) return;
-    T const* __restrict__ e = vecs[it.prob].x;
-    double* __restrict__ x = x64[it.prob];
+    ItemRows const rows(it.begin, it.end);
+    T const* __restrict__ e = rows.of(vecs[it.prob].x);
+    double* __restrict__ x = rows.of(x64[it.prob]);
     double const scale = s->scale;
-    int const end = static_cast<int>(it.end);
     if (s->pending) {
         // the last iteration's step is still to be added to x
-        T const* __restrict__ p = s->pbuf == 0 ? vecs[it.prob].p : vecs[it.prob].p2;
+        T const* __restrict__ p = rows.of(s->pbuf == 0 ? vecs[it.prob].p : vecs[it.prob].p2);
         T const alpha = static_cast<T>(s->alpha);
 #pragma unroll 4
-        for (int row = static_cast<int>(it.begin) + threadIdx.x; row < end; row += kThreads)
+        for (int row = static_cast<int>(threadIdx.x); row < rows.count; row += kThreads)
             x[row] += scale * static_cast<double>(e[row] + alpha * p[row]);
         return;
     }
 #pragma unroll 4
-    for (int row = static_cast<int>(it.begin) + threadIdx.x; row < end; row += kThreads)
+    for (int row = static_cast<int>(threadIdx.x); row < rows.count; row += kThreads)
         x[row] += scale * static_cast<double>(e[row]);
 }
 
