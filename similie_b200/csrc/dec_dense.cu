@@ -21,6 +21,7 @@
 #include <cstdlib>
 #include <type_traits>
 
+#include "run_plan.cuh"
 #include "sil_internal.cuh"
 
 namespace sil {
@@ -914,30 +915,6 @@ Dense<T, N> dense_args(Geometry const* geo, sil_field const& in, sil_field const
 // Dynamic shared memory a kernel may take without asking for it, so that the
 // marching launches have no call that can fail before them.
 constexpr size_t kPlainSmem = 48 * 1024;
-
-// Planes per run: `columns` tiles of `length` planes over `resident` CTAs at a
-// time, a run of n planes costing n + 2 steps: the cheapest total of whole waves.
-int run_length(int64_t columns, int64_t length, int64_t resident)
-{
-    int64_t const most = std::min(length, 8 * resident / columns + 1);
-    int64_t best = length, best_cost = INT64_MAX;
-    for (int64_t runs = 1; runs <= most; ++runs) {
-        int64_t const n = (length + runs - 1) / runs;
-        int64_t const waves = (columns * ((length + n - 1) / n) + resident - 1) / resident;
-        if (waves * (n + 2) < best_cost) {
-            best_cost = waves * (n + 2);
-            best = n;
-        }
-    }
-    return static_cast<int>(best);
-}
-
-int multiprocessors()
-{
-    int dev = 0, n = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n;
-}
 
 // Tile height and resident CTAs: at 161x144x130 the FP64 1-form took 62.9 us
 // with two CTAs of 8 rows, 53.8 with three, 61.6 with four, 58.9 with two of 12

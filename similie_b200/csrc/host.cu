@@ -1,6 +1,7 @@
 // host.cu -- host-side plumbing: errors, field checks, chain and Hodge rule
 // tables, geometry objects.
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -28,6 +29,19 @@ sil_status cuda_fail(cudaError_t err, char const* what)
 {
     set_error(std::string(what) + ": " + cudaGetErrorString(err));
     return err == cudaErrorMemoryAllocation ? SIL_ERR_ALLOC : SIL_ERR_CUDA;
+}
+
+int multiprocessors()
+{
+    static std::atomic<int> known[16];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+    int n = dev < 16 ? known[dev].load(std::memory_order_relaxed) : 0;
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+        if (dev < 16) known[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
 }
 
 FieldView to_view(sil_field const& f)

@@ -17,7 +17,6 @@
 // x = 0 with the inverse diagonal as preconditioner, stopped when
 // ||r|| <= tol ||b||; the final residual is re-evaluated in FP64.
 #include <algorithm>
-#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdlib>
@@ -30,6 +29,7 @@
 #include "mag3d_march.cuh"
 #include "mag_ops.cuh"
 #include "precond_net.cuh"
+#include "run_plan.cuh"
 #include "sil_internal.cuh"
 
 namespace sil {
@@ -641,20 +641,6 @@ __global__ void __launch_bounds__(kThreads) cg_init_kernel(Item const* items, Pr
     }
 }
 
-// Multiprocessors of the current device (looked up once per process and device 0..15).
-int sm_count()
-{
-    static std::atomic<int> known[16];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 148;
-    int n = dev < 16 ? known[dev].load(std::memory_order_relaxed) : 0;
-    if (n == 0) {
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
-        if (dev < 16) known[dev].store(n, std::memory_order_relaxed);
-    }
-    return n;
-}
-
 // ------------------------------------------------------------------ marching tiles (mag3d_march.cuh)
 
 template <class T>
@@ -680,9 +666,8 @@ __host__ __device__ Grid3<T> march_grid(ProbInfo const& pi)
 int march_tiles_x(ProbInfo const& pi) { return static_cast<int>((pi.nx + kMarchCols - 1) / kMarchCols); }
 int march_tiles_y(ProbInfo const& pi) { return static_cast<int>((pi.ny + kMarchOwnRows - 1) / kMarchOwnRows); }
 
-// Planes per run for a set of grids over `resident` CTAs at a time, a run of z
-// planes costing z + 2 plane steps (two planes of start-up): the cheapest
-// total of whole waves.
+// run_length for a set of grids, once a solve: every number of runs is tried, as
+// the grids' waves do not fill alike.
 int march_planes(std::vector<ProbInfo> const& grids, int64_t resident)
 {
     int64_t columns = 0, nz = 1;
@@ -855,7 +840,7 @@ int strip_rows(std::vector<ProbInfo> const& grids)
     for (; rows < 32; rows += kStripBatch) {
         int64_t ctas = 0;
         for (ProbInfo const& g : grids) ctas += strips_of(g.nx, g.ny, rows).ctas;
-        if (ctas <= 2 * static_cast<int64_t>(sm_count())) break;
+        if (ctas <= 2 * static_cast<int64_t>(multiprocessors())) break;
     }
     return rows;
 }
@@ -2324,7 +2309,7 @@ void const* resident_kernel(int per_thread)
 // limit (a lane polls kMailPerLane of a group's slots).
 int chip_blocks(sil_chip_limits const& limits)
 {
-    return limits.blocks < 0 ? sm_count() : std::min(limits.blocks, 32 * kMailPerLane);
+    return limits.blocks < 0 ? multiprocessors() : std::min(limits.blocks, 32 * kMailPerLane);
 }
 
 template <class T>
@@ -2360,7 +2345,7 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
         // A problem has at most one wave of four CTAs a multiprocessor, as every
         // CTA sums its partials (64^3 + 80^3 + 96^3, an iteration: at most 592
         // items 62 us FP32 and 104 FP64, at most 1,024 65 and 107)
-        int64_t const most = 4 * static_cast<int64_t>(sm_count());
+        int64_t const most = 4 * static_cast<int64_t>(multiprocessors());
         int64_t const rows = std::max<int64_t>(item_rows, (pi.n / most + kThreads) / kThreads * kThreads);
         int64_t const step = q.dim == 3 && q.gauge != 0 ? (4 * rows / 3) * 3 : rows / 3 * 3;
         for (int64_t b = 0; b < pi.n; b += step, ++idx) items.push_back({p, idx, b, std::min(pi.n, b + step)});
@@ -2383,7 +2368,7 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
     });
     std::vector<Tile> tiles;
     if (march) {
-        int const planes = march_planes(info, 4 * static_cast<int64_t>(sm_count()));
+        int const planes = march_planes(info, 4 * static_cast<int64_t>(multiprocessors()));
         for (int p = 0; p < np; ++p) {
             ProbInfo& pi = info[p];
             pi.first_tile = static_cast<int>(tiles.size());
@@ -2978,7 +2963,7 @@ sil_status choose_item_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
     for (ProblemDesc const& q : probs) total += (q.dim == 3 ? 3 : 1) * q.nx * q.ny * (q.dim == 3 ? q.nz : 1);
     // small batches: one wave of four CTAs per multiprocessor (fewer than two
     // rows a thread cost more in partials than they gain)
-    int64_t const wave = 4 * static_cast<int64_t>(sm_count());
+    int64_t const wave = 4 * static_cast<int64_t>(multiprocessors());
     int64_t const spread = ((total + wave - 1) / wave + kThreads - 1) / kThreads * kThreads;
     *rows = static_cast<int>(std::max<int64_t>(2 * kThreads, std::min<int64_t>(kItemNodes, spread)));
     if (char const* e = std::getenv("SIMILIE_B200_ITEM_ROWS")) {
@@ -3241,7 +3226,7 @@ sil_status launch_mag3d_apply(ProbInfo const& pi, double const* nu, double const
     } else {
         Grid3<double> const g = march_grid<double>(pi);
         int const tx = march_tiles_x(pi), ty = march_tiles_y(pi);
-        int const planes = march_planes({pi}, static_cast<int64_t>(kApplyCtas) * sm_count());
+        int const planes = run_length(static_cast<int64_t>(tx) * ty, g.nz, static_cast<int64_t>(kApplyCtas) * multiprocessors());
         int const runs = (g.nz + planes - 1) / planes;
         mag3d_march_kernel<<<static_cast<unsigned>(tx) * ty * runs, kMarchThreads, 0, s>>>(g, nu, a, y, tx, ty, planes);
     }

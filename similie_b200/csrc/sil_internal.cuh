@@ -23,6 +23,9 @@ void set_error(std::string const& msg);
 sil_status fail(sil_status status, std::string const& msg);
 sil_status cuda_fail(cudaError_t err, char const* what);
 
+// Multiprocessors of the current device (looked up once per process and device 0..15).
+int multiprocessors();
+
 #define SIL_CUDA_CHECK(call)                                 \
     do {                                                     \
         cudaError_t const err_ = (call);                     \
