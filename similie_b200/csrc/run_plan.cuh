@@ -14,8 +14,9 @@ constexpr int kRunCandidates = 10;
 // total of whole waves, the longest run among equals.  Beyond eight waves of
 // runs the start-up only costs more.  Among the cuts of as many waves the one
 // into most runs is the cheapest, so a cut per wave count is looked at, and no
-// more than kRunCandidates in all: trying every number of runs took 6 us of host
-// time at each launch of a 512x512 field and 27 at 3800x48.
+// more than kRunCandidates in all.  Host time of a call, every number of runs
+// tried -> this: the 3D operator on 12x12x4000 nodes 25.9 -> 7.2 us, a 1-form
+// Laplacian on 400x20x20 16.9 -> 13.5.
 inline int run_length(int64_t columns, int64_t length, int64_t resident, int* looked_at = nullptr)
 {
     int64_t const most = std::min(length, 8 * resident / columns + 1);
