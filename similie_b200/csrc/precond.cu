@@ -2004,7 +2004,8 @@ Table Workspace::table(int level, int aux_level, bool) const
         t.px_base[k + 1] = t.px_base[k] + static_cast<int64_t>(L.img[k].h + 2) * (L.img[k].w + 2);
         int64_t const tiles = (static_cast<int64_t>(L.img[k].w + 2) * L.img[k].h + kTilePx - 1) / kTilePx;
         t.tile_base[k + 1] = t.tile_base[k] + static_cast<int32_t>(tiles);
-        if (aux_level >= 0) {
+        // (a batch of one-level images has no other level: aux stays empty)
+        if (aux_level >= 0 && aux_level < static_cast<int>(levels.size())) {
             Level const& A = levels[aux_level];
             int const sidx = L.images[k];
             auto it = std::find(A.images.begin(), A.images.end(), sidx);
