@@ -3207,26 +3207,40 @@ __global__ void __launch_bounds__(kMarchThreads, kApplyCtas)
                 [&](int row, double q, double) { y[row] = q; });
 }
 
-// The marching tiles from 300,000 nodes on, below that a thread per node: a
-// run's two planes of start-up are a tenth or more of the few planes a small
-// grid leaves each CTA.  B200, thread per node -> tiles: 33x70x41 5.3 -> 5.7 us,
-// 64^3 8.9 -> 9.4, 250x90x30 17.2 -> 13.0, 96^3 21.9 -> 18.3, 128^3 50 -> 37,
-// 256^3 358 -> 218 us (4.3 TB/s of the 56 bytes a node; from a CUDA graph).  What
-// bounds the tiles is their issue rate: about 200 instructions per warp and
+// Whether the operator marches: from 300,000 nodes on, below which a run's two
+// planes of start-up are a tenth or more of the few planes a grid leaves each
+// CTA, and where the tiles cover the grid well enough.  A march takes `waves` of
+// planes + 2 steps of every resident thread; a thread per node works on the rows
+// of interior nodes (a warp of a boundary row ends at once).  Of 58 grids of 0.3
+// to 17 M nodes the tiles were the faster ones at three thread steps a node and
+// fewer.  B200, thread per node -> tiles, by steps a node: 1.5 256^3 358 -> 218 us
+// (4.3 TB/s of the 56 bytes a node; from a CUDA graph), 1.9 250x90x30 17.2 ->
+// 12.9, 2.2 96^3 21.7 -> 18.2, 2.8 33x33x1000 30.8 -> 27.9, 3.0 100x60x55 10.6 ->
+// 9.9, and beyond: 3.1 40x100x100 13.2 -> 12.9, 3.4 64x64x80 10.9 -> 11.1, 3.8
+// 10x1000x1000 300 -> 349, 4.5 2000x8x33 10.8 -> 14.1, 88 3x3x40000 7.1 -> 70.7.
+// What bounds the tiles is their issue rate: about 200 instructions per warp and
 // plane at 56 % of the issue slots.
 constexpr int64_t kMarchMinNodes = 300000;
+constexpr int64_t kMarchSteps = 3;   // per interior node
+
+bool mag3d_marches(ProbInfo const& pi, int64_t columns, int planes, int64_t resident)
+{
+    int64_t const runs = (pi.nz + planes - 1) / planes, waves = (columns * runs + resident - 1) / resident;
+    return waves * (planes + 2) * resident * kMarchThreads <= kMarchSteps * pi.nx * (pi.ny - 2) * (pi.nz - 2);
+}
 
 sil_status launch_mag3d_apply(ProbInfo const& pi, double const* nu, double const* a, double* y, cudaStream_t s)
 {
     unsigned const blocks = static_cast<unsigned>((pi.nodes + 255) / 256);
+    int const tx = march_tiles_x(pi), ty = march_tiles_y(pi);
+    int64_t const columns = static_cast<int64_t>(tx) * ty, resident = static_cast<int64_t>(kApplyCtas) * multiprocessors();
+    int const planes = pi.gauge || pi.nodes < kMarchMinNodes ? 0 : run_length(columns, pi.nz, resident);
     if (pi.gauge) {
         mag3d_apply_kernel<true><<<blocks, 256, 0, s>>>(pi, nu, a, y);
-    } else if (pi.nodes < kMarchMinNodes) {
+    } else if (planes == 0 || !mag3d_marches(pi, columns, planes, resident)) {
         mag3d_apply_kernel<false><<<blocks, 256, 0, s>>>(pi, nu, a, y);
     } else {
         Grid3<double> const g = march_grid<double>(pi);
-        int const tx = march_tiles_x(pi), ty = march_tiles_y(pi);
-        int const planes = run_length(static_cast<int64_t>(tx) * ty, g.nz, static_cast<int64_t>(kApplyCtas) * multiprocessors());
         int const runs = (g.nz + planes - 1) / planes;
         mag3d_march_kernel<<<static_cast<unsigned>(tx) * ty * runs, kMarchThreads, 0, s>>>(g, nu, a, y, tx, ty, planes);
     }
