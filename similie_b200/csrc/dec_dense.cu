@@ -925,11 +925,22 @@ constexpr int kLap3Ctas = sizeof(T) == 8 && K == 1 ? 3 : 2;
 
 // From how many nodes on the 3D march is taken.  1- and 2-forms: always (node
 // kernel -> march, 1-form FP64: 16^3 6.4 -> 3.1 us, 64^3 20.2 -> 9.6, 161x144x130
-// 143 -> 54).  0- and 3-forms read seven nodes and gain only once they leave L2
-// (0-form FP64: 64^3 5.9 -> 6.8, 96^3 11.9 -> 14.4, 161x144x130 30.1 -> 26.7;
-// 3-form 39.1 -> 29.7).
+// 143 -> 54), but for boxes whose columns the tiles cover badly (kLap3Steps).
+// 0- and 3-forms read seven nodes and gain less: at similar sides once they leave
+// L2 (0-form FP64: 64^3 5.9 -> 6.8, 96^3 11.9 -> 14.4, 161x144x130 30.1 -> 26.7;
+// 3-form 39.1 -> 29.7); long boxes lie to either side of it (4000x7x31 14.1 -> 6.7,
+// 2000x33x33 33.2 -> 45.7).
 template <int K>
 constexpr int64_t kLap3Min = K == 1 || K == 2 ? 1 : 2000000;
+
+// 1- and 2-forms: the most thread steps a node (threads of the tiles times
+// planes + 2 over columns times planes) at which a box of more than kLap3Small
+// nodes marches; smaller ones gain from the march's shorter chain whatever the
+// tiles cover.  Node kernel -> march, 1-form FP64 us, by steps: 5.0 4000x8x32 73 ->
+// 48, 5.2 12x1000x12 13.9 -> 9.9, 7.3 4000x31x7 62.9 -> 57.0 (component first 62.4
+// -> 85.2), 8.5 3x3x100000 24.6 -> 27.9, 11 700x700x5 164 -> 225, 65 100000x3x3 39.8
+// -> 246; small: 10 16^3 6.4 -> 3.1, 24 100x9x9 6.0 -> 4.1.
+constexpr int64_t kLap3Steps = 7, kLap3Small = 40000;
 
 // The output box lies inside the input box.
 template <int N, class T>
@@ -949,6 +960,9 @@ bool launch_lap3(cudaStream_t stream, Dense<T, 3> const& a)
     int const tz = (a.oext[2] + kMarchZ - 3) / (kMarchZ - 2), ty = (a.oext[1] + kLap3Y - 3) / (kLap3Y - 2);
     int64_t const columns = static_cast<int64_t>(tz) * ty;
     int const planes = run_length(columns, a.oext[0], static_cast<int64_t>(kLap3Ctas<T, K>) * multiprocessors());
+    if ((K == 1 || K == 2) && a.total > kLap3Small
+        && columns * (kMarchZ * kLap3Y) * (planes + 2) > kLap3Steps * a.oext[1] * a.oext[2] * planes)
+        return false;
     int64_t const blocks = columns * ((a.oext[0] + planes - 1) / planes);
     if (blocks >= (int64_t(1) << 31)) return false;
     kernel<<<static_cast<unsigned>(blocks), kMarchZ * kLap3Y, smem, stream>>>(a, tz, ty, planes);

@@ -1,13 +1,16 @@
-"""Boxes that the marching kernels' tiles cover badly (a few columns, or a few rows of them): the 3D curl-curl operator
-takes a thread per node there, and the tiles on grids of an exact number of them, one more and one fewer.
+"""Boxes that the marching kernels' tiles cover badly (a few columns, or a few rows of them): the 3D curl-curl operator and
+the 1- and 2-form Laplacians take a thread per node there, and the tiles on grids of an exact number of them, one more and
+one fewer.
 
-Values against the CPU oracle; that the dispatch does it shows in the time, against a cube of as many nodes: a march
-over 3x3x40000 nodes took 6 times the cube's, a thread per node takes less than it.
+Values against the CPU oracle and the table-driven kernels; that the dispatch does it shows in the time, against a cube
+of as many nodes: a march over 3x3x40000 nodes took 6 times the cube's, over 100000x3x3 21 times, a thread per node
+takes less and 4 times.
 """
 import numpy as np
 import pytest
 
 import oracle as O
+from test_gpu_dec_dense import _run
 from test_gpu_mag3d_march import _coords
 
 pytestmark = pytest.mark.gpu
@@ -38,6 +41,21 @@ def test_operator(shape):
     assert np.max(np.abs(y.cpu().numpy() - ref)) <= 1e-12 * np.max(np.abs(ref))
 
 
+@pytest.mark.parametrize("shape", [(2000, 6, 6), (3, 5000, 5), (4, 4, 6000), (300, 300, 2), (120, 31, 13)])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_laplacian_bits(shape, dtype):
+    import similie_b200 as sb
+    rng = np.random.default_rng(2)
+    geo = sb.Geometry([np.cumsum(rng.uniform(0.3, 1.7, s + 4)) for s in shape])
+    for k in (1, 2):
+        inp = torch.from_numpy(rng.standard_normal(shape + (3,))).cuda().to(dtype)
+        oshape = tuple(s - 1 for s in shape)
+        for layout in ("last", "first", "reversed"):
+            got, ref = (_run(sb, "laplacian", geo, shape, k, k, inp, oshape, (0, 0, 0), layout, dtype, sp)
+                        for sp in (False, True))
+            assert torch.equal(got, ref), (k, layout)
+
+
 def _time(call):
     call()
     torch.cuda.synchronize()
@@ -64,3 +82,16 @@ def test_thin_operators_are_not_marched():
         return _time(lambda: op.apply(x, y))
 
     assert time_of((3, 3, 40000)) <= 3 * time_of((72, 71, 70))
+
+
+def test_thin_laplacians_are_not_marched():
+    import similie_b200 as sb
+
+    def time_of(shape):
+        geo = sb.Geometry([np.linspace(0.0, 1.0, s) for s in shape])
+        inp = torch.randn(*shape, 3, device="cuda", dtype=torch.float64)
+        out = torch.zeros(*[s - 1 for s in shape], 3, device="cuda", dtype=torch.float64)
+        plan = sb.make_staged_laplacian(geo, out, inp, 1)
+        return _time(lambda: plan.run(out, inp))
+
+    assert time_of((100000, 3, 3)) <= 10 * time_of((74, 74, 74))
