@@ -2318,8 +2318,7 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
                             sil_chip_limits& limits, int item_rows)
 {
     int const np = static_cast<int>(probs.size());
-    // Work items: contiguous row ranges of item_rows rows per problem (3D:
-    // whole nodes, four thirds of that), one CTA each.
+    // Work items: contiguous row ranges of each problem (item_step), one CTA each.
     std::vector<Item> items;
     std::vector<ProbInfo> info(np);
     int64_t total_rows = 0;
@@ -2340,14 +2339,7 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
         pi.max_iters = set.max_iterations > 0 ? set.max_iterations : 100000;
         pi.first_item = static_cast<int>(items.size());
         int idx = 0;
-        // 3D divergence-gauge items: whole nodes (3 rows each), four times the
-        // others, so the per-CTA prologue is amortised over the costlier apply.
-        // A problem has at most one wave of four CTAs a multiprocessor, as every
-        // CTA sums its partials (64^3 + 80^3 + 96^3, an iteration: at most 592
-        // items 62 us FP32 and 104 FP64, at most 1,024 65 and 107)
-        int64_t const most = 4 * static_cast<int64_t>(multiprocessors());
-        int64_t const rows = std::max<int64_t>(item_rows, (pi.n / most + kThreads) / kThreads * kThreads);
-        int64_t const step = q.dim == 3 && q.gauge != 0 ? (4 * rows / 3) * 3 : rows / 3 * 3;
+        int64_t const step = item_step(pi.n, item_rows, multiprocessors());
         for (int64_t b = 0; b < pi.n; b += step, ++idx) items.push_back({p, idx, b, std::min(pi.n, b + step)});
         pi.nitems = idx;
         total_rows += pi.n;

@@ -17,3 +17,13 @@ def test_rows_stay_in_their_item(tmp_path):
                            os.path.join(ROOT, "tests", "cpp", "item_rows.cpp"), "-o", exe])
     run = subprocess.run([exe], capture_output=True, text=True)
     assert run.returncode == 0 and run.stdout.strip() == "rows ok", run.stdout + run.stderr
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="no g++")
+def test_items_of_a_problem(tmp_path):
+    """Whole nodes, at most one wave of CTAs, and enough of them (the divergence gauge had a quarter)."""
+    exe = str(tmp_path / "item_step")
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-Wall", "-Wextra", "-Werror",
+                           os.path.join(ROOT, "tests", "cpp", "item_step.cpp"), "-o", exe])
+    run = subprocess.run([exe], capture_output=True, text=True)
+    assert run.returncode == 0 and run.stdout.strip() == "items ok", run.stdout + run.stderr
