@@ -794,7 +794,9 @@ int sm_count()
 } // namespace
 
 // Fields the specialised 2D kernels accept: both form dims, contiguous DDC
-// layout (component fastest, then y, then x), output box inside the input.
+// layout (component fastest, then y, then x), output box inside the input.  The
+// scalar one has a row of blocks per output row, so no more rows than a grid has
+// along y.
 bool lap2d_layout_ok(sil_field const& in, sil_field const& out, int ncomp)
 {
     if (in.ndims != 2 || out.ndims != 2 || in.ncomp != ncomp || out.ncomp != ncomp) return false;
@@ -807,6 +809,7 @@ bool lap2d_layout_ok(sil_field const& in, sil_field const& out, int ncomp)
         if (out.front[d] < in.front[d]) return false;
         if (out.front[d] + out.extent[d] > in.front[d] + in.extent[d]) return false;
     }
+    if (ncomp == 1 && out.extent[0] > 65535) return false;
     return in.extent[0] >= 2 && in.extent[1] >= 2;
 }
 
