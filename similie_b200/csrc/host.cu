@@ -28,6 +28,9 @@ sil_status fail(sil_status status, std::string const& msg)
 sil_status cuda_fail(cudaError_t err, char const* what)
 {
     set_error(std::string(what) + ": " + cudaGetErrorString(err));
+    // reported here: the next call's launches are not to find it (an error that
+    // lost the context stays)
+    cudaGetLastError();
     return err == cudaErrorMemoryAllocation ? SIL_ERR_ALLOC : SIL_ERR_CUDA;
 }
 

@@ -3361,9 +3361,11 @@ sil_status sil_mag3d_operator_create(sil_mag3d_operator* out, sil_stream stream,
     auto* op = new sil_mag3d_operator_s;
     if (cudaMalloc(&op->mem, nu_bytes + gauge_bytes + sp.size() * sizeof(double)) != cudaSuccess) {
         delete op;
+        cudaGetLastError();   // as cuda_fail
         return fail(SIL_ERR_CUDA, "sil_mag3d_operator_create: device allocation failed");
     }
     auto bail = [&](sil_status e) {
+        cudaGetLastError();
         cudaFree(op->mem);
         delete op;
         return e;
