@@ -97,8 +97,9 @@ __host__ __device__ inline Strips strips_of(int64_t nx, int64_t ny, int rows)
     return s;
 }
 
-// Src: Raw load(row), T value(Raw), and out(row, q, raw): the result of an
-// owned row and its operand.
+// Src: Raw load(row) and T value(Raw), the operand at a row; Own own(row), what
+// only an owned row needs beside it.  out(row, q, operand, raw, own) takes the
+// result of an owned row.
 template <class T, class Src, class Out>
 __device__ __forceinline__ void mag2d_strip(Src const& src, T const* __restrict__ nu, int nx, int ny, int c0, int j0,
                                             int j1, Out const& out)

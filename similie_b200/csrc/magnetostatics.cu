@@ -726,7 +726,7 @@ struct Tile
 // 512^2 23.3 -> 12.7, 1024^2 26.9 -> 19.8, those 60 problems 549 -> 373 (FP64)
 // and 382 -> 267 (FP32).
 
-// Everything a CTA needs to know of its item, in one 128-byte record.
+// Everything a CTA needs to know of its item, in one record.
 template <class T>
 struct alignas(16) Work
 {
@@ -734,10 +734,8 @@ struct alignas(16) Work
     T* r;
     T* z;
     T* p;
-    T* p2;
     T* q;
     T const* dinv;
-    T const* nu;
     Scalars* s;
     double* part_pq;
     double* part_rz;
@@ -1197,12 +1195,6 @@ __global__ void __launch_bounds__(kThreads) cg_replace_kernel(Item const* items,
 // p = z + beta p.  A problem whose residual has not dropped 10x over `window`
 // iterations is marked for the plain solver.
 
-template <class T>
-__device__ __forceinline__ T* fcg_slot(T* base, int64_t hstride, int slot)
-{
-    return base + static_cast<int64_t>(slot) * hstride;
-}
-
 // x = 0, r = r64 / scale (precision T), rr0 = r.r; stall window reset.
 // Problems already handed to the plain solver get a zero correction.  After
 // the first pass (fresh = 0) the stored directions are kept: the projections
@@ -1633,14 +1625,6 @@ __global__ void copy_kernel(Item const* items, double const* const* src, double*
     Item const it = items[blockIdx.x];
     (void)sc;
     for (int64_t row = it.begin + threadIdx.x; row < it.end; row += kThreads) dst[it.prob][row] = src[it.prob][row];
-}
-
-template <class T>
-__global__ void copy_from_vec_kernel(Item const* items, Vecs<T> const* vecs, double* const* dst)
-{
-    Item const it = items[blockIdx.x];
-    T const* x = vecs[it.prob].x;
-    for (int64_t row = it.begin + threadIdx.x; row < it.end; row += kThreads) dst[it.prob][row] = static_cast<double>(x[row]);
 }
 
 // ------------------------------------------------------------------ resident solve (2D)
@@ -2593,7 +2577,7 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
             Item const& it = items[i];
             ProbInfo const& pi = info[it.prob];
             Vecs<T> const& v = vecs[it.prob];
-            work.push_back({v.x, v.r, v.z, v.p, v.p2, v.q, v.dinv, v.nu, d_sc + it.prob,
+            work.push_back({v.x, v.r, v.z, v.p, v.q, v.dinv, d_sc + it.prob,
                             part_a + (march ? pi.first_tile : (flat ? strip_part[it.prob] : pi.first_item)),
                             part_b + pi.first_item, part_c + pi.first_item, static_cast<int>(it.begin),
                             static_cast<int>(it.end), it.index, pi.nitems,

@@ -119,11 +119,6 @@ __device__ __forceinline__ Float2x fma2(Float2x a, Float2x b, Float2x c)
     return r;
 }
 
-__device__ __forceinline__ uint4 ld_chunk(bf16 const* base, int64_t px, int c)
-{
-    return __ldg(reinterpret_cast<uint4 const*>(base + px * kCh) + c);
-}
-
 __device__ __forceinline__ int find_image(Table const& t, int tile)
 {
     int lo = 0, hi = t.nimg - 1;
@@ -1359,17 +1354,6 @@ __global__ void jacobi_kernel(const __grid_constant__ Samples ss, float const* n
     out[o + row] = bv + w * (dinv[o + row] * r);
 }
 
-// out = b - K e
-__global__ void residual_kernel(const __grid_constant__ Samples ss, float const* nu, float const* b, float const* e,
-                                float* out)
-{
-    int64_t row;
-    Sample sm;
-    if (!node_of(ss, row, sm)) return;
-    int64_t const o = sm.offset;
-    out[o + row] = b[o + row] - mag_apply_node(e + o, nu + o, sm.nx, sm.ny, row);
-}
-
 // out = K e
 __global__ void kapply_kernel(const __grid_constant__ Samples ss, float const* nu, float const* e, float* out)
 {
@@ -1528,20 +1512,6 @@ struct WrapItem
     int32_t sample, begin, end, index;   // index: item number within its sample
 };
 
-// K e at interior node (i, j) of an nx-wide grid for an e given by a functor.
-// e(q, i, j) gets the node's coordinates, so no index division per neighbour.
-template <class E>
-__device__ __forceinline__ float k_row(E const& e, float const* nu, int nx, int row, int i, int j)
-{
-    float const a0 = e(row, i, j);
-    float res = 0.0f;
-    if (j >= 2) res = res + (a0 - e(row - nx, i, j - 1)) * nu[row - nx];
-    res = res + (a0 - e(row + nx, i, j + 1)) * nu[row];
-    if (i >= 2) res = res + (a0 - e(row - 1, i - 1, j)) * nu[row - 1];
-    res = res + (a0 - e(row + 1, i + 1, j)) * nu[row];
-    return res;
-}
-
 __device__ __forceinline__ double block_sum_d(double v, double* red)
 {
     for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
@@ -1649,17 +1619,6 @@ __global__ void wrap_finish_kernel(const __grid_constant__ Samples ss, double co
     for (int k = ss.strip_base[sidx] + static_cast<int>(threadIdx.x); k < ss.strip_base[sidx + 1]; k += 32) t += part[k];
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     if (threadIdx.x == 0) dots[sidx * 3] = t;
-}
-
-// The active samples' nodes as one compacted range: f(k, row) for node row
-// of sample k (walk_range).  No barrier may sit inside f.
-template <class F>
-__device__ __forceinline__ void walk_nodes(Samples const& ss, int64_t* pre, F const& f)
-{
-    scan_active(
-        ss.n, [&](int k) { return sample_active(ss, k) ? static_cast<int64_t>(ss.s[k].nx) * ss.s[k].ny : int64_t(0); },
-        pre);
-    walk_range(pre, ss.n, 1, f);
 }
 
 // s = rms(D^-1/2 r1) per sample (dots[k*3] = |D^-1/2 r1|^2), staged in shared
