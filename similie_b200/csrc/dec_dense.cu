@@ -361,9 +361,11 @@ __global__ void __launch_bounds__(kDenseBlock) dense_kernel(const __grid_constan
 // boxes that reach outside the input keep the per-node kernel.
 //
 // B200, per-node kernel -> march: 3D 1-form 161x144x130 FP64 143 -> 54 us (2.7
-// TB/s), FP32 107 -> 38; 2D 1-form 1999x2741 FP32 46 -> 21 us (4.1 TB/s).  The 3D
-// march is bound by its instructions and the 30 % of its threads that only
-// serve their neighbours, the 2D one by memory.
+// TB/s), FP32 107 -> 38; 2D 1-form 1999x2741 FP32 46 -> 21 us (4.1 TB/s, its
+// fields in L2; 28 when they are not).  The 3D march is bound by the data pipe
+// of L1 and shared memory (68 % busy), its instructions (58 % of the issue slots)
+// and the 30 % of its threads that only serve their neighbours, the 2D one by
+// the loads its sixteen warps a multiprocessor have in flight.
 
 // Chain-order sum like chain(), the sampler taking the face's dim and shift.
 template <int N, int R, bool TR, int C, class T, class V>
@@ -642,10 +644,11 @@ __global__ void __launch_bounds__(kMarchZ* Y, CTAS)
 // and z neighbours through a double-buffered plane, its x neighbour kept.  Only
 // lower neighbours are read, so the tile owns 31 x (Y - 1) columns.
 //
-// Bound by its loads in flight and the idle threads of its tiles (63 % of the
-// copy rate at 150x171x128, FP64).  B200, node kernel -> march at that size: 2-form
-// FP64 52.8 -> 39.8 us, FP32 47.2 -> 27.5; 1-form 34.5 -> 30.1, 32.0 -> 24.1;
-// 3-form 36.2 -> 30.2, 33.4 -> 20.1.
+// Bound by the data pipe of L1 and shared memory (65 % busy, half of its shared
+// wavefronts bank conflicts of the three-component ring) and the idle threads of
+// its tiles; 63 % of the copy rate at 150x171x128, FP64.  B200, node kernel ->
+// march at that size: 2-form FP64 52.8 -> 39.8 us, FP32 47.2 -> 27.5; 1-form 34.5
+// -> 30.1, 32.0 -> 24.1; 3-form 36.2 -> 30.2, 33.4 -> 20.1.
 template <class T, int K, int Y>
 struct Codiff3Smem
 {

@@ -1640,9 +1640,14 @@ __global__ void copy_kernel(Item const* items, double const* const* src, double*
 //
 // B200, per iteration against two kernels: four problems of 96^2 .. 161^2 11.2 ->
 // 6.2 us, 512^2 12.7 -> 7.2, 1024^2 19.8 -> 12.5 (FP64), six problems of 128^2 ..
-// 1024^2 41 -> 28, sixty 373 -> 237 (FP64) and 267 -> 137 (FP32).  What bounds it:
-// small problems the two meetings (about 1.7 us each at sixteen CTAs), 1024^2 the
-// shared-memory reads of 7,168 nodes by sixteen warps.
+// 1024^2 41 -> 28, sixty 373 -> 237 (FP64) and 267 -> 137 (FP32).  What bounds it
+// is waiting, in the two meetings (about 1.7 us each at sixteen CTAs) and at the
+// barriers between the loops: two thirds of the stalls at 128^2 and half at
+// 1024^2, where the shared-memory reads of 7,168 nodes keep their pipe busy for
+// 35 % of the time.
+//
+// A launch that the device refuses, and a group of which a wait ran out, leave
+// their problems to the kernels per iteration.
 constexpr int kResThreads = 512;
 // Nodes of a thread at most (r, x and q take three registers of T each): 7,168
 // a CTA in FP64, 14,336 in FP32.
@@ -3194,8 +3199,9 @@ __global__ void __launch_bounds__(kMarchThreads, kApplyCtas)
 // 12.9, 2.2 96^3 21.7 -> 18.2, 2.8 33x33x1000 30.8 -> 27.9, 3.0 100x60x55 10.6 ->
 // 9.9, and beyond: 3.1 40x100x100 13.2 -> 12.9, 3.4 64x64x80 10.9 -> 11.1, 3.8
 // 10x1000x1000 300 -> 349, 4.5 2000x8x33 10.8 -> 14.1, 88 3x3x40000 7.1 -> 70.7.
-// What bounds the tiles is their issue rate: about 200 instructions per warp and
-// plane at 56 % of the issue slots.
+// What bounds the tiles is the data pipe of L1 and shared memory (71 % busy) and
+// their issue rate: about 200 instructions per warp and plane at 61 % of the
+// issue slots.
 constexpr int64_t kMarchMinNodes = 300000;
 constexpr int64_t kMarchSteps = 3;   // per interior node
 
