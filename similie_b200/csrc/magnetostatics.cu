@@ -2931,7 +2931,8 @@ sil_status solve_batch_rows(std::vector<ProblemDesc> const& probs, sil_solve_set
 // caller's solution buffers, which the real solve overwrites).  Smaller
 // batches take the rows that make one wave, at most 4,096.
 // SIMILIE_B200_ITEM_ROWS=<rows> forces a size; SIMILIE_B200_AUTOTUNE=0 keeps
-// the default.
+// the default.  (Whatever the size, a problem has at most one wave of items:
+// item_step.)
 constexpr int kItemCandidates[3] = {2048, 4096, 8192};
 std::mutex g_item_mutex;
 int g_item_rows_tuned[4] = {0, 0, 0, 0};  // [precision FP64 / FP32][first problem 2D / 3D]
