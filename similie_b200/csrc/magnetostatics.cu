@@ -726,9 +726,9 @@ struct Tile
 // 512^2 23.3 -> 12.7, 1024^2 26.9 -> 19.8, those 60 problems 549 -> 373 (FP64)
 // and 382 -> 267 (FP32).
 
-// Everything a CTA needs to know of its item, in one record.
+// Everything a CTA needs to know of its item, in one 128-byte line.
 template <class T>
-struct alignas(16) Work
+struct alignas(128) Work
 {
     T* x;
     T* r;
